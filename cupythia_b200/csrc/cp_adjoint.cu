@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(CP_ADJ_THREADS) k_adjoint(const CpHadParams P,
   for (int k = 0; k < 8; ++k) { acc[k] = 0.f; cmp[k] = 0.f; }
   float wmax = 0.f;
   uint32_t nbad = 0;
-  float* my = sDyn + warp * 12 * nb;
+  float* const my[3] = {sDyn + warp * 12 * nb, sDyn + (warp * 12 + 4) * nb, sDyn + (warp * 12 + 8) * nb};
 
   for (uint64_t r = 0; r < rounds; ++r) {
     const uint64_t p = r * stride + gtid;
@@ -128,14 +128,15 @@ __global__ void __launch_bounds__(CP_ADJ_THREADS) k_adjoint(const CpHadParams P,
         }
       }
     }
+    float hv[3][4];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      float* h = my + d * 4 * nb;
-      cp_warp_hist_add(h, bin[d], dlo[d]);
-      cp_warp_hist_add(h + nb, bin[d], dhi[d]);
-      cp_warp_hist_add(h + 2 * nb, bin[d], wq * dlo[d]);
-      cp_warp_hist_add(h + 3 * nb, bin[d], wq * dhi[d]);
+      hv[d][0] = dlo[d];
+      hv[d][1] = dhi[d];
+      hv[d][2] = wq * dlo[d];
+      hv[d][3] = wq * dhi[d];
     }
+    cp_warp_hist_add<3, 4>(my, nb, bin, hv);
   }
   // block reduction of the head sums, FP64 across warps in fixed order
   double v[CP_ADJ_HEAD];

@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(CP_THREADS, CP_MIN_BLOCKS) k_had_accum(const _
   const uint64_t rounds = (L.n + stride - 1) / stride;
   float s1 = 0.f, c1 = 0.f, s2 = 0.f, c2 = 0.f, wmax = 0.f;
   uint32_t nbad = 0;
-  float* myHist = &sHist[warp][0][0];
+  float* const myHist[3] = {&sHist[warp][0][0], &sHist[warp][1][0], &sHist[warp][2][0]};
 
   for (uint64_t r = 0; r < rounds; ++r) {
     const uint64_t p = r * stride + gtid;
@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(CP_THREADS, CP_MIN_BLOCKS) k_had_accum(const _
       }
     }
     const float w2 = w * w;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) cp_warp_hist_add(myHist + d * CP_MAX_BINS, bin[d], w2);
+    const float hv[3][1] = {{w2}, {w2}, {w2}};
+    cp_warp_hist_add<3, 1>(myHist, 0, bin, hv);
   }
 
   // compensated warp trees: Kahan sum s with compensation -c is the pair (s, -c)
