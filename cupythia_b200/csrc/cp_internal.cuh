@@ -118,6 +118,7 @@ struct cp_handle {
   double wmax_host = 0.0;                  // the unweighting threshold d_wmax[0], as last set
   double* d_wmax = nullptr;                // [0] threshold used by cp_unweight, [1] quantile q
   unsigned long long* d_counter = nullptr; // accepted-event counter
+  unsigned* d_ticket = nullptr;            // last-block ticket of the iteration's finish (0 between launches)
   // production staging for pdfbuf_cap points (K1 -> K2): PDFs and record tails per point, accept
   // masks per 32-point block, totals and output offsets per 1024-point range; per-chunk sums
   float4* d_pdfbuf = nullptr;
@@ -368,9 +369,8 @@ __device__ __forceinline__ void cp_warp_hist_add(float* const (&h)[ND], int ld, 
 
 // out[k] = sum over blocks of slots[b][k], or their max for k == max_col; fixed order, FP64.
 // One warp per output element.
-template <int UNUSED>
-__global__ void k_reduce_slots(const double* __restrict__ slots, int nblocks, int width, double* out,
-                               int max_col = 2)
+__device__ __forceinline__ void cp_reduce_column(const double* __restrict__ slots, int nblocks, int width, double* out,
+                                                 int max_col)
 {
   const int k = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -384,6 +384,13 @@ __global__ void k_reduce_slots(const double* __restrict__ slots, int nblocks, in
     acc = cp_warp_sum_d(acc);
   }
   if (lane == 0) out[k] = acc;
+}
+
+template <int UNUSED>
+__global__ void k_reduce_slots(const double* __restrict__ slots, int nblocks, int width, double* out,
+                               int max_col = 2)
+{
+  cp_reduce_column(slots, nblocks, width, out, max_col);
 }
 
 #endif
