@@ -565,74 +565,99 @@ struct PartonicArgs {
 };
 
 // Sigma2gg2gg::sigmaKin (pythia8317/src/SigmaQCD.cc:115-129; pipeline/physics.cuh:9-16) for a fixed
-// s-hat.  With s + t + u = 0 the three brackets sigTS + sigUS + sigTU sum to
-// (9/2) (3 - t u / s^2 - s u / t^2 - s t / u^2), the textbook form of the g g -> g g matrix element,
-// which takes one FP64 reciprocal (of t u; 1/t = u / (t u), 1/u = t / (t u)) and about half the
-// operations of the bracket form.  With u = -s - t rounded as the reference rounds it, the two
-// forms agree to 1.1e-15 relative over |cos theta| < 0.9.  The prefactor (pi / s^2) alpha_s^2 / 2
-// is the same for every draw and is formed once.
-struct CpGG2GG {
-  double s, is2, pre, cMax;
-  __device__ __forceinline__ CpGG2GG(double s_, double aS, double cMax_) : s(s_), cMax(cMax_)
+// s-hat.  With s + t + u = 0 the three brackets sigTS + sigUS + sigTU sum to the textbook form
+// (9/2) (3 - t u / s^2 - s u / t^2 - s t / u^2) of the g g -> g g matrix element.  With
+// t = -s (1 - c) / 2, u = -s (1 + c) / 2 and p = 1 - c^2 = 4 t u / s^2 it depends on p alone,
+//   s u / t^2 + s t / u^2 = s (t^3 + u^3) / (t u)^2 = -s^2 (s^2 - 3 t u) / (t u)^2
+//                         = 12 / p - 16 / p^2,
+// so it is 3 - p/4 + (16 y - 12) y with y = 1 / p: with p <= 1 both 3 - p/4 and 16 y - 12 >= 4 y
+// are sums without cancellation, and p is the FMA 1 - c c, rounded once, so the form is within a
+// few 1e-16 of the exact value at its c (the bracket form: 1.1e-15 over |cos theta| < 0.9).
+// Twelve FP64 operations a draw with the sums, against 27 and an IEEE division in terms of t and u
+// (1.05e9 SplitMix64 draws: 3.03 ms there, 1.86 ms here); the prefactor
+// (pi / s^2) alpha_s^2 / 2 (9/2) is the same for every draw and multiplies the sums.
+__device__ __forceinline__ double cp_gg2gg_form(double c)
+{
+  const double p = fma(-c, c, 1.0);
+  // 1 / p for p in (0, 1], normal: the hardware's approximation (its input and result are the upper
+  // words, so within about 2^-19) and one third-order step y (1 + e + e^2), e = 1 - p y, which
+  // leaves e^3 < 2^-56 and the rounding
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(p));
+  const double e = fma(-p, y, 1.0);
+  y = fma(y, fma(e, e, e), y);
+  return fma(fma(16.0, y, -12.0), y, fma(-0.25, p, 3.0));
+}
+
+// cos theta = (2 u01 - 1) cMax of 64 random bits, u01 = (v >> 11) 2^-53.  2 u01 - 1 is exact: the
+// upper 32 bits and the next 21 become the low mantissa words of 2^21 + H 2^-31 and 1 + L 2^-52, and
+// both additions are exact (multiples of 2^-52 below 2), without a 64-bit integer conversion.
+__device__ __forceinline__ double cp_partonic_cos(uint32_t hi, uint32_t lo, double cMax)
+{
+  const double dh = __hiloint2double(0x41400000, (int)hi), dl = __hiloint2double(0x3FF00000, (int)(lo >> 11));
+  return ((dh - 2097154.0) + dl) * cMax;
+}
+
+// Sums of the matrix element over draws.
+struct CpPartonicSums {
+  double s1 = 0.0, s2 = 0.0, wm = 0.0;
+  __device__ __forceinline__ void add(double v)
   {
-    const double is = 1.0 / s;
-    is2 = is * is;
-    pre = M_PI * is * is * (aS * aS) * 0.5 * 4.5;
-  }
-  // dsigma/dt at cos theta = (2 u01 - 1) cMax
-  __device__ __forceinline__ double operator()(double u01) const
-  {
-    const double c = (2.0 * u01 - 1.0) * cMax;
-    const double tH = -0.5 * s * (1.0 - c), uH = -s - tH;
-    const double tu = tH * uH, itu = 1.0 / tu;
-    const double it = uH * itu, iu = tH * itu;
-    return pre * (3.0 - tu * is2 - (s * uH) * (it * it) - (s * tH) * (iu * iu));
+    s1 += v;
+    s2 = fma(v, v, s2);
+    if (v > wm) wm = v;
   }
 };
 
-__device__ __forceinline__ double cp_philox_u01_d(uint64_t seed, uint64_t point)
-{
-  uint32_t wd[4];
-  cp_point_words(seed, point, 0, 0, wd);
-  const uint64_t v = ((uint64_t)wd[1] << 32) | wd[0];
-  return (double)(v >> 11) * (1.0 / 9007199254740992.0);
-}
-
 // MODE 0: Philox sums over points; 1: SplitMix64 sums over the reference's (thread, draw) pairs;
-// 2: Philox per-point weights.  Sums are of dsigma/dt; each block scales its slot by `scale`.
+// 2: Philox per-point weights.  Sums are of the bare form above; each block scales its slot.
+// Bound by instruction issue: about 20 integer operations (SplitMix64) and 12 FP64 a draw.
 template <int MODE>
 __global__ void __launch_bounds__(CP_THREADS, 5) k_partonic(const PartonicArgs a)
 {
   __shared__ double sRed[CP_WARPS][3];
-  const CpGG2GG f(a.s, a.aS, a.cMax);
-  double s1 = 0.0, s2 = 0.0, wm = 0.0;
+  const double scale = M_PI / (a.s * a.s) * (a.aS * a.aS) * 0.5 * 4.5 * a.scale;
+  CpPartonicSums S;
   const uint64_t nthr = (uint64_t)gridDim.x * CP_THREADS;
   const uint64_t t = (uint64_t)blockIdx.x * CP_THREADS + threadIdx.x;
   if (MODE == 1) {
     // the reference's thread i makes draws k = 0 .. kper-1 from counter seed + i 0x100000001B3 + k
     // (cuPythia/03_fused_resident_me/fused_gg2gg.cu:43-50); the n kper pairs are split into
-    // equal contiguous shares, so every thread here does the same number of draws
+    // equal contiguous shares, so every thread here does the same number of draws (the first
+    // total % nthr threads one more).  Within a reference thread the counters are consecutive; a
+    // warp advances by the draws that all of its lanes have left in theirs, so its lanes stay
+    // converged (lanes that loop over their own runs were 59% active at 1000 draws a thread).
     const uint64_t total = a.n * a.kper, q = total / nthr, rem = total % nthr;
-    const uint64_t w0 = q * t + (t < rem ? t : rem), cnt = q + (t < rem ? 1 : 0);
-    uint64_t i = w0 / a.kper, k = w0 - i * a.kper;
+    const uint64_t w0 = q * t + (t < rem ? t : rem);
+    uint64_t left = q, i = w0 / a.kper, k = w0 - i * a.kper;
     uint64_t ctr = a.seed + i * 0x100000001B3ULL + k;
-    for (uint64_t w = 0; w < cnt; ++w) {
-      const double v = f(cp_u01(cp_splitmix64(ctr)));
-      s1 += v; s2 += v * v; wm = fmax(wm, v);
-      if (++k == a.kper) { k = 0; ++i; ctr = a.seed + i * 0x100000001B3ULL; }
-      else ++ctr;
+    const auto draw = [&](uint64_t c) {
+      const uint64_t v = cp_splitmix64(c);
+      S.add(cp_gg2gg_form(cp_partonic_cos((uint32_t)(v >> 32), (uint32_t)v, a.cMax)));
+    };
+    while (left) {
+      uint64_t run = a.kper - k;
+      run = run < left ? run : left;
+      const uint32_t m = __reduce_min_sync(0xffffffffu, run < (1u << 30) ? (uint32_t)run : (1u << 30));
+#pragma unroll 4
+      for (uint32_t j = 0; j < m; ++j) draw(ctr + j);
+      left -= m;
+      k += m;
+      ctr += m;
+      if (k == a.kper) { k = 0; ++i; ctr = a.seed + i * 0x100000001B3ULL; }
     }
+    if (t < rem) draw(ctr);
   } else {
     for (uint64_t i = t; i < a.n; i += nthr) {
-      const double v = f(cp_philox_u01_d(a.seed, a.p0 + i));
-      if (MODE == 2) { a.w_out[i] = v * a.scale; continue; }
-      s1 += v; s2 += v * v; wm = fmax(wm, v);
+      uint32_t wd[4];
+      cp_point_words(a.seed, a.p0 + i, 0, 0, wd);
+      const double v = cp_gg2gg_form(cp_partonic_cos(wd[1], wd[0], a.cMax));
+      if (MODE == 2) { a.w_out[i] = v * scale; continue; }
+      S.add(v);
     }
   }
   if (MODE == 2) return;
-  s1 = cp_warp_sum_d(s1);
-  s2 = cp_warp_sum_d(s2);
-  wm = cp_warp_max_d(wm);
+  const double s1 = cp_warp_sum_d(S.s1), s2 = cp_warp_sum_d(S.s2), wm = cp_warp_max_d(S.wm);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) { sRed[warp][0] = s1; sRed[warp][1] = s2; sRed[warp][2] = wm; }
   __syncthreads();
@@ -640,7 +665,7 @@ __global__ void __launch_bounds__(CP_THREADS, 5) k_partonic(const PartonicArgs a
     double b1 = 0, b2 = 0, bm = 0;
     for (int k = 0; k < CP_WARPS; ++k) { b1 += sRed[k][0]; b2 += sRed[k][1]; bm = fmax(bm, sRed[k][2]); }
     double* slot = a.slots + 4 * (size_t)blockIdx.x;
-    slot[0] = b1 * a.scale; slot[1] = b2 * (a.scale * a.scale); slot[2] = bm * a.scale; slot[3] = 0.0;
+    slot[0] = b1 * scale; slot[1] = b2 * (scale * scale); slot[2] = bm * scale; slot[3] = 0.0;
   }
 }
 
