@@ -111,7 +111,7 @@ struct cp_handle {
   float* d_uH = nullptr;          // uHat, formed at the input precision (FP64 for cp_set2kin_batch_f64)
   // launch shapes (resident blocks per SM on this handle's device; -1 until first use)
   int had_blocks = 0;
-  int adj_per_sm_nt[2] = {-1, -1}, flow_per_sm = -1, unw_per_sm = -1;   // adjoint: x tangents only / all six
+  int adj_per_sm_nt[2] = {-1, -1}, flow_per_sm = -1;   // adjoint: x tangents only / all six
   int build_per_sm[2] = {-1, -1};   // record builder without / with scale weights
   // weight histogram of the last iteration and the unweighting threshold (device)
   unsigned long long* d_qhist = nullptr;   // CP_QBINS

@@ -65,7 +65,7 @@ __device__ __forceinline__ CpMapped cp_map_any(const float2 (*sEdge)[CP_MAX_BINS
 
 __device__ __forceinline__ void cp_stage_edges(float2 (*sEdge)[CP_MAX_BINS], const double* edges, int nb)
 {
-  for (int k = threadIdx.x; k < 3 * nb; k += CP_THREADS) {
+  for (int k = threadIdx.x; k < 3 * nb; k += blockDim.x) {
     int d = k / nb, b = k - d * nb;
     const double* e = edges + d * (nb + 1);
     double lo = e[b], hi = e[b + 1];
@@ -78,23 +78,27 @@ __device__ __forceinline__ void cp_stage_edges(float2 (*sEdge)[CP_MAX_BINS], con
 // block's staging slots in point order; K2 builds the record from them.
 // FLOW_U: the points' accept draws come from the flow forward's output (L.flow_u) instead of their
 // Philox blocks; a separate instance, so the plain form's kernel carries no code for it
+//
+// The grid is not the resident blocks but many small blocks of L.rounds x CP_UNW_THREADS
+// consecutive points: the scheduler serves a multiprocessor's warps unevenly, so with one share of
+// the chunk per resident warp some finished early and left 3.2 of 4 warps per scheduler on average
+// (issue 68%); a finished block is replaced at once (issue 73%, FMA pipe
+// 72%): 2^27 points 7.39 -> 7.00 ms.
 template <bool FLOW_U>
-__global__ void __launch_bounds__(CP_THREADS, CP_MIN_BLOCKS) k_unw_accept(const __grid_constant__ CpHadParams P,
-                                                                           const __grid_constant__ UnwLaunch L)
+__global__ void __launch_bounds__(CP_UNW_THREADS, CP_UNW_RESIDENT)
+    k_unw_accept(const __grid_constant__ CpHadParams P, const __grid_constant__ UnwLaunch L)
 {
   __shared__ float2 sEdge[3][CP_MAX_BINS];
-  __shared__ double sRed[CP_WARPS][7];
+  __shared__ double sRed[CP_UNW_THREADS / 32][7];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  cp_stage_edges(sEdge, L.edges, L.nb);
+  if (!L.flow) cp_stage_edges(sEdge, L.edges, L.nb);
   __syncthreads();
   const float wmax = (float)L.wmax[0];
-  const uint64_t stride = (uint64_t)gridDim.x * CP_THREADS;
-  const uint64_t gtid = (uint64_t)blockIdx.x * CP_THREADS + threadIdx.x;
-  const uint64_t rounds = (L.n + stride - 1) / stride;
+  const uint64_t first = (uint64_t)blockIdx.x * L.rounds * CP_UNW_THREADS;
   CpUnwSums S;
-  for (uint64_t r = 0; r < rounds; ++r) {
-    // the warp's 32 points are one block: p - lane is a multiple of 32 (stride and block slices are)
-    const uint64_t p = r * stride + gtid;
+  for (unsigned r = 0; r < L.rounds; ++r) {
+    // the warp's 32 points are one block: p - lane is a multiple of 32 (block and round sizes are)
+    const uint64_t p = first + r * CP_UNW_THREADS + threadIdx.x;
     uint32_t wd[4] = {0u, 0u, 0u, 0u};
     CpMapped m{};
     float u = 0.f;
@@ -116,30 +120,68 @@ __global__ void __launch_bounds__(CP_THREADS, CP_MIN_BLOCKS) k_unw_accept(const 
   if (lane == 0)
     for (int k = 0; k < 7; ++k) sRed[warp][k] = v[k];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double* slot = L.slots + (size_t)blockIdx.x * CP_UNW_SLOT;
-    for (int k = 0; k < 7; ++k) {
-      double a = 0.0;
-      for (int q = 0; q < CP_WARPS; ++q) a = (k == 2) ? fmax(a, sRed[q][k]) : a + sRed[q][k];
-      slot[k] = a;
-    }
-    slot[7] = 0.0;
+  if (threadIdx.x < CP_UNW_SLOT) {
+    const int k = threadIdx.x;
+    double a = 0.0;
+    if (k < 7)
+      for (int q = 0; q < CP_UNW_THREADS / 32; ++q) a = (k == 2) ? fmax(a, sRed[q][k]) : a + sRed[q][k];
+    L.slots[(size_t)blockIdx.x * CP_UNW_SLOT + k] = a;
   }
 }
 
-// Output offsets: roff[r] = *base_io + the records of the ranges before r; then *base_io +=
-// the chunk's records.  One block of 1024 threads scans the range totals in tiles of 1024
-// (coalesced loads, warp shuffles, one running carry): fixed order.
-__global__ void __launch_bounds__(1024) k_unw_scan(const unsigned* __restrict__ rsum, uint64_t nrange,
-                                                   unsigned long long* base_io, unsigned long long* __restrict__ roff)
+// Between the accept kernel and the record builder, in one launch of two blocks: block 0 adds the
+// accept blocks' sums (fixed order: thread t takes column t % 8 of slots t / 8, t / 8 + 128, ...,
+// then the xor tree of a warp, then the warps in order), block 1 turns the range totals into output
+// offsets: roff[r] = *base_io (0 for `first`) + the records of the ranges before r; then
+// *base_io = the records so far.  Sixteen ranges a thread, so the 16,384 ranges of a full chunk are
+// one tile: one scan over the block (warp shuffles, a warp over the warps' sums) instead of sixteen
+// (18 us of every chunk, 13 of them saved).  The totals are cleared as they are read, for the next chunk.
+#define CP_SCAN_PER 16
+__global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ slots, int nslots, double* __restrict__ red,
+                                                     uint4* __restrict__ rsum, uint64_t nrange, int first,
+                                                     unsigned long long* base_io, unsigned long long* __restrict__ roff)
 {
+  __shared__ double sRed[32][CP_UNW_SLOT];
   __shared__ unsigned long long wsum[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  unsigned long long carry = *base_io;
-  for (uint64_t i0 = 0; i0 < nrange; i0 += 1024) {
-    const uint64_t i = i0 + t;
-    const unsigned long long v = i < nrange ? rsum[i] : 0ull;
-    unsigned long long x = v;
+  if (blockIdx.x == 0) {
+    const int c = t & 7;
+    double a = 0.0;
+    for (int b = t >> 3; b < nslots; b += 128) {
+      const double v = slots[(size_t)b * CP_UNW_SLOT + c];
+      a = c == 2 ? fmax(a, v) : a + v;
+    }
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+      const double v = __shfl_xor_sync(0xffffffffu, a, o);
+      a = c == 2 ? fmax(a, v) : ((lane & o) ? v + a : a + v);
+    }
+    if (lane < CP_UNW_SLOT) sRed[w][lane] = a;
+    __syncthreads();
+    if (t < CP_UNW_SLOT) {
+      a = 0.0;
+      for (int q = 0; q < 32; ++q) a = t == 2 ? fmax(a, sRed[q][t]) : a + sRed[q][t];
+      red[t] = a;
+    }
+    return;
+  }
+  unsigned long long carry = first ? 0ull : *base_io;
+  for (uint64_t i0 = 0; i0 < nrange; i0 += 1024 * CP_SCAN_PER) {
+    const uint64_t i = i0 + (uint64_t)t * CP_SCAN_PER;
+    unsigned v[CP_SCAN_PER] = {};
+    // rsum and roff are allocated, and rsum zero, to a multiple of CP_SCAN_PER ranges
+    if (i < nrange) {
+#pragma unroll
+      for (int q = 0; q < CP_SCAN_PER / 4; ++q) {
+        const uint4 x = rsum[i / 4 + q];
+        rsum[i / 4 + q] = make_uint4(0u, 0u, 0u, 0u);
+        v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+      }
+    }
+    unsigned own = 0;   // at most 16 x 1024 records
+#pragma unroll
+    for (int q = 0; q < CP_SCAN_PER; ++q) own += v[q];
+    unsigned long long x = own;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
@@ -157,12 +199,18 @@ __global__ void __launch_bounds__(1024) k_unw_scan(const unsigned* __restrict__ 
       wsum[lane] = z;
     }
     __syncthreads();
-    if (i < nrange) roff[i] = carry + (w ? wsum[w - 1] : 0ull) + x - v;
+    unsigned long long at = carry + (w ? wsum[w - 1] : 0ull) + x - own;
+    if (i < nrange) {
+#pragma unroll
+      for (int q = 0; q < CP_SCAN_PER; q += 2) {
+        reinterpret_cast<ulonglong2*>(roff + i)[q / 2] = make_ulonglong2(at, at + v[q]);
+        at += v[q] + v[q + 1];
+      }
+    }
     carry += wsum[31];
     __syncthreads();   // wsum is rewritten by the next tile
   }
-  __syncthreads();     // every thread has read *base_io
-  if (t == 0) *base_io = carry;
+  if (t == 0) *base_io = carry;   // every thread has read it: the loop's barriers (nrange >= 1)
 }
 
 // K2: work units of a quarter range (8 blocks, 256 points: 65,536 per 2^24-point chunk, so the
@@ -249,16 +297,18 @@ __global__ void __launch_bounds__(CP_THREADS, SCALEW ? 2 : 4) k_unw_build(const 
 
 __global__ void k_set_wmax(double* wmax, double v) { wmax[0] = v; }
 
-static int unw_blocks(cp_handle* h)
+// Points per thread of an accept block for n points.  With `share` the points of a resident thread
+// of the whole device: share / 8 (eight waves of blocks), at most CP_UNW_MAXROUNDS; but a block's
+// start (edges, threshold) costs about a round, so three rounds from twelve points of share on, and
+// share / 4 below.  Accept kernel, 10^6 points (share 13): 72 us with one round, 67 with three, 67
+// with one wave; 2^22 points (share 55): 233 us with six, 241 with 13, 241 with one wave; 2^24
+// (share 221): 875 us with 27, 924 with one wave.
+static unsigned accept_rounds(const cp_handle* h, uint64_t n)
 {
-  if (h->unw_per_sm < 0) {
-    int per_sm = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_unw_accept<false>, CP_THREADS, 0) != cudaSuccess ||
-        per_sm < 1)
-      per_sm = 1;
-    h->unw_per_sm = per_sm;
-  }
-  return h->num_sms * h->unw_per_sm;
+  const uint64_t share = n / ((uint64_t)h->num_sms * CP_UNW_RESIDENT * CP_UNW_THREADS);
+  uint64_t r = share / 8;
+  if (r < 3) r = share / 4 < 3 ? share / 4 : 3;
+  return r < 1 ? 1u : (r > CP_UNW_MAXROUNDS ? (unsigned)CP_UNW_MAXROUNDS : (unsigned)r);
 }
 
 // The record builder loops grid-stride over the records: its grid is exactly the blocks that
@@ -290,8 +340,10 @@ static int unw_staging(cp_handle* h, uint64_t n)
   CP_CUDA(h, cudaMalloc(&h->d_pdfbuf, sizeof(float4) * 4 * n));
   CP_CUDA(h, cudaMalloc(&h->d_tails, sizeof(uint4) * n));
   CP_CUDA(h, cudaMalloc(&h->d_bmask, sizeof(unsigned) * nblk));
-  CP_CUDA(h, cudaMalloc(&h->d_roff, sizeof(unsigned long long) * nrange));
-  CP_CUDA(h, cudaMalloc(&h->d_rsum, sizeof(unsigned) * nrange));
+  const uint64_t nscan = (nrange + CP_SCAN_PER - 1) / CP_SCAN_PER * CP_SCAN_PER;   // whole threads of k_unw_finish
+  CP_CUDA(h, cudaMalloc(&h->d_roff, sizeof(unsigned long long) * nscan));
+  CP_CUDA(h, cudaMalloc(&h->d_rsum, sizeof(unsigned) * nscan));
+  CP_CUDA(h, cudaMemsetAsync(h->d_rsum, 0, sizeof(unsigned) * nscan, h->stream));   // k_unw_finish leaves it zero
   h->pdfbuf_cap = n;
   return CP_OK;
 }
@@ -334,20 +386,23 @@ static bool fused_production(const cp_handle* h) { return h->flow_on && h->flow_
 
 // Enqueue one production chunk of n <= CP_UNW_CHUNK points on h->stream (no host
 // synchronisation).  Its records go to out[*base_dev ...] in point order (records at or beyond
-// `capacity` are counted, not stored) and *base_dev advances by the chunk's accepted points;
-// red_dst receives the chunk's sums.  With the flow on, flow_pre holds the flow output of the
+// `capacity` are counted, not stored) and *base_dev (taken as 0 for the pass's first chunk,
+// `first`) advances by the chunk's accepted points; red_dst receives the chunk's sums.  With the flow on, flow_pre holds the flow output of the
 // chunk's points (the caller ran the forward pass for the whole pass), or is null and the chunk
 // runs its own.  tslot >= 0 records the chunk's timing events.
 static int unweight_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t iter, cp_event* out,
                             uint64_t capacity, double* red_dst, float* scalew, unsigned long long* base_dev,
-                            const float4* flow_pre, const float* flow_u_pre, int tslot)
+                            int first, const float4* flow_pre, const float* flow_u_pre, int tslot)
 {
   if (n > CP_UNW_CHUNK) return cp_fail(h, CP_ERR_INVALID, "production chunk above CP_UNW_CHUNK points");
-  const int blocks = unw_blocks(h);
-  int rc = cp_ensure_slots(h, (size_t)blocks * CP_UNW_SLOT);
+  UnwLaunch L;
+  L.rounds = accept_rounds(h, n);
+  const uint64_t per_block = (uint64_t)L.rounds * CP_UNW_THREADS;
+  const int blocks = (int)((n + per_block - 1) / per_block);
+  // the fused flow form launches at most one block per SM
+  int rc = cp_ensure_slots(h, (size_t)(blocks > h->num_sms ? blocks : h->num_sms) * CP_UNW_SLOT);
   if (rc) return rc;
   point0 += h->point_offset;
-  UnwLaunch L;
   L.seed = h->cfg.seed; L.point0 = point0; L.n = n; L.iter = iter; L.nb = h->nb;
   L.edges = h->d_edges; L.wmax = h->d_wmax;
   L.out = reinterpret_cast<CpEventRec*>(out);
@@ -360,7 +415,6 @@ static int unweight_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t 
     rc = unw_staging(h, n);
     if (rc) return rc;
     L.pdf = h->d_pdfbuf; L.tails = h->d_tails; L.bmask = h->d_bmask; L.roff = h->d_roff; L.rsum = h->d_rsum;
-    CP_CUDA(h, cudaMemsetAsync(h->d_rsum, 0, sizeof(unsigned) * L.nrange, h->stream));
   }
   L.flow = nullptr;
   L.flow_u = nullptr;
@@ -386,16 +440,21 @@ static int unweight_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t 
     rc = cp_flow_tc_accept_enqueue(h, L, &red_blocks);
     if (rc) return rc;
   } else {
-    if (L.flow_u) k_unw_accept<true><<<blocks, CP_THREADS, 0, h->stream>>>(h->P, L);
-    else k_unw_accept<false><<<blocks, CP_THREADS, 0, h->stream>>>(h->P, L);
+    if (L.flow_u) k_unw_accept<true><<<blocks, CP_UNW_THREADS, 0, h->stream>>>(h->P, L);
+    else k_unw_accept<false><<<blocks, CP_UNW_THREADS, 0, h->stream>>>(h->P, L);
     CP_LAUNCH_CHECK(h, "k_unw_accept");
   }
   if (ev) cudaEventRecord(ev[1], h->stream);
-  k_reduce_slots<0><<<1, CP_UNW_SLOT * 32, 0, h->stream>>>(h->d_slots, red_blocks, CP_UNW_SLOT, red_dst);
-  CP_LAUNCH_CHECK(h, "k_reduce_slots");
+  // without records there are no offsets to form: the sums' block alone
+  k_unw_finish<<<capacity ? 2 : 1, 1024, 0, h->stream>>>(h->d_slots, red_blocks, red_dst,
+                                                         reinterpret_cast<uint4*>(L.rsum), L.nrange, first, base_dev,
+                                                         h->d_roff);
+  const cudaError_t fe = cudaGetLastError();
+  if (fe != cudaSuccess) {
+    h->pdfbuf_cap = 0;   // the range totals were not cleared: the next pass allocates them anew
+    return cp_fail_cuda(h, fe, "k_unw_finish");
+  }
   if (capacity) {
-    k_unw_scan<<<1, 1024, 0, h->stream>>>(h->d_rsum, L.nrange, base_dev, h->d_roff);
-    CP_LAUNCH_CHECK(h, "k_unw_scan");
     if (L.scalew) k_unw_build<true><<<build_blocks(h, true), CP_THREADS, 0, h->stream>>>(h->P, L);
     else k_unw_build<false><<<build_blocks(h, false), CP_THREADS, 0, h->stream>>>(h->P, L);
     CP_LAUNCH_CHECK(h, "k_unw_build");
@@ -465,7 +524,7 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   }
   int rc = timing_reserve(h, nsub);
   if (rc) return rc;
-  CP_CUDA(h, cudaMemsetAsync(h->d_counter, 0, sizeof(unsigned long long), h->stream));
+  if (!capacity) CP_CUDA(h, cudaMemsetAsync(h->d_counter, 0, sizeof(unsigned long long), h->stream));
   // the flow forward once for the whole pass (20 B per point: (v, ln J) and the accept draw), then the chunks; the fused form
   // runs the forward inside each chunk's accept kernel
   const bool fused = fused_production(h);
@@ -480,7 +539,7 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   }
   for (uint64_t c = 0; c < nsub; ++c) {
     const uint64_t p0 = c * CP_UNW_CHUNK, n = p0 + CP_UNW_CHUNK <= n_points ? CP_UNW_CHUNK : n_points - p0;
-    rc = unweight_enqueue(h, p0, n, iter, records_dev, capacity, h->d_unw_red + 8 * c, h->scalew, h->d_counter,
+    rc = unweight_enqueue(h, p0, n, iter, records_dev, capacity, h->d_unw_red + 8 * c, h->scalew, h->d_counter, c == 0,
                           (h->flow_on && !fused) ? h->d_flow_buf + p0 : nullptr,
                           (h->flow_on && !fused && cp_flow_writes_u(h)) ? h->d_flow_u + p0 : nullptr, (int)c);
     if (rc) return rc;
@@ -586,13 +645,12 @@ extern "C" int cp_generate_host(cp_handle* h, uint64_t n_points, uint32_t iter, 
   };
   do {
     if ((e = cudaHostGetDevicePointer((void**)&dcnt_mapped, hcnt, 0)) != cudaSuccess) break;
-    if ((e = cudaMemsetAsync(h->d_gen_cnt, 0, sizeof(unsigned long long) * nchunks, h->stream)) != cudaSuccess) break;
     for (uint64_t c = 0; c < nchunks; ++c) {
       const int b = (int)(c % CP_GEN_BUFS);
       const uint64_t p0 = c * chunk, n = (p0 + chunk <= n_points) ? chunk : n_points - p0;
       if (c >= CP_GEN_BUFS && (e = cudaStreamWaitEvent(h->stream, h->gen_copied[b], 0)) != cudaSuccess) break;
       rc = unweight_enqueue(h, p0, n, iter, h->d_gen_stage + (uint64_t)b * chunk, chunk, h->d_gen_red + 8 * c,
-                            nullptr, h->d_gen_cnt + c, nullptr, nullptr, -1);
+                            nullptr, h->d_gen_cnt + c, 1, nullptr, nullptr, -1);
       if (rc) break;
       k_gen_count<<<1, 1, 0, h->stream>>>(h->d_gen_cnt + c, dcnt_mapped + c);
       if ((e = cudaGetLastError()) != cudaSuccess) break;

@@ -7,6 +7,12 @@
 #define CP_UNW_SLOT 8   // sum w, sum w^2, max w, n_bad, n_acc, sum event weight, n_over, unused
 #define CP_UNW_CHUNK (1ull << 24)   // points per production chunk (staging: 80 B per point)
 #define CP_UNW_RANGE 32             // 32-point blocks per record-builder warp (1024 points)
+// accept blocks: 128 threads, four resident per SM (128 registers a thread; five at 96 or six at 80
+// registers measure within 2%: the FMA pipe bounds the kernel, not the warps in flight), up to 32
+// points a thread
+#define CP_UNW_THREADS 128
+#define CP_UNW_RESIDENT 4
+#define CP_UNW_MAXROUNDS 32
 
 struct UnwLaunch {
   uint64_t seed, point0, n;
@@ -24,6 +30,7 @@ struct UnwLaunch {
   float* scalew;               // per record: 6 scale-variation ratios, or null
   uint64_t capacity;
   double* slots;
+  unsigned rounds;             // points per thread of an accept block (k_unw_accept)
   const float4* flow;          // flow output (v, ln J) per in-call point, or null (K1 only)
   const float* flow_u;         // the flow forward's accept draw per in-call point, or null: K1 draws it
 };
