@@ -18,16 +18,30 @@
 int cp_flow_ensure(cp_handle* h);
 int cp_flow_repack(cp_handle* h);
 
+// Layout of the BF16 operands of the weight gradients, written by the backward pass: per coupling,
+// stages of 64 points; in a stage of F features the feature groups of 8 one after the other, each
+// its 8 core matrices (8 points x 8 features, 128 bytes: point q at (q % 8) * 16, feature f at
+// (f % 8) * 2) and 32 bytes of padding.  A warp's mma.sync fragment register is one core matrix, so
+// it stores as one contiguous 128-byte line (row-major rows of 128 bytes took eight half-used
+// sectors a store: the backward pass of 65,536 points 79.5 -> 53 us); a stage is copied into shared memory as it is, one bulk copy per operand, where
+// the core matrices are the MN-major no-swizzle operand (feature groups CP_WGT_FG apart, point
+// groups 128); and the padding puts the four feature groups that a warp adds up for the bias into
+// different banks.
+#define CP_WGT_STAGE 64                            // points per stage (four K = 16 MMAs)
+#define CP_WGT_FG (CP_WGT_STAGE * 16 + 32)         // bytes from a feature group to the next
+#define CP_WGT_BYTES(F) ((F) / 8 * CP_WGT_FG)      // bytes of a stage of F features
+
 struct FlowTrainBufs {
   float* zs;           // [B][4][3] input z of each coupling
   float4* vj;          // [B] (v0, v1, v2, ln J)
   float4* wg;          // [B] (w, d ln F / dv)
-  uint16_t* X;         // [4][B][16]  bf16 MLP inputs
-  uint16_t* H1;        // [4][B][64]  bf16 post-ReLU hidden 1
-  uint16_t* H2;        // [4][B][64]  bf16 post-ReLU hidden 2
-  uint16_t* D1;        // [4][B][64]  bf16 d pre-activation 1
-  uint16_t* D2;        // [4][B][64]  bf16 d pre-activation 2
-  uint16_t* DO;        // [4][B][16]  bf16 d outputs (s_raw, t)
+  uint64_t nst;        // stages per coupling; the arrays below are [4][nst] stages
+  uint8_t* X;          // 16 wide: bf16 MLP inputs
+  uint8_t* H1;         // 64: bf16 post-ReLU hidden 1
+  uint8_t* H2;         // 64: bf16 post-ReLU hidden 2
+  uint8_t* D1;         // 64: bf16 d pre-activation 1
+  uint8_t* D2;         // 64: bf16 d pre-activation 2
+  uint8_t* DO;         // 16: bf16 d outputs (s_raw, t)
   double* sums;        // [2] sum w, sum w^2 of the batch
   double* loss;        // per-step relative second moment
   float* gpart;        // [CP_WG_MAXBLK][CP_FLOW_NPARAM] per-block weight and bias gradients
@@ -174,21 +188,21 @@ __global__ void __launch_bounds__(128) k_flow_igrad(const CpHadParams P, const C
 // ------------------------------------------------------------------------------------------
 // 3. backward through the couplings (MLPs recomputed), writing the GEMM operands
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ void cp_store_rowfrag(uint16_t* base, int ld, uint64_t row0, uint64_t n, int gid, int tig,
-                                                 const uint32_t h[4][4])
+// writes a 16 x 64 bf16 tile held as A fragments: register (kt, 0 | 1) is the core matrix of feature
+// group 2 kt and the tile's first | second 8 points, (kt, 2 | 3) that of group 2 kt + 1.  `dst`: the
+// tile's first point group in its stage + 4 lane; ra, rb: this lane's two rows lie inside the batch
+__device__ __forceinline__ void cp_store_rowfrag(uint8_t* dst, bool ra, bool rb, const uint32_t h[4][4])
 {
-  // writes a 16 x 64 bf16 tile held as A fragments (rows row0 + gid, row0 + gid + 8)
-  const uint64_t ra = row0 + gid, rb = row0 + gid + 8;
 #pragma unroll
   for (int kt = 0; kt < 4; ++kt) {
-    const int c0 = 16 * kt + 2 * tig;
-    if (ra < n) {
-      *reinterpret_cast<uint32_t*>(base + ra * ld + c0) = h[kt][0];
-      *reinterpret_cast<uint32_t*>(base + ra * ld + c0 + 8) = h[kt][2];
+    uint8_t* d = dst + 2 * kt * CP_WGT_FG;
+    if (ra) {
+      *reinterpret_cast<uint32_t*>(d) = h[kt][0];
+      *reinterpret_cast<uint32_t*>(d + CP_WGT_FG) = h[kt][2];
     }
-    if (rb < n) {
-      *reinterpret_cast<uint32_t*>(base + rb * ld + c0) = h[kt][1];
-      *reinterpret_cast<uint32_t*>(base + rb * ld + c0 + 8) = h[kt][3];
+    if (rb) {
+      *reinterpret_cast<uint32_t*>(d + 128) = h[kt][1];
+      *reinterpret_cast<uint32_t*>(d + CP_WGT_FG + 128) = h[kt][3];
     }
   }
 }
@@ -233,19 +247,22 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
       if (active)
         for (int d = 0; d < 3; ++d) zin[d] = zs[(p * CP_FLOW_NC + c) * 3 + d];
       const float in0 = zin[k.cin[0]], in1 = k.nin > 1 ? zin[k.cin[1]] : 0.f;
-      const uint64_t off = (uint64_t)c * n;
+      const uint64_t st0 = (uint64_t)c * out.nst;
 #pragma unroll 1
       for (int tile = 0; tile < 2; ++tile) {
         const int tb = 16 * tile;
         const uint64_t row0 = base + tb;
+        const bool rowa = row0 + gid < n, rowb = row0 + gid + 8 < n;
+        // this lane's word of the tile's first core matrix in its stage (16- and 64-wide arrays)
+        const uint64_t stage = st0 + row0 / CP_WGT_STAGE;
+        const uint32_t inst = (uint32_t)(row0 % CP_WGT_STAGE) * 16u + 4u * lane;
+        const size_t at16 = stage * CP_WGT_BYTES(16) + inst, at64 = stage * CP_WGT_BYTES(64) + inst;
         // ---- recompute the MLP forward of this tile (A fragments kept for the ReLU masks)
         float r0a = __shfl_sync(0xffffffffu, in0, tb + gid), r0b = __shfl_sync(0xffffffffu, in1, tb + gid);
         float r8a = __shfl_sync(0xffffffffu, in0, tb + gid + 8), r8b = __shfl_sync(0xffffffffu, in1, tb + gid + 8);
         uint32_t a[4] = {tig == 0 ? cp_bf2(r0a, r0b) : 0u, tig == 0 ? cp_bf2(r8a, r8b) : 0u, 0u, 0u};
-        if (tig == 0) {
-          if (row0 + gid < n) *reinterpret_cast<uint32_t*>(out.X + (off + row0 + gid) * 16) = a[0];
-          if (row0 + gid + 8 < n) *reinterpret_cast<uint32_t*>(out.X + (off + row0 + gid + 8) * 16) = a[1];
-        }
+        if (rowa) *reinterpret_cast<uint32_t*>(out.X + at16) = a[0];
+        if (rowb) *reinterpret_cast<uint32_t*>(out.X + at16 + 128) = a[1];
         float acc[8][4];
         uint32_t h1[4][4], h2[4][4];
 #pragma unroll
@@ -275,8 +292,8 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
           h2[kt][2] = cp_bf2(fmaxf(acc[2 * kt + 1][0], 0.f), fmaxf(acc[2 * kt + 1][1], 0.f));
           h2[kt][3] = cp_bf2(fmaxf(acc[2 * kt + 1][2], 0.f), fmaxf(acc[2 * kt + 1][3], 0.f));
         }
-        cp_store_rowfrag(out.H1 + off * 64, 64, row0, n, gid, tig, h1);
-        cp_store_rowfrag(out.H2 + off * 64, 64, row0, n, gid, tig, h2);
+        cp_store_rowfrag(out.H1 + at64, rowa, rowb, h1);
+        cp_store_rowfrag(out.H2 + at64, rowa, rowb, h2);
         float c3[4] = {b[128 + 2 * tig], b[128 + 2 * tig + 1], b[128 + 2 * tig], b[128 + 2 * tig + 1]};
 #pragma unroll
         for (int kt = 0; kt < 4; ++kt) cp_mma_bf16(c3, h2[kt], pk[CP_FLOW_P_W3 + kt * 32 + lane]);
@@ -315,10 +332,8 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
         const bool odd = tig & 1;
         uint32_t ad[4] = {tig < 2 ? cp_bf2(odd ? g0[2] : g0[0], odd ? g0[3] : g0[1]) : 0u,
                           tig < 2 ? cp_bf2(odd ? g8[2] : g8[0], odd ? g8[3] : g8[1]) : 0u, 0u, 0u};
-        if (tig < 2) {
-          if (row0 + gid < n) *reinterpret_cast<uint32_t*>(out.DO + (off + row0 + gid) * 16 + 2 * tig) = ad[0];
-          if (row0 + gid + 8 < n) *reinterpret_cast<uint32_t*>(out.DO + (off + row0 + gid + 8) * 16 + 2 * tig) = ad[1];
-        }
+        if (rowa) *reinterpret_cast<uint32_t*>(out.DO + at16) = ad[0];
+        if (rowb) *reinterpret_cast<uint32_t*>(out.DO + at16 + 128) = ad[1];
         // dH2 = dO W3^T, masked by the ReLU of layer 2
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
@@ -338,7 +353,7 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
           d2[kt][2] = cp_bf2(acc[2 * kt + 1][0], acc[2 * kt + 1][1]);
           d2[kt][3] = cp_bf2(acc[2 * kt + 1][2], acc[2 * kt + 1][3]);
         }
-        cp_store_rowfrag(out.D2 + off * 64, 64, row0, n, gid, tig, d2);
+        cp_store_rowfrag(out.D2 + at64, rowa, rowb, d2);
         // dH1 = dH2 W2^T, masked by the ReLU of layer 1
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
@@ -359,7 +374,7 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
           d1[kt][2] = cp_bf2(acc[2 * kt + 1][0], acc[2 * kt + 1][1]);
           d1[kt][3] = cp_bf2(acc[2 * kt + 1][2], acc[2 * kt + 1][3]);
         }
-        cp_store_rowfrag(out.D1 + off * 64, 64, row0, n, gid, tig, d1);
+        cp_store_rowfrag(out.D1 + at64, rowa, rowb, d1);
         // dX = dH1 W1^T: columns 0..1 are the gradients of the two input features
         float cx[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -381,7 +396,7 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
 // 4. weight and bias gradients of one layer shape for all couplings (blockIdx.y = coupling):
 //    block b's chunk of points gives G_b[M][N] = sum_p A[p][0:M]^T B[p][0:N] on the tensor cores
 //    and the bias gradient Gb_b[N] = sum_p B[p][0:N] from the same staged tiles, stored into its
-//    own slot of the partial buffer (A, B bf16 row-major with leading dims M and N; M in {16, 64},
+//    own slot of the partial buffer (A, B bf16 in the stage layout above; M in {16, 64},
 //    N in {16, 64}); k_flow_gsum then adds the slots in block order, so a training run is
 //    reproducible bit for bit (no floating-point atomics).
 // ------------------------------------------------------------------------------------------
@@ -392,12 +407,19 @@ __device__ __forceinline__ void cp_ldsm_x4_t(uint32_t r[4], const void* p)
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 
+// byte offset of (point p, feature f) in a coupling's operand of F features
+template <int F>
+__device__ __forceinline__ size_t cp_wgt_at(uint64_t p, int f)
+{
+  return p / CP_WGT_STAGE * CP_WGT_BYTES(F) + (size_t)((f >> 3) * CP_WGT_FG + (int)(p % CP_WGT_STAGE) * 16 + (f & 7) * 2);
+}
+
 #define CP_WG_ROWS 64   // points staged per iteration
 #define CP_WG_MAXBLK 64 // blocks per coupling and layer (the batch is cut into at most this many chunks)
 
 template <int M, int N>
-__global__ void __launch_bounds__(128) k_flow_wgrad(const uint16_t* __restrict__ A0, const uint16_t* __restrict__ B0,
-                                                    uint64_t n, float* __restrict__ part, int goff, int ldg, int nvalid,
+__global__ void __launch_bounds__(128) k_flow_wgrad(const uint8_t* __restrict__ A0, const uint8_t* __restrict__ B0,
+                                                    uint64_t nst, uint64_t n, float* __restrict__ part, int goff, int ldg, int nvalid,
                                                     int chunk, int bias_rel)
 {
   constexpr int MT = M / 16, NT = N / 8, TPW = (MT * NT + 3) / 4;
@@ -405,8 +427,8 @@ __global__ void __launch_bounds__(128) k_flow_wgrad(const uint16_t* __restrict__
   __shared__ __align__(16) uint16_t sB[CP_WG_ROWS * N];
   __shared__ float sBias[128];
   const int c = blockIdx.y;
-  const uint16_t* A = A0 + (uint64_t)c * n * M;
-  const uint16_t* B = B0 + (uint64_t)c * n * N;
+  const uint8_t* A = A0 + (uint64_t)c * nst * CP_WGT_BYTES(M);
+  const uint8_t* B = B0 + (uint64_t)c * nst * CP_WGT_BYTES(N);
   float* G = part + (size_t)blockIdx.x * CP_FLOW_NPARAM + c * CP_FLOW_PER + goff;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   const int mi = lane >> 3, rw = lane & 7;
@@ -421,13 +443,13 @@ __global__ void __launch_bounds__(128) k_flow_wgrad(const uint16_t* __restrict__
     for (int e = threadIdx.x; e < CP_WG_ROWS * M / 8; e += blockDim.x) {
       const int row = e / (M / 8), col = (e % (M / 8)) * 8;
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (p0 + row < p_end) v = *reinterpret_cast<const uint4*>(A + (p0 + row) * M + col);
+      if (p0 + row < p_end) v = *reinterpret_cast<const uint4*>(A + cp_wgt_at<M>(p0 + row, col));
       *reinterpret_cast<uint4*>(&sA[row * M + col]) = v;
     }
     for (int e = threadIdx.x; e < CP_WG_ROWS * N / 8; e += blockDim.x) {
       const int row = e / (N / 8), col = (e % (N / 8)) * 8;
       uint4 v = make_uint4(0, 0, 0, 0);
-      if (p0 + row < p_end) v = *reinterpret_cast<const uint4*>(B + (p0 + row) * N + col);
+      if (p0 + row < p_end) v = *reinterpret_cast<const uint4*>(B + cp_wgt_at<N>(p0 + row, col));
       *reinterpret_cast<uint4*>(&sB[row * N + col]) = v;
     }
     __syncthreads();
@@ -482,115 +504,101 @@ __global__ void __launch_bounds__(128) k_flow_wgrad(const uint16_t* __restrict__
 //       layer 0: dW1^T[n][k] = sum_p D1[p][n] X[p][k]    M = 64 (n), N = 16 (k), bias b1 = sum D1
 //       layer 1: dW2[k][n]   = sum_p H1[p][k] D2[p][n]   M = 64 (k), N = 64 (n), bias b2 = sum D2
 //       layer 2: dW3[k][n]   = sum_p H2[p][k] DO[p][n]   M = 64 (k), N = 16 (n), bias b3 = sum DO
-//     so D[M][N] += A[M][K] B[N][K]^T with K = the block's points, 64 per stage: A and B are the
-//     row-major [point][feature] arrays read as MN-major operands (features contiguous).  Shared
-//     memory holds them in the no-swizzle MN-major canonical layout: core matrices of 8 features
-//     (16 bytes) x 8 points, 128 bytes; element (feature f, point q) of a stage at
-//     (q / 8) * (F / 8) * 128 + (f / 8) * 128 + (q % 8) * 16 + (f % 8) * 2, so the descriptor's
-//     stride in the feature direction (SBO) is 128 bytes and in the point direction (LBO)
-//     (F / 8) * 128.  Stages are copied with cp.async (16-byte chunks, zero fill past the chunk's
-//     end) into two buffers; one thread issues a stage's four K = 16 MMAs and commits them to the
-//     buffer's mbarrier, which every thread waits on (bounded) before the buffer is refilled.  The
-//     M = 64 accumulator occupies TMEM lanes 0-15 of each 32-lane quarter (row r in lane
-//     r % 16 + 32 (r / 16)), so thread t < 16 of warp w reads row 16 w + t.  Each block writes its
+//     so D[M][N] += A[M][K] B[N][K]^T with K = the block's points, 64 per stage, both operands
+//     MN-major (features contiguous) in the stage layout: the descriptor's stride in the feature
+//     direction (SBO) is CP_WGT_FG and in the point direction (LBO) 128 bytes.  Thread 0 fetches each
+//     stage with one bulk copy per operand (two stages in flight), issues its four K = 16 MMAs and
+//     commits them; warps 2 and 3 add up the bias columns from the same stage; a stage's buffer is
+//     refilled once its `empty` barrier has the commit and those two warps' arrivals.  Every wait is
+//     bounded.  The M = 64 accumulator occupies TMEM lanes 0-15 of each 32-lane quarter (row r in
+//     lane r % 16 + 32 (r / 16)), so thread t < 16 of warp w reads row 16 w + t.  Each block writes its
 //     own slot of the partial buffer; k_flow_gsum adds the slots in block order.
+//
+//     What bounds it is reading the operands, 151 MB per 65,536 points, mostly from L2 where the
+//     backward pass left them.  34 KB of stages let six blocks reside on an SM, so all 768 of a batch
+//     run at once (five before, with 28 blocks left for a second wave):
+//     71 -> 33 us per 65,536 points.
 // ------------------------------------------------------------------------------------------
-#define CP_WGT_STAGE 64   // points per stage (four K = 16 MMAs)
-
-__device__ __forceinline__ void cp_cp_async16(uint32_t dst, const void* src, bool valid)
-{
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// one stage of F-wide rows [q0, q0 + 64) of X (row-major, leading dim F) into the MN-major layout
-template <int F>
-__device__ __forceinline__ void cp_wgt_stage_load(uint32_t sdst, const uint16_t* __restrict__ X, uint64_t q0,
-                                                  uint64_t q_end)
-{
-  constexpr int CH = CP_WGT_STAGE * F / 8;   // 16-byte chunks
-  for (int e = threadIdx.x; e < CH; e += blockDim.x) {
-    // e = (point group, feature group, point within group): consecutive threads fill a core
-    // matrix's consecutive 16-byte rows
-    const int qg = e / (F / 8 * 8), fg = (e / 8) % (F / 8), r = e % 8;
-    const uint64_t q = q0 + qg * 8 + r;
-    const bool ok = q < q_end;
-    cp_cp_async16(sdst + (uint32_t)e * 16u, X + (ok ? q : q0) * F + fg * 8, ok);
+// two bias columns (a pair of features) and one residue class of the stage's points per thread of
+// warps 2 and 3: 64 features x 2 residues, 16 features x 8; `res`: points res, res + step, ...
+struct CpWgtBias {
+  int fg, w, res, step;
+  float lo = 0.f, hi = 0.f;
+  __device__ __forceinline__ CpWgtBias(int width, int t)   // t in [0, 64)
+  {
+    w = t & 3;
+    if (width == 64) { res = (t >> 2) & 1; fg = t >> 3; step = 2; }
+    else { res = (t >> 2) & 7; fg = t >> 5; step = 8; }
   }
-}
-
-__device__ __forceinline__ float cp_wgt_elem(const uint8_t* s, int F, int f, int q)
-{
-  const uint16_t v = *reinterpret_cast<const uint16_t*>(s + (q / 8) * (F / 8) * 128 + (f / 8) * 128 + (q % 8) * 16 + (f % 8) * 2);
-  return __uint_as_float((uint32_t)v << 16);
-}
+  __device__ __forceinline__ void add(const uint8_t* s)   // a stage's shared-memory copy
+  {
+    const uint8_t* at = s + fg * CP_WGT_FG + 4 * w;
+    for (int q = res; q < CP_WGT_STAGE; q += step) {
+      const uint32_t v = *reinterpret_cast<const uint32_t*>(at + 16 * q);
+      lo += __uint_as_float(v << 16);
+      hi += __uint_as_float(v & 0xffff0000u);
+    }
+  }
+};
 
 template <int NB>
-__device__ __forceinline__ void cp_wgt_layer(const uint16_t* __restrict__ A, const uint16_t* __restrict__ B, bool bias_of_a,
-                                             uint64_t p_begin, uint64_t p_end, float* __restrict__ G, int layer,
-                                             uint8_t* smem, uint32_t tmem, uint32_t mbar0, float* sBias,
+__device__ __forceinline__ void cp_wgt_layer(const uint8_t* __restrict__ A, const uint8_t* __restrict__ B, bool bias_of_a,
+                                             uint64_t st_begin, uint64_t st_end, float* __restrict__ G, int layer,
+                                             uint8_t* smem, uint32_t tmem, uint32_t mbar, float* sBias,
                                              int* __restrict__ status)
 {
-  constexpr int ABYTES = CP_WGT_STAGE * 64 * 2, BBYTES = CP_WGT_STAGE * NB * 2;
+  constexpr uint32_t AB = CP_WGT_BYTES(64), BB = CP_WGT_BYTES(NB);
   const uint32_t sbase = cp_smem_u32(smem);
-  const uint32_t sA[2] = {sbase, sbase + ABYTES}, sB[2] = {sbase + 2 * ABYTES, sbase + 2 * ABYTES + BBYTES};
+  // barriers: full[0..1] (bulk copies landed), empty[0..1] (MMAs and bias reads done), all MMAs, drain
+  const uint32_t full = mbar, empty = mbar + 16, done = mbar + 32, drain = mbar + 40;
   const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(NB >> 3) << 17) |
                          ((uint32_t)(64 >> 4) << 24);
-  const int nst = (int)((p_end - p_begin + CP_WGT_STAGE - 1) / CP_WGT_STAGE);
-  const int tid = threadIdx.x;
-  // bias column of this thread and its share of a stage's points (fixed order)
-  constexpr int BW = 64;   // the bias side is 64 wide for layer 0 (A = D1), NB wide otherwise
-  const int bw = bias_of_a ? BW : NB;
-  const int bcol = tid % bw, bsplit = 128 / bw, brow0 = tid / bw;
-  float bsum = 0.f;
-  uint32_t phase[2] = {0u, 0u};
+  const int nst = (int)(st_end - st_begin), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   volatile int abort_flag = 0;
   bool ok = true;
-  cp_wgt_stage_load<64>(sA[0], A, p_begin, p_end);
-  cp_wgt_stage_load<NB>(sB[0], B, p_begin, p_end);
-  cp_cp_async_commit();
-  for (int st = 0; st < nst; ++st) {
-    const int b = st & 1;
-    if (st + 1 < nst) {
-      // the other buffer was read by stage st - 1's MMAs: wait for their commit before refilling
-      if (st >= 1) {
-        ok = ok && cp_mbar_wait_bounded(mbar0 + 8 * (1 - b), phase[1 - b], &abort_flag);
-        phase[1 - b] ^= 1u;
-      }
-      const uint64_t q0 = p_begin + (uint64_t)(st + 1) * CP_WGT_STAGE;
-      cp_wgt_stage_load<64>(sA[1 - b], A, q0, p_end);
-      cp_wgt_stage_load<NB>(sB[1 - b], B, q0, p_end);
-      cp_cp_async_commit();
-      cp_cp_async_wait<1>();
-    } else {
-      cp_cp_async_wait<0>();
-    }
-    cp_fence_proxy_async();
-    __syncthreads();
-    {
-      const uint8_t* sb = smem + (bias_of_a ? (b ? ABYTES : 0) : 2 * ABYTES + (b ? BBYTES : 0));
-      for (int q = brow0; q < CP_WGT_STAGE; q += bsplit) bsum += cp_wgt_elem(sb, bias_of_a ? 64 : NB, bcol, q);
-    }
-    if (tid == 0 && ok) {
+  CpWgtBias bias(bias_of_a ? 64 : NB, tid & 63);
+  if (tid == 0) {
+    auto fetch = [&](int st) {
+      const int b = st & 1;
+      cp_mbar_expect_tx(full + 8 * b, AB + BB);
+      cp_bulk_load(sbase + b * AB, A + (st_begin + st) * AB, AB, full + 8 * b);
+      cp_bulk_load(sbase + 2 * AB + b * BB, B + (st_begin + st) * BB, BB, full + 8 * b);
+    };
+    int fetched = 0;
+    for (; fetched < nst && fetched < 2; ++fetched) fetch(fetched);
+    int st = 0;
+    for (; st < nst; ++st) {
+      const int b = st & 1;
+      if (!(ok = cp_mbar_wait_bounded(full + 8 * b, (st >> 1) & 1, &abort_flag))) break;
       cp_tc_fence_after();
 #pragma unroll
       for (int k = 0; k < CP_WGT_STAGE / 16; ++k) {
-        // K = 16 points = two point groups: +2 groups of (F / 8) core matrices
-        const uint64_t da = cp_tc_desc(sA[b] + k * 2 * (64 / 8) * 128, (64 / 8) * 128, 128);
-        const uint64_t db = cp_tc_desc(sB[b] + k * 2 * (NB / 8) * 128, (NB / 8) * 128, 128);
+        const uint64_t da = cp_tc_desc(sbase + b * AB + k * 256, 128, CP_WGT_FG);   // K = 16: two point groups
+        const uint64_t db = cp_tc_desc(sbase + 2 * AB + b * BB + k * 256, 128, CP_WGT_FG);
         cp_tc_mma(tmem, da, db, idesc, (st > 0 || k > 0) ? 1u : 0u);
       }
-      cp_tc_commit(mbar0 + 8 * b);
-    } else if (tid == 0) {
-      cp_tc_commit(mbar0 + 8 * b);   // nothing issued: the barrier still completes its phase
+      cp_tc_commit(empty + 8 * b);
+      if (fetched < nst) {
+        if (!(ok = cp_mbar_wait_bounded(empty + 8 * b, (st >> 1) & 1, &abort_flag))) break;
+        fetch(fetched++);
+      }
+    }
+    cp_tc_commit(done);
+    if (!ok) {   // the copies in flight land before the shared memory is given up
+      volatile int drain_abort = 0;
+      for (int f = st; f < fetched; ++f) cp_mbar_wait_bounded(full + 8 * (f & 1), (f >> 1) & 1, &drain_abort);
+    }
+  } else if (warp >= 2) {
+    for (int st = 0; st < nst; ++st) {
+      const int b = st & 1;
+      if (!(ok = cp_mbar_wait_bounded(full + 8 * b, (st >> 1) & 1, &abort_flag))) break;
+      bias.add(smem + (bias_of_a ? b * AB : 2 * AB + b * BB));
+      __syncwarp();
+      if (lane == 0) cp_mbar_arrive(empty + 8 * b);
     }
   }
-  // the last stage's MMAs (and, in order, every earlier one) have completed
-  const int bl = (nst - 1) & 1;
-  ok = ok && cp_mbar_wait_bounded(mbar0 + 8 * bl, phase[bl], &abort_flag);
-  if (nst >= 2) ok = ok && cp_mbar_wait_bounded(mbar0 + 8 * (1 - bl), phase[1 - bl], &abort_flag);
+  __syncwarp();
+  ok = cp_mbar_wait_bounded(done, 0u, &abort_flag) && ok;
   cp_tc_fence_after();
   ok = __syncthreads_and(ok) != 0;
   if (!ok) {
@@ -598,15 +606,15 @@ __device__ __forceinline__ void cp_wgt_layer(const uint16_t* __restrict__ A, con
     // complete (a fresh barrier, bounded wait)
     if (tid == 0) {
       atomicOr(status, 2);
-      cp_tc_commit(mbar0 + 16);
+      cp_tc_commit(drain);
       volatile int drain_abort = 0;
-      cp_mbar_wait_bounded(mbar0 + 16, 0u, &drain_abort);
+      cp_mbar_wait_bounded(drain, 0u, &drain_abort);
     }
     __syncthreads();
     return;
   }
   // accumulator: warp w, lane t < 16 = row 16 w + t
-  const int warp = tid >> 5, lane = tid & 31, row = 16 * warp + lane;
+  const int row = 16 * warp + lane;
   const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16);
 #pragma unroll
   for (int half = 0; half < NB / 16; half += 2) {
@@ -633,28 +641,33 @@ __device__ __forceinline__ void cp_wgt_layer(const uint16_t* __restrict__ A, con
       }
     }
   }
-  // bias: the bsplit threads of a column add their sums in thread order
-  sBias[tid] = bsum;
+  // bias: the residue classes of a column added in order (a column's points res, res + step, ...
+  // form one running sum, so the sums are those of 128 / width threads a column)
+  const int bw = bias_of_a ? 64 : NB;
+  if (warp >= 2) {
+    const int col = bias.fg * 8 + 2 * bias.w;
+    sBias[bias.res * bw + col] = bias.lo;
+    sBias[bias.res * bw + col + 1] = bias.hi;
+  }
   __syncthreads();
   const int nb_valid = layer == 2 ? 8 : 64;
   if (tid < bw && tid < nb_valid) {
     float acc = 0.f;
-    for (int r = 0; r < bsplit; ++r) acc += sBias[r * bw + tid];
+    for (int r = 0; r < 128 / bw; ++r) acc += sBias[r * bw + tid];
     G[(layer == 0 ? CP_FLOW_B1 : (layer == 1 ? CP_FLOW_B2 : CP_FLOW_B3)) + tid] = acc;
   }
 }
 
 __global__ void __launch_bounds__(128) k_flow_wgrad_tc(FlowTrainBufs t, uint64_t n, int chunk, int* __restrict__ status)
 {
-  // two A and two B stage buffers (32 KB), plus 8 KB so that the operand ranges of every
-  // descriptor stay inside this array whichever of its two strides a layout reading applies
-  __shared__ __align__(1024) uint8_t smem[2 * (CP_WGT_STAGE * 64 * 2) + 2 * (CP_WGT_STAGE * 64 * 2) + 8192];
+  __shared__ __align__(1024) uint8_t smem[4 * CP_WGT_BYTES(64)];   // two A and two B stages
   __shared__ float sBias[128];
-  __shared__ __align__(8) uint64_t mbar[3];   // the two stage buffers' MMA commits, the drain
+  __shared__ __align__(8) uint64_t mbar[6];
   __shared__ uint32_t tmem_slot;
   const int c = blockIdx.y, layer = blockIdx.z, tid = threadIdx.x;
   if (tid == 0) {
-    for (int i = 0; i < 3; ++i) cp_mbar_init(cp_smem_u32(&mbar[i]), 1);
+    // full: the fetching thread's arrival (and the copies' bytes); empty: the MMAs' commit and warps 2, 3
+    for (int i = 0; i < 6; ++i) cp_mbar_init(cp_smem_u32(&mbar[i]), i == 2 || i == 3 ? 3 : 1);
     cp_mbar_init_fence();
   }
   if ((tid >> 5) == 0) {
@@ -665,18 +678,16 @@ __global__ void __launch_bounds__(128) k_flow_wgrad_tc(FlowTrainBufs t, uint64_t
   __syncthreads();
   cp_tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const uint64_t p_begin = (uint64_t)blockIdx.x * chunk;
-  const uint64_t p_end = p_begin + chunk < n ? p_begin + chunk : n;
+  // chunk is a whole number of stages; rows beyond n of the last one are zero
+  const uint64_t sb = (uint64_t)blockIdx.x * (chunk / CP_WGT_STAGE);
+  const uint64_t se = sb + chunk / CP_WGT_STAGE < t.nst ? sb + chunk / CP_WGT_STAGE : t.nst;
   float* G = t.gpart + (size_t)blockIdx.x * CP_FLOW_NPARAM + c * CP_FLOW_PER;
-  const uint64_t off = (uint64_t)c * n;
+  const size_t o16 = (size_t)c * t.nst * CP_WGT_BYTES(16), o64 = (size_t)c * t.nst * CP_WGT_BYTES(64);
   const uint32_t mb = cp_smem_u32(&mbar[0]);
-  if (p_begin < p_end) {
-    if (layer == 0)
-      cp_wgt_layer<16>(t.D1 + off * 64, t.X + off * 16, true, p_begin, p_end, G, 0, smem, tmem, mb, sBias, status);
-    else if (layer == 1)
-      cp_wgt_layer<64>(t.H1 + off * 64, t.D2 + off * 64, false, p_begin, p_end, G, 1, smem, tmem, mb, sBias, status);
-    else
-      cp_wgt_layer<16>(t.H2 + off * 64, t.DO + off * 16, false, p_begin, p_end, G, 2, smem, tmem, mb, sBias, status);
+  if (sb < se) {
+    if (layer == 0) cp_wgt_layer<16>(t.D1 + o64, t.X + o16, true, sb, se, G, 0, smem, tmem, mb, sBias, status);
+    else if (layer == 1) cp_wgt_layer<64>(t.H1 + o64, t.D2 + o64, false, sb, se, G, 1, smem, tmem, mb, sBias, status);
+    else cp_wgt_layer<16>(t.H2 + o64, t.DO + o16, false, sb, se, G, 2, smem, tmem, mb, sBias, status);
   }
   cp_tc_fence_before();
   __syncthreads();
@@ -757,30 +768,37 @@ __global__ void k_flow_batch_loss(const double* moments, double n, double* sums,
 // ------------------------------------------------------------------------------------------
 // host
 // ------------------------------------------------------------------------------------------
-static size_t train_bytes(uint64_t B)
+// The training buffers of B points, one after the other at multiples of 256 bytes; with base = null
+// only their total size.
+static size_t carve(void* base, uint64_t B, FlowTrainBufs& t)
 {
-  return B * (sizeof(float) * 12 + sizeof(float4) * 2 + 2 * CP_FLOW_NC * (16 + 64 * 4 + 16)) + 4096 +
-         sizeof(float) * CP_WG_MAXBLK * CP_FLOW_NPARAM;
+  size_t at = 0;
+  const auto take = [&](size_t bytes) {
+    uint8_t* q = static_cast<uint8_t*>(base) + at;
+    at += (bytes + 255) & ~(size_t)255;
+    return q;
+  };
+  t.nst = (B + CP_WGT_STAGE - 1) / CP_WGT_STAGE;
+  const size_t w16 = CP_FLOW_NC * t.nst * CP_WGT_BYTES(16), w64 = CP_FLOW_NC * t.nst * CP_WGT_BYTES(64);
+  t.vj = reinterpret_cast<float4*>(take(sizeof(float4) * B));
+  t.wg = reinterpret_cast<float4*>(take(sizeof(float4) * B));
+  t.zs = reinterpret_cast<float*>(take(sizeof(float) * 12 * B));
+  t.X = take(w16);
+  t.H1 = take(w64);
+  t.H2 = take(w64);
+  t.D1 = take(w64);
+  t.D2 = take(w64);
+  t.DO = take(w16);
+  t.sums = reinterpret_cast<double*>(take(2 * sizeof(double)));
+  t.loss = reinterpret_cast<double*>(take(sizeof(double)));
+  t.gpart = reinterpret_cast<float*>(take(sizeof(float) * CP_WG_MAXBLK * CP_FLOW_NPARAM));
+  return at;
 }
 
-static FlowTrainBufs carve(void* base, uint64_t B)
+static size_t train_bytes(uint64_t B)
 {
-  char* q = static_cast<char*>(base);
   FlowTrainBufs t;
-  t.vj = reinterpret_cast<float4*>(q); q += sizeof(float4) * B;
-  t.wg = reinterpret_cast<float4*>(q); q += sizeof(float4) * B;
-  t.zs = reinterpret_cast<float*>(q); q += sizeof(float) * 12 * B;
-  t.X = reinterpret_cast<uint16_t*>(q); q += 2 * CP_FLOW_NC * 16 * B;
-  t.H1 = reinterpret_cast<uint16_t*>(q); q += 2 * CP_FLOW_NC * 64 * B;
-  t.H2 = reinterpret_cast<uint16_t*>(q); q += 2 * CP_FLOW_NC * 64 * B;
-  t.D1 = reinterpret_cast<uint16_t*>(q); q += 2 * CP_FLOW_NC * 64 * B;
-  t.D2 = reinterpret_cast<uint16_t*>(q); q += 2 * CP_FLOW_NC * 64 * B;
-  t.DO = reinterpret_cast<uint16_t*>(q); q += 2 * CP_FLOW_NC * 16 * B;
-  q = reinterpret_cast<char*>(((uintptr_t)q + 255) & ~(uintptr_t)255);
-  t.sums = reinterpret_cast<double*>(q); q += 64;
-  t.loss = reinterpret_cast<double*>(q); q += 64;
-  t.gpart = reinterpret_cast<float*>(q);
-  return t;
+  return carve(nullptr, B, t);
 }
 
 static size_t bwd_smem() { return sizeof(uint2) * CP_FLOW_NC * CP_FLOW_P_PER + sizeof(float) * CP_FLOW_NC * CP_FLOW_NB; }
@@ -804,7 +822,7 @@ static int train_buffers(cp_handle* h, uint64_t count, FlowTrainBufs& t)
   }
   if (count != h->ftrain_count) CP_CUDA(h, cudaMemsetAsync(h->d_ftrain, 0, train_bytes(count), h->stream));
   h->ftrain_count = count;
-  t = carve(h->d_ftrain, count);
+  carve(h->d_ftrain, count, t);
   // per-device attributes: set on every use (host-side, cheap)
   CP_CUDA(h, cudaFuncSetAttribute(k_flow_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem()));
   CP_CUDA(h, cudaFuncSetAttribute(k_flow_fwd_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fwd_smem()));
@@ -867,12 +885,12 @@ static int flow_phase_gradient(cp_handle* h, const FlowTrainBufs& t, uint64_t co
   } else {
     // warp-level mma.sync, one launch per layer shape (the cross-check path)
     const dim3 grid((unsigned)nblk, CP_FLOW_NC);
-    k_flow_wgrad<16, 64><<<grid, 128, 0, h->stream>>>(t.X, t.D1, count, t.gpart, CP_FLOW_W1, 64, 64, (int)chunk,
+    k_flow_wgrad<16, 64><<<grid, 128, 0, h->stream>>>(t.X, t.D1, t.nst, count, t.gpart, CP_FLOW_W1, 64, 64, (int)chunk,
                                                       CP_FLOW_B1 - CP_FLOW_W1);
-    k_flow_wgrad<64, 64><<<grid, 128, 0, h->stream>>>(t.H1, t.D2, count, t.gpart, CP_FLOW_W2, 64, 64, (int)chunk,
+    k_flow_wgrad<64, 64><<<grid, 128, 0, h->stream>>>(t.H1, t.D2, t.nst, count, t.gpart, CP_FLOW_W2, 64, 64, (int)chunk,
                                                       CP_FLOW_B2 - CP_FLOW_W2);
     // W3 [64][8] from the 16-wide output-gradient rows (columns 8..15 are zero padding)
-    k_flow_wgrad<64, 16><<<grid, 128, 0, h->stream>>>(t.H2, t.DO, count, t.gpart, CP_FLOW_W3, 8, 8, (int)chunk,
+    k_flow_wgrad<64, 16><<<grid, 128, 0, h->stream>>>(t.H2, t.DO, t.nst, count, t.gpart, CP_FLOW_W3, 8, 8, (int)chunk,
                                                       CP_FLOW_B3 - CP_FLOW_W3);
     CP_LAUNCH_CHECK(h, "k_flow_wgrad");
   }
@@ -1004,7 +1022,8 @@ extern "C" int cp_flow_step_gradient(cp_handle* h, const double* moments_dev, ui
   CP_CHECK_HANDLE(h);
   if (!h->d_ftrain || !h->ftrain_count || !moments_dev || batch_total < h->ftrain_count)
     return cp_fail(h, CP_ERR_INVALID, "cp_flow_step_gradient: call cp_flow_step_moments first (batch_total >= count)");
-  FlowTrainBufs t = carve(h->d_ftrain, h->ftrain_count);
+  FlowTrainBufs t;
+  carve(h->d_ftrain, h->ftrain_count, t);
   int rc = flow_phase_gradient(h, t, h->ftrain_count, moments_dev, batch_total, t.loss);
   if (rc) return rc;
   if (grad_dev)

@@ -138,6 +138,19 @@ __device__ __forceinline__ void cp_mbar_arrive(uint32_t mbar)
 {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
+// one arrival that also adds `bytes` to what the current phase waits for from bulk copies
+__device__ __forceinline__ void cp_mbar_expect_tx(uint32_t mbar, uint32_t bytes)
+{
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+// `bytes` (a multiple of 16) from global to this CTA's shared memory, both 16-byte aligned; the
+// mbarrier counts them as they land
+__device__ __forceinline__ void cp_bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar)
+{
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(mbar)
+               : "memory");
+}
 // non-blocking test of the phase `parity` of an mbarrier
 __device__ __forceinline__ bool cp_mbar_test(uint32_t mbar, uint32_t parity)
 {
