@@ -37,13 +37,28 @@ int cp_ensure_slots(cp_handle* h, size_t doubles)
 int cp_ensure_iters(cp_handle* h, int n)
 {
   if (n <= h->iters_cap) return CP_OK;
-  if (h->d_iters) {
+  if (h->h_iters) {
     CP_CUDA(h, cudaStreamSynchronize(h->stream));
-    CP_CUDA(h, cudaFree(h->d_iters));
-    h->d_iters = nullptr;
+    CP_CUDA(h, cudaFreeHost(h->h_iters));
+    h->h_iters = nullptr;
+    h->iters_cap = 0;
   }
-  CP_CUDA(h, cudaMalloc(&h->d_iters, sizeof(CpIterDev) * (size_t)n));
+  CP_CUDA(h, cudaHostAlloc(&h->h_iters, sizeof(CpIterDev) * (size_t)n, cudaHostAllocMapped | cudaHostAllocPortable));
   h->iters_cap = n;
+  return CP_OK;
+}
+
+int cp_ensure_losses(cp_handle* h, int n)
+{
+  if (n <= h->losses_cap) return CP_OK;
+  if (h->h_losses) {
+    CP_CUDA(h, cudaStreamSynchronize(h->stream));
+    CP_CUDA(h, cudaFreeHost(h->h_losses));
+    h->h_losses = nullptr;
+    h->losses_cap = 0;
+  }
+  CP_CUDA(h, cudaHostAlloc(&h->h_losses, sizeof(double) * (size_t)n, cudaHostAllocMapped | cudaHostAllocPortable));
+  h->losses_cap = n;
   return CP_OK;
 }
 
@@ -120,7 +135,8 @@ extern "C" int cp_create(const cp_config* cfg, cp_handle** out)
   int cur = -1;
   if (cudaGetDevice(&cur) != cudaSuccess || cur != h->device) { delete h; return CP_ERR_CUDA; }
   cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, h->device);
-  bool ok = cudaMalloc(&h->d_edges, sizeof(double) * 3 * (CP_MAX_BINS + 1)) == cudaSuccess &&
+  bool ok = cudaHostAlloc(&h->mail, sizeof(CpMail), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess &&
+            cudaMalloc(&h->d_edges, sizeof(double) * 3 * (CP_MAX_BINS + 1)) == cudaSuccess &&
             cudaMalloc(&h->d_red, sizeof(double) * (CP_SLOT_HEAD + 3 * CP_MAX_BINS)) == cudaSuccess &&
             cudaMalloc(&h->d_qhist, sizeof(unsigned long long) * CP_QBINS) == cudaSuccess &&
             cudaMalloc(&h->d_wmax, sizeof(double) * 2) == cudaSuccess &&
@@ -130,6 +146,7 @@ extern "C" int cp_create(const cp_config* cfg, cp_handle** out)
             cudaMemset(h->d_ticket, 0, sizeof(unsigned)) == cudaSuccess &&
             cudaMalloc(&h->d_cteq, sizeof(CpCteqPoly) * 8) == cudaSuccess &&
             cudaMemcpy(h->d_cteq, h->P.cteq, sizeof(CpCteqPoly) * 8, cudaMemcpyHostToDevice) == cudaSuccess;
+  if (h->mail) memset(h->mail, 0, sizeof(CpMail));
   if (!ok || cp_had_launch_shape(h) != CP_OK || cp_ensure_iters(h, 16) != CP_OK) {
     cp_destroy(h);
     return CP_ERR_NOMEM;
@@ -152,12 +169,14 @@ extern "C" int cp_destroy(cp_handle* h)
     if (h->gen_copied[k]) cudaEventDestroy(h->gen_copied[k]);
   }
   if (h->gen_copy) cudaStreamDestroy(h->gen_copy);
-  if (h->h_gen_cnt) cudaFreeHost(h->h_gen_cnt);
-  void* bufs[] = {h->d_edges, h->d_slots, h->d_red, h->d_iters, h->d_x1, h->d_x2, h->d_sH,
+  void* pinned[] = {h->h_gen_cnt, h->h_gen_red, h->h_unw_red, h->h_iters, h->h_losses, h->mail};
+  for (void* b : pinned)
+    if (b) cudaFreeHost(b);
+  void* bufs[] = {h->d_edges, h->d_slots, h->d_red, h->d_x1, h->d_x2, h->d_sH,
                   h->d_tH, h->d_uH, h->d_as, h->d_q2r, h->d_q2f, h->d_qhist, h->d_wmax, h->d_counter, h->d_cteq, h->d_flow, h->d_flow_pk,
-                  h->d_flow_bias, h->d_flow_buf, h->d_flow_tc, h->d_flow_status, h->d_flow_ticket, h->d_pdfbuf,
-                  h->d_gen_stage, h->d_gen_red, h->d_gen_cnt, h->d_ftrain, h->d_tails, h->d_bmask,
-                  h->d_rsum, h->d_roff, h->d_unw_red, h->d_ticket};
+                  h->d_flow_bias, h->d_flow_buf, h->d_flow_tc, h->d_flow_ticket, h->d_pdfbuf,
+                  h->d_gen_stage, h->d_ftrain, h->d_tails, h->d_bmask,
+                  h->d_rsum, h->d_roff, h->d_ticket, h->d_adj};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete h;
@@ -684,11 +703,10 @@ static int partonic_run(cp_handle* h, int mode, PartonicArgs a, uint64_t npoints
   if (mode == 0) k_partonic<0><<<blocks, CP_THREADS, 0, h->stream>>>(a);
   else k_partonic<1><<<blocks, CP_THREADS, 0, h->stream>>>(a);
   CP_LAUNCH_CHECK(h, "k_partonic");
-  k_reduce_slots<0><<<1, 4 * 32, 0, h->stream>>>(h->d_slots, blocks, 4, h->d_red);
+  k_reduce_slots<0><<<1, 4 * 32, 0, h->stream>>>(h->d_slots, blocks, 4, h->mail->sums);
   CP_LAUNCH_CHECK(h, "k_reduce_slots");
-  double red[4];
-  CP_CUDA(h, cudaMemcpyAsync(red, h->d_red, sizeof red, cudaMemcpyDeviceToHost, h->stream));
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  const double* red = h->mail->sums;
   if (out) {
     double n = (double)npoints, mean = red[0] / n, var = (red[1] / n - mean * mean) / (n - 1.0);
     out->sigma = mean;

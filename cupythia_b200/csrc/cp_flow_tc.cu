@@ -505,7 +505,7 @@ __device__ __forceinline__ void cp_flow_tc_body(const uint4* __restrict__ img_g,
       }
       if (cp_bar_wg_or(bar_id, *abort != 0)) break;
     }
-    if (row == 0 && *abort) atomicOr(status, 1);
+    if (row == 0 && *abort) *(volatile int*)status = 1;
     if constexpr (ACCEPT) {
       double v[7];
       cp_unw_warp_sums(S, v);
@@ -565,10 +565,6 @@ int cp_flow_tc_repack(cp_handle* h)
 int cp_flow_tc_alloc(cp_handle* h)
 {
   if (!h->d_flow_tc) CP_CUDA(h, cudaMalloc(&h->d_flow_tc, CP_TC_IMG));
-  if (!h->d_flow_status) {
-    CP_CUDA(h, cudaMalloc(&h->d_flow_status, sizeof(int)));
-    CP_CUDA(h, cudaMemsetAsync(h->d_flow_status, 0, sizeof(int), h->stream));
-  }
   CP_CUDA(h, cudaFuncSetAttribute(k_flow_fwd_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, CpTcLayout<CP_TC_WG>::SMEM));
   CP_CUDA(h, cudaFuncSetAttribute(k_flow_accept_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   CpTcLayout<CP_TC_WG_ACC>::SMEM));
@@ -590,7 +586,7 @@ int cp_flow_tc_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t iter,
   k_flow_fwd_tc<<<grid, CpTcLayout<CP_TC_WG>::THREADS, CpTcLayout<CP_TC_WG>::SMEM, h->stream>>>(reinterpret_cast<const uint4*>(h->d_flow_tc), h->d_flow,
                                                                  h->d_edges,
                                                                  h->nb, h->cfg.seed, point0, n, iter, stream, out,
-                                                                 uout, h->d_flow_status, h->flow_stall);
+                                                                 uout, h->mail->status, h->flow_stall);
   CP_LAUNCH_CHECK(h, "k_flow_fwd_tc");
   return CP_OK;
 }
@@ -611,25 +607,21 @@ int cp_flow_tc_accept_enqueue(cp_handle* h, const UnwLaunch& L, int* blocks)
   if (grid < 1) return CP_OK;
   using Lay = CpTcLayout<CP_TC_WG_ACC>;
   k_flow_accept_tc<<<grid, Lay::THREADS, Lay::SMEM, h->stream>>>(reinterpret_cast<const uint4*>(h->d_flow_tc),
-                                                                  h->d_flow, h->P, L, h->d_flow_status, h->flow_stall);
+                                                                  h->d_flow, h->P, L, h->mail->status, h->flow_stall);
   CP_LAUNCH_CHECK(h, "k_flow_accept_tc");
   *blocks = grid;
   return CP_OK;
 }
 
-// Reads and clears the device status of the tensor-core flow kernel, in order on the handle's
-// stream (which may be a non-blocking stream): CP_ERR_TIMEOUT if a bounded wait expired since
-// the last check.
+// Synchronises the handle's stream, then reads and clears the status words of the tensor-core
+// kernels (mapped host memory): CP_ERR_TIMEOUT if a bounded wait expired since the last check.
 int cp_flow_tc_status(cp_handle* h)
 {
-  if (!h->d_flow_status) return CP_OK;
-  int s = 0;
-  CP_CUDA(h, cudaMemcpyAsync(&s, h->d_flow_status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (!s) return CP_OK;
-  CP_CUDA(h, cudaMemsetAsync(h->d_flow_status, 0, sizeof(int), h->stream));
-  CP_CUDA(h, cudaStreamSynchronize(h->stream));
-  return cp_fail(h, CP_ERR_TIMEOUT, (s & 2) ? "k_flow_wgrad_tc: a tensor-core wait expired (this training step's gradient is invalid)"
+  const bool wgrad = h->mail->status[1] != 0;
+  if (!h->mail->status[0] && !wgrad) return CP_OK;
+  h->mail->status[0] = h->mail->status[1] = 0;
+  return cp_fail(h, CP_ERR_TIMEOUT, wgrad ? "k_flow_wgrad_tc: a tensor-core wait expired (this training step's gradient is invalid)"
                                             : "k_flow_fwd_tc / k_flow_accept_tc: a tensor-core wait expired (results of this pass are invalid)");
 }
 

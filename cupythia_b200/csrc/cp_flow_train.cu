@@ -605,7 +605,7 @@ __device__ __forceinline__ void cp_wgt_layer(const uint8_t* __restrict__ A, cons
     // a wait expired: record it, and before TMEM is released let every MMA this thread issued
     // complete (a fresh barrier, bounded wait)
     if (tid == 0) {
-      atomicOr(status, 2);
+      *(volatile int*)status = 1;
       cp_tc_commit(drain);
       volatile int drain_abort = 0;
       cp_mbar_wait_bounded(drain, 0u, &drain_abort);
@@ -805,7 +805,7 @@ static size_t bwd_smem() { return sizeof(uint2) * CP_FLOW_NC * CP_FLOW_P_PER + s
 static size_t fwd_smem() { return sizeof(uint2) * CP_FLOW_NC * CP_FLOW_P_FWD + sizeof(float) * CP_FLOW_NC * CP_FLOW_NB; }
 
 // Training buffers for `count` points of a step, kept in the handle between the phases of a
-// step.  A new layout (another count) starts from zeros: columns the kernels never write (the
+// step and between calls.  A new layout (another count) starts from zeros: columns the kernels never write (the
 // padding of the 16-wide operands) must read as zero.
 static int train_buffers(cp_handle* h, uint64_t count, FlowTrainBufs& t)
 {
@@ -818,10 +818,10 @@ static int train_buffers(cp_handle* h, uint64_t count, FlowTrainBufs& t)
     }
     CP_CUDA(h, cudaMalloc(&h->d_ftrain, train_bytes(count)));
     h->ftrain_cap = count;
-    h->ftrain_count = 0;
+    h->ftrain_zeroed = 0;
   }
-  if (count != h->ftrain_count) CP_CUDA(h, cudaMemsetAsync(h->d_ftrain, 0, train_bytes(count), h->stream));
-  h->ftrain_count = count;
+  if (count != h->ftrain_zeroed) CP_CUDA(h, cudaMemsetAsync(h->d_ftrain, 0, train_bytes(count), h->stream));
+  h->ftrain_count = h->ftrain_zeroed = count;
   carve(h->d_ftrain, count, t);
   // per-device attributes: set on every use (host-side, cheap)
   CP_CUDA(h, cudaFuncSetAttribute(k_flow_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bwd_smem()));
@@ -829,13 +829,18 @@ static int train_buffers(cp_handle* h, uint64_t count, FlowTrainBufs& t)
   return CP_OK;
 }
 
-static void train_buffers_release(cp_handle* h)
+// Ends a call's use of the training buffers: no step is pending any more, and buffers above
+// CP_TRAIN_KEEP bytes go back to the device.  Smaller ones stay in the handle until it is destroyed
+// (batches of 65,536 points: 160 MB), since allocating and freeing them took up to 3 ms of a call.
+#define CP_TRAIN_KEEP ((size_t)1 << 30)
+static void train_buffers_done(cp_handle* h)
 {
-  if (!h->d_ftrain) return;
+  h->ftrain_count = 0;
+  if (!h->d_ftrain || train_bytes(h->ftrain_cap) <= CP_TRAIN_KEEP) return;
   cudaStreamSynchronize(h->stream);
   cudaFree(h->d_ftrain);
   h->d_ftrain = nullptr;
-  h->ftrain_cap = h->ftrain_count = 0;
+  h->ftrain_cap = h->ftrain_zeroed = 0;
 }
 
 // Phase 1 of a step: forward and integrand over the batch points [point0, point0 + count) at
@@ -880,7 +885,7 @@ static int flow_phase_gradient(cp_handle* h, const FlowTrainBufs& t, uint64_t co
   if (h->flow_kernel == 0) {
     // tensor cores (tcgen05): every coupling and layer shape in one launch
     k_flow_wgrad_tc<<<dim3((unsigned)nblk, CP_FLOW_NC, 3), 128, 0, h->stream>>>(t, count, (int)chunk,
-                                                                             h->d_flow_status);
+                                                                             h->mail->status + 1);
     CP_LAUNCH_CHECK(h, "k_flow_wgrad_tc");
   } else {
     // warp-level mma.sync, one launch per layer shape (the cross-check path)
@@ -952,25 +957,23 @@ extern "C" int cp_flow_train(cp_handle* h, int n_steps, uint64_t batch, double l
   if (!h->d_flow) return cp_fail(h, CP_ERR_INVALID, "flow not initialised (cp_flow_init)");
   if (n_steps < 1 || batch < 64 || batch > (1ull << 24) || (batch & 31))
     return cp_fail(h, CP_ERR_INVALID, "cp_flow_train: batch must be a multiple of 32 in [64, 2^24]");
-  h->ftrain_count = 0;   // a fresh layout: the buffers start from zeros
-  FlowTrainBufs t;
-  int rc = train_buffers(h, batch, t);
+  int rc = cp_ensure_losses(h, n_steps);
   if (rc) return rc;
-  double* losses = nullptr;
-  CP_CUDA(h, cudaMalloc(&losses, sizeof(double) * (size_t)n_steps));
+  FlowTrainBufs t;
+  rc = train_buffers(h, batch, t);
+  if (rc) return rc;
+  double* losses = h->h_losses;   // each step's last integrand block writes its own
   for (int s = 0; s < n_steps && rc == CP_OK; ++s) {
     int nblk = 0;
     rc = flow_phase_moments(h, t, 0, batch, (uint32_t)h->flow_t, t.sums, losses + s);
     if (!rc) rc = flow_phase_gradient(h, t, batch, t.sums, batch, losses + s, true, &nblk);
     if (!rc) rc = flow_phase_update_local(h, t, nblk, lr);
   }
-  cudaError_t e = cudaSuccess;
-  if (!rc && loss_host) e = cudaMemcpyAsync(loss_host, losses, sizeof(double) * n_steps, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (!rc && e != cudaSuccess) rc = cp_fail_cuda(h, e, "cp_flow_train readback");
+  const cudaError_t e = cudaStreamSynchronize(h->stream);
+  if (!rc && e != cudaSuccess) rc = cp_fail_cuda(h, e, "cp_flow_train");
+  if (!rc && loss_host) memcpy(loss_host, losses, sizeof(double) * n_steps);
   if (!rc) rc = cp_flow_tc_status(h);
-  cudaFree(losses);
-  train_buffers_release(h);
+  train_buffers_done(h);
   return rc;
 }
 
@@ -981,7 +984,6 @@ extern "C" int cp_flow_loss_grad(cp_handle* h, uint64_t batch, uint32_t iter, fl
   CP_CHECK_HANDLE(h);
   if (!h->d_flow) return cp_fail(h, CP_ERR_INVALID, "flow not initialised (cp_flow_init)");
   if (batch < 64 || batch > (1ull << 24) || (batch & 31)) return cp_fail(h, CP_ERR_INVALID, "bad batch");
-  h->ftrain_count = 0;
   FlowTrainBufs t;
   int rc = train_buffers(h, batch, t);
   if (rc) return rc;
@@ -997,7 +999,7 @@ extern "C" int cp_flow_loss_grad(cp_handle* h, uint64_t batch, uint32_t iter, fl
     if (e != cudaSuccess) rc = cp_fail_cuda(h, e, "cp_flow_loss_grad readback");
   }
   if (!rc) rc = cp_flow_tc_status(h);
-  train_buffers_release(h);
+  train_buffers_done(h);
   return rc;
 }
 

@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(CP_THREADS) k_to_device_events(const HandoffLa
     for (int q = 0; q < 4; ++q) dst[q] = src[q];
     int col[4], acol[4];
     if (!cp_colour_expand(r.process, r.colour, col, acol)) {
-      atomicOr(L.bad, 1);
+      *(volatile int*)L.bad = 1;
       for (int k = 0; k < 4; ++k) col[k] = acol[k] = 0;
     }
     const uint64_t e = L.e0 + i;
@@ -109,15 +109,13 @@ extern "C" int cp_records_to_device_events(cp_handle* h, const cp_event* records
                         ev->flavB, ev->active, ev->weight};
   for (const void* p : ptrs)
     if (!p) return cp_fail(h, CP_ERR_INVALID, "cp_records_to_device_events: null member array");
-  int* bad = nullptr;
-  CP_CUDA(h, cudaMallocAsync(reinterpret_cast<void**>(&bad), sizeof(int), h->stream));
-  CP_CUDA(h, cudaMemsetAsync(bad, 0, sizeof(int), h->stream));
+  h->mail->bad = 0;   // no earlier call's kernel is still running: every one ends synchronised
   HandoffLaunch L;
   L.rec = records_dev; L.n = n; L.e0 = e0; L.seed = h->cfg.seed; L.ratios = scale_ratios_dev;
   L.sqrt_kf = sqrt(h->cfg.k_fac);
   L.inv_ebeam = 2.0 / h->cfg.sqrt_s;
   L.ev = *ev;
-  L.bad = bad;
+  L.bad = &h->mail->bad;
   const uint64_t want = (n + CP_THREADS - 1) / CP_THREADS;
   const unsigned blocks = (unsigned)(want < (uint64_t)h->num_sms * 8 ? want : (uint64_t)h->num_sms * 8);
   bool vec4 = ev->maxPart == 4;
@@ -127,11 +125,8 @@ extern "C" int cp_records_to_device_events(cp_handle* h, const cp_event* records
   if (vec4) k_to_device_events<true><<<blocks, CP_THREADS, 0, h->stream>>>(L);
   else k_to_device_events<false><<<blocks, CP_THREADS, 0, h->stream>>>(L);
   cudaError_t e = cudaGetLastError();
-  int hb = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&hb, bad, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-  cudaFreeAsync(bad, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return cp_fail_cuda(h, e, "cp_records_to_device_events");
-  if (hb) return cp_fail(h, CP_ERR_INVALID, "cp_records_to_device_events: a record's process code or colour flow is invalid");
+  if (h->mail->bad) return cp_fail(h, CP_ERR_INVALID, "cp_records_to_device_events: a record's process code or colour flow is invalid");
   return CP_OK;
 }

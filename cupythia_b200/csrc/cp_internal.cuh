@@ -87,6 +87,18 @@ struct CpIterDev {
   double sumw, sumw2, wmax, nbad, n, sigma, err, pad;
 };
 
+// What a call's kernels hand back to the host: in mapped pinned memory, which they write themselves,
+// so a call ends with one stream synchronisation instead of device-to-host copies into pageable
+// memory (each of which waits for the device by itself; 50,021 points of production: 54 -> 38 us).
+struct CpMail {
+  int status[2];                              // tensor-core waits that expired: flow forward, weight gradients
+  int bad;                                    // record hand-off: an invalid record
+  double wq[2];                               // threshold quantile, q
+  double sums[4];                             // partonic: sum w, sum w^2, max w, unused
+  unsigned long long count;                   // accepted events of a production pass
+  double adj[10 + 6 * (CP_MAX_BINS + 1)];     // adjoint record and edge gradients
+};
+
 struct cp_handle {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -102,7 +114,8 @@ struct cp_handle {
   double* d_slots = nullptr;
   size_t slots_cap = 0;           // doubles
   double* d_red = nullptr;        // CP_SLOT_HEAD + 3*CP_MAX_BINS doubles
-  CpIterDev* d_iters = nullptr;   // per-iteration records
+  CpMail* mail = nullptr;         // mapped pinned memory
+  CpIterDev* h_iters = nullptr;   // per-iteration records, mapped pinned memory
   int iters_cap = 0;
   // SigmaProcess batch state (SoA FP32)
   int64_t kin_n = 0, kin_cap = 0;
@@ -127,18 +140,16 @@ struct cp_handle {
   unsigned* d_rsum = nullptr;
   unsigned long long* d_roff = nullptr;
   uint64_t pdfbuf_cap = 0;
-  double* d_unw_red = nullptr;
+  double* h_unw_red = nullptr;             // mapped pinned memory
   uint64_t unw_red_cap = 0;
   float* scalew = nullptr;                 // caller's scale-variation weights (6 per record), or null
   uint64_t scalew_cap = 0;
   // cp_generate_host pipeline, kept between calls: CP_GEN_BUFS record staging buffers of gen_cap
-  // slots each, per-chunk reductions and counters, the counters' host copy in mapped pinned
-  // memory (written by a kernel, so that no count waits behind a record copy), the copy stream
-  // and its events
+  // slots each, per-chunk sums and counts in mapped pinned memory (written by the kernels, so that
+  // no count waits behind a record copy), the copy stream and its events
   cp_event* d_gen_stage = nullptr;
   uint64_t gen_cap = 0;
-  double* d_gen_red = nullptr;
-  unsigned long long* d_gen_cnt = nullptr;
+  double* h_gen_red = nullptr;
   unsigned long long* h_gen_cnt = nullptr;
   uint64_t gen_chunks_cap = 0;
   cudaStream_t gen_copy = nullptr;
@@ -163,10 +174,13 @@ struct cp_handle {
   // ftrain_count points), kept between the phases of a data-parallel step
   void* d_ftrain = nullptr;
   uint64_t ftrain_cap = 0, ftrain_count = 0;
-  // tensor-core (tcgen05) forward: shared-memory weight image, bounded-wait status flag;
+  uint64_t ftrain_zeroed = 0;              // the layout (count) whose never-written parts are zero
+  double* h_losses = nullptr;              // batch losses of a training run, mapped pinned memory
+  int losses_cap = 0;
+  double* d_adj = nullptr;                 // sums of an adjoint pass
+  // tensor-core (tcgen05) forward: shared-memory weight image (bounded-wait status: mail->status);
   // flow_kernel 0 = tcgen05 kernel, 1 = the warp-level mma.sync kernel
   uint8_t* d_flow_tc = nullptr;
-  int* d_flow_status = nullptr;
   unsigned* d_flow_ticket = nullptr;       // last-block ticket of the training integrand kernel (0 between launches)
   int flow_kernel = 0;
   int flow_tc_stale = 1;                   // the tcgen05 weight image lags the master parameters
@@ -185,6 +199,7 @@ int cp_fail(cp_handle* h, int code, const std::string& msg);
 int cp_fail_cuda(cp_handle* h, cudaError_t e, const char* what);
 int cp_ensure_slots(cp_handle* h, size_t doubles);
 int cp_ensure_iters(cp_handle* h, int n);
+int cp_ensure_losses(cp_handle* h, int n);
 int cp_flow_buffer(cp_handle* h, uint64_t n);
 // uout, if not null, receives each point's accept draw u24(word 3) of its Philox block when the
 // tensor-core forward runs (cp_flow_writes_u); the mma.sync forward leaves it untouched.

@@ -21,7 +21,6 @@
 // Random numbers: the accept draw is word 3 of the point's Philox block (stream 0); accepted
 // points draw a second block from stream 1 for the process / pair / azimuth / new-flavour picks
 // (high 24 bits of words 0..3) and the colour topology / orientation (their low bytes).
-#include <vector>
 #include "cp_internal.cuh"
 
 #include "cp_unweight.cuh"
@@ -133,13 +132,14 @@ __global__ void __launch_bounds__(CP_UNW_THREADS, CP_UNW_RESIDENT)
 // accept blocks' sums (fixed order: thread t takes column t % 8 of slots t / 8, t / 8 + 128, ...,
 // then the xor tree of a warp, then the warps in order), block 1 turns the range totals into output
 // offsets: roff[r] = *base_io (0 for `first`) + the records of the ranges before r; then
-// *base_io = the records so far.  Sixteen ranges a thread, so the 16,384 ranges of a full chunk are
+// *base_io = the records so far, also handed to the host (as the sums are, through `red`).  Sixteen ranges a thread, so the 16,384 ranges of a full chunk are
 // one tile: one scan over the block (warp shuffles, a warp over the warps' sums) instead of sixteen
 // (18 us of every chunk, 13 of them saved).  The totals are cleared as they are read, for the next chunk.
 #define CP_SCAN_PER 16
 __global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ slots, int nslots, double* __restrict__ red,
                                                      uint4* __restrict__ rsum, uint64_t nrange, int first,
-                                                     unsigned long long* base_io, unsigned long long* __restrict__ roff)
+                                                     unsigned long long* base_io, unsigned long long* __restrict__ roff,
+                                                     unsigned long long* host_count)
 {
   __shared__ double sRed[32][CP_UNW_SLOT];
   __shared__ unsigned long long wsum[32];
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ 
     carry += wsum[31];
     __syncthreads();   // wsum is rewritten by the next tile
   }
-  if (t == 0) *base_io = carry;   // every thread has read it: the loop's barriers (nrange >= 1)
+  if (t == 0) *host_count = *base_io = carry;   // every thread has read it: the loop's barriers (nrange >= 1)
 }
 
 // K2: work units of a quarter range (8 blocks, 256 points: 65,536 per 2^24-point chunk, so the
@@ -392,7 +392,7 @@ static bool fused_production(const cp_handle* h) { return h->flow_on && h->flow_
 // runs its own.  tslot >= 0 records the chunk's timing events.
 static int unweight_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t iter, cp_event* out,
                             uint64_t capacity, double* red_dst, float* scalew, unsigned long long* base_dev,
-                            int first, const float4* flow_pre, const float* flow_u_pre, int tslot)
+                            int first, unsigned long long* host_count, const float4* flow_pre, const float* flow_u_pre, int tslot)
 {
   if (n > CP_UNW_CHUNK) return cp_fail(h, CP_ERR_INVALID, "production chunk above CP_UNW_CHUNK points");
   UnwLaunch L;
@@ -448,7 +448,7 @@ static int unweight_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t 
   // without records there are no offsets to form: the sums' block alone
   k_unw_finish<<<capacity ? 2 : 1, 1024, 0, h->stream>>>(h->d_slots, red_blocks, red_dst,
                                                          reinterpret_cast<uint4*>(L.rsum), L.nrange, first, base_dev,
-                                                         h->d_roff);
+                                                         h->d_roff, host_count);
   const cudaError_t fe = cudaGetLastError();
   if (fe != cudaSuccess) {
     h->pdfbuf_cap = 0;   // the range totals were not cleared: the next pass allocates them anew
@@ -516,15 +516,15 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   const uint64_t nsub = (n_points + CP_UNW_CHUNK - 1) / CP_UNW_CHUNK;
   if (nsub > h->unw_red_cap) {
     CP_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (h->d_unw_red) CP_CUDA(h, cudaFree(h->d_unw_red));
-    h->d_unw_red = nullptr;
+    if (h->h_unw_red) CP_CUDA(h, cudaFreeHost(h->h_unw_red));
+    h->h_unw_red = nullptr;
     h->unw_red_cap = 0;
-    CP_CUDA(h, cudaMalloc(&h->d_unw_red, sizeof(double) * 8 * nsub));
+    CP_CUDA(h, cudaHostAlloc(&h->h_unw_red, sizeof(double) * 8 * nsub, cudaHostAllocMapped | cudaHostAllocPortable));
     h->unw_red_cap = nsub;
   }
   int rc = timing_reserve(h, nsub);
   if (rc) return rc;
-  if (!capacity) CP_CUDA(h, cudaMemsetAsync(h->d_counter, 0, sizeof(unsigned long long), h->stream));
+  h->mail->count = 0;   // without records no kernel writes it
   // the flow forward once for the whole pass (20 B per point: (v, ln J) and the accept draw), then the chunks; the fused form
   // runs the forward inside each chunk's accept kernel
   const bool fused = fused_production(h);
@@ -539,31 +539,21 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   }
   for (uint64_t c = 0; c < nsub; ++c) {
     const uint64_t p0 = c * CP_UNW_CHUNK, n = p0 + CP_UNW_CHUNK <= n_points ? CP_UNW_CHUNK : n_points - p0;
-    rc = unweight_enqueue(h, p0, n, iter, records_dev, capacity, h->d_unw_red + 8 * c, h->scalew, h->d_counter, c == 0,
+    rc = unweight_enqueue(h, p0, n, iter, records_dev, capacity, h->h_unw_red + 8 * c, h->scalew, h->d_counter, c == 0, &h->mail->count,
                           (h->flow_on && !fused) ? h->d_flow_buf + p0 : nullptr,
                           (h->flow_on && !fused && cp_flow_writes_u(h)) ? h->d_flow_u + p0 : nullptr, (int)c);
     if (rc) return rc;
   }
-  std::vector<double> hred(8 * nsub, 0.0);
-  unsigned long long cnt = 0;
-  CP_CUDA(h, cudaMemcpyAsync(hred.data(), h->d_unw_red, sizeof(double) * 8 * nsub, cudaMemcpyDeviceToHost, h->stream));
-  CP_CUDA(h, cudaMemcpyAsync(&cnt, h->d_counter, sizeof cnt, cudaMemcpyDeviceToHost, h->stream));
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  const unsigned long long cnt = h->mail->count;
   timing_collect(h, nsub, h->flow_on && !fused, capacity > 0);
   if (h->flow_on && (rc = cp_flow_tc_status(h)) != CP_OK) return rc;
   double red[8];
-  combine_chunks(hred.data(), nsub, red);
+  combine_chunks(h->h_unw_red, nsub, red);
   if (out) fill_unw(red, (double)n_points, wm0, out);
   if (cnt > capacity) return cp_fail(h, CP_ERR_CAPACITY, "cp_unweight: record buffer too small (n_accepted reported)");
   if (red[3] > 0) return cp_fail(h, CP_ERR_NUMERIC, "non-finite or negative weights were zeroed");
   return CP_OK;
-}
-
-// one counter, copied by a kernel into the mapped pinned host array (no copy engine involved)
-__global__ void k_gen_count(const unsigned long long* __restrict__ src, unsigned long long* dst_mapped)
-{
-  *(volatile unsigned long long*)dst_mapped = *src;
-  __threadfence_system();
 }
 
 // Buffers and streams of the host-delivery pipeline, grown on demand and kept in the handle.
@@ -582,13 +572,12 @@ static int gen_reserve(cp_handle* h, uint64_t cap, uint64_t nchunks)
   }
   if (nchunks > h->gen_chunks_cap) {
     CP_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (h->d_gen_red) { CP_CUDA(h, cudaFree(h->d_gen_red)); h->d_gen_red = nullptr; }
-    if (h->d_gen_cnt) { CP_CUDA(h, cudaFree(h->d_gen_cnt)); h->d_gen_cnt = nullptr; }
+    if (h->h_gen_red) { CP_CUDA(h, cudaFreeHost(h->h_gen_red)); h->h_gen_red = nullptr; }
     if (h->h_gen_cnt) { CP_CUDA(h, cudaFreeHost(h->h_gen_cnt)); h->h_gen_cnt = nullptr; }
     h->gen_chunks_cap = 0;
-    CP_CUDA(h, cudaMalloc(&h->d_gen_red, sizeof(double) * 8 * nchunks));
-    CP_CUDA(h, cudaMalloc(&h->d_gen_cnt, sizeof(unsigned long long) * nchunks));
-    CP_CUDA(h, cudaHostAlloc(&h->h_gen_cnt, sizeof(unsigned long long) * nchunks, cudaHostAllocMapped));
+    const unsigned flags = cudaHostAllocMapped | cudaHostAllocPortable;
+    CP_CUDA(h, cudaHostAlloc(&h->h_gen_red, sizeof(double) * 8 * nchunks, flags));
+    CP_CUDA(h, cudaHostAlloc(&h->h_gen_cnt, sizeof(unsigned long long) * nchunks, flags));
     h->gen_chunks_cap = nchunks;
   }
   if (!h->gen_copy) {
@@ -622,11 +611,9 @@ extern "C" int cp_generate_host(cp_handle* h, uint64_t n_points, uint32_t iter, 
   // a chunk accepts at most every point: staging slots = chunk
   int rc = gen_reserve(h, chunk, nchunks);
   if (rc) return rc;
-  std::vector<double> hred(nchunks * 8, 0.0);
   uint64_t written = 0, total_acc = 0;
   cudaError_t e = cudaSuccess;
   unsigned long long* const hcnt = h->h_gen_cnt;
-  unsigned long long* dcnt_mapped = nullptr;
   // records of chunk j: wait for its count, copy what fits
   auto drain = [&](uint64_t j) -> cudaError_t {
     const int b = (int)(j % CP_GEN_BUFS);
@@ -644,23 +631,18 @@ extern "C" int cp_generate_host(cp_handle* h, uint64_t n_points, uint32_t iter, 
     return cudaEventRecord(h->gen_copied[b], h->gen_copy);
   };
   do {
-    if ((e = cudaHostGetDevicePointer((void**)&dcnt_mapped, hcnt, 0)) != cudaSuccess) break;
     for (uint64_t c = 0; c < nchunks; ++c) {
       const int b = (int)(c % CP_GEN_BUFS);
       const uint64_t p0 = c * chunk, n = (p0 + chunk <= n_points) ? chunk : n_points - p0;
       if (c >= CP_GEN_BUFS && (e = cudaStreamWaitEvent(h->stream, h->gen_copied[b], 0)) != cudaSuccess) break;
-      rc = unweight_enqueue(h, p0, n, iter, h->d_gen_stage + (uint64_t)b * chunk, chunk, h->d_gen_red + 8 * c,
-                            nullptr, h->d_gen_cnt + c, 1, nullptr, nullptr, -1);
+      rc = unweight_enqueue(h, p0, n, iter, h->d_gen_stage + (uint64_t)b * chunk, chunk, h->h_gen_red + 8 * c,
+                            nullptr, h->d_counter, 1, hcnt + c, nullptr, nullptr, -1);
       if (rc) break;
-      k_gen_count<<<1, 1, 0, h->stream>>>(h->d_gen_cnt + c, dcnt_mapped + c);
-      if ((e = cudaGetLastError()) != cudaSuccess) break;
       if ((e = cudaEventRecord(h->gen_counted[b], h->stream)) != cudaSuccess) break;
       if (c >= 1 && (e = drain(c - 1)) != cudaSuccess) break;
     }
     if (e != cudaSuccess || rc) break;
     if ((e = drain(nchunks - 1)) != cudaSuccess) break;
-    if ((e = cudaMemcpyAsync(hred.data(), h->d_gen_red, sizeof(double) * 8 * nchunks, cudaMemcpyDeviceToHost,
-                             h->stream)) != cudaSuccess) break;
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) break;
     e = cudaStreamSynchronize(h->gen_copy);
   } while (0);
@@ -671,7 +653,7 @@ extern "C" int cp_generate_host(cp_handle* h, uint64_t n_points, uint32_t iter, 
   if (rc) return rc;
   if (h->flow_on && (rc = cp_flow_tc_status(h)) != CP_OK) return rc;
   double tot[8];
-  combine_chunks(hred.data(), nchunks, tot);
+  combine_chunks(h->h_gen_red, nchunks, tot);
   if (out) fill_unw(tot, (double)n_points, wm0, out);
   if (total_acc > capacity) return cp_fail(h, CP_ERR_CAPACITY, "cp_generate_host: record buffer too small");
   if (tot[3] > 0) return cp_fail(h, CP_ERR_NUMERIC, "non-finite or negative weights were zeroed");

@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(CP_THREADS, CP_MIN_BLOCKS) k_had_accum(const _
 // a thread: with S(b) the weights in bins >= b (integers, so exact in any order), the threshold
 // bin is the largest b >= 1 with S(b) > (1 - q) n, or 0.  One thread walking the 4096 bins twice
 // took 92 us, longer than a pass of a million points.
-__global__ void __launch_bounds__(1024) k_quantile(const unsigned long long* __restrict__ qhist, double q, double* wmax)
+__global__ void __launch_bounds__(1024) k_quantile(const unsigned long long* __restrict__ qhist, double q, double* wmax,
+                                                   double* host)
 {
   static_assert(CP_QBINS == 4 * 1024, "four bins a thread");
   __shared__ unsigned long long sWarp[32];
@@ -177,8 +178,8 @@ __global__ void __launch_bounds__(1024) k_quantile(const unsigned long long* __r
   if (lane == 0 && best) atomicMax(&sBest, best);
   __syncthreads();
   if (t == 0) {
-    wmax[0] = (double)cp_qbin_hi(sBest);
-    wmax[1] = q;
+    host[0] = wmax[0] = (double)cp_qbin_hi(sBest);
+    host[1] = wmax[1] = q;
   }
 }
 
@@ -398,11 +399,10 @@ extern "C" int cp_vegas_iteration(cp_handle* h, uint64_t n_points, uint32_t iter
   if (n_points < 2) return cp_fail(h, CP_ERR_INVALID, "cp_vegas_iteration: n_points < 2");
   int rc = cp_ensure_iters(h, 1);
   if (rc) return rc;
-  rc = had_iteration(h, n_points, iter, alpha, h->d_iters, 1, 0);
+  rc = had_iteration(h, n_points, iter, alpha, h->h_iters, 1, 0);
   if (rc) return rc;
-  CpIterDev r;
-  CP_CUDA(h, cudaMemcpyAsync(&r, h->d_iters, sizeof r, cudaMemcpyDeviceToHost, h->stream));
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  const CpIterDev& r = h->h_iters[0];
   if (h->flow_on && (rc = cp_flow_tc_status(h)) != CP_OK) return rc;
   if (out) fill_result(r, out);
   if (r.nbad > 0) return cp_fail(h, CP_ERR_NUMERIC, "non-finite or negative weights were zeroed");
@@ -417,15 +417,12 @@ extern "C" int cp_integrate(cp_handle* h, int n_iter, uint64_t n_points, double 
   int rc = cp_ensure_iters(h, n_iter);
   if (rc) return rc;
   for (int it = 0; it < n_iter; ++it) {
-    rc = had_iteration(h, n_points, (uint32_t)it, alpha, h->d_iters + it, it == 0, it + 1 < n_iter);
+    rc = had_iteration(h, n_points, (uint32_t)it, alpha, h->h_iters + it, it == 0, it + 1 < n_iter);
     if (rc) return rc;
   }
-  CpIterDev* recs = new CpIterDev[n_iter];
-  cudaError_t e = cudaMemcpyAsync(recs, h->d_iters, sizeof(CpIterDev) * n_iter,
-                                  cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) { delete[] recs; return cp_fail_cuda(h, e, "cp_integrate readback"); }
-  if (h->flow_on && (rc = cp_flow_tc_status(h)) != CP_OK) { delete[] recs; return rc; }
+  CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  const CpIterDev* recs = h->h_iters;
+  if (h->flow_on && (rc = cp_flow_tc_status(h)) != CP_OK) return rc;
   double wsum = 0, w2 = 0, sw = 0, sw2 = 0, wmax = 0, nbad = 0, npts = 0;
   for (int it = 0; it < n_iter; ++it) {
     if (per_iter) fill_result(recs[it], per_iter + it);
@@ -436,7 +433,6 @@ extern "C" int cp_integrate(cp_handle* h, int n_iter, uint64_t n_points, double 
     sw += recs[it].sumw; sw2 += recs[it].sumw2; npts += recs[it].n;
     wmax = recs[it].wmax > wmax ? recs[it].wmax : wmax;
   }
-  delete[] recs;
   if (combined) {
     combined->sigma = w2 > 0 ? wsum / w2 : 0;
     combined->sigma_err = w2 > 0 ? 1.0 / sqrt(w2) : 0;
@@ -488,11 +484,10 @@ extern "C" int cp_weight_quantile(cp_handle* h, double q, double* w_q)
   CP_CHECK_HANDLE(h);
   if (!(q > 0.0 && q < 1.0)) return cp_fail(h, CP_ERR_INVALID, "cp_weight_quantile: q must be in (0, 1)");
   if (h->last_n == 0) return cp_fail(h, CP_ERR_INVALID, "cp_weight_quantile: run an iteration first");
-  k_quantile<<<1, 1024, 0, h->stream>>>(h->d_qhist, q, h->d_wmax);
+  k_quantile<<<1, 1024, 0, h->stream>>>(h->d_qhist, q, h->d_wmax, h->mail->wq);
   CP_LAUNCH_CHECK(h, "k_quantile");
-  double v[2];
-  CP_CUDA(h, cudaMemcpyAsync(v, h->d_wmax, sizeof v, cudaMemcpyDeviceToHost, h->stream));
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  const double* v = h->mail->wq;
   h->wmax_host = v[0];   // production passes check the threshold without reading the device
   if (w_q) *w_q = v[0];
   return CP_OK;
@@ -524,11 +519,10 @@ extern "C" int cp_vegas_refine_sums(cp_handle* h, const double* sums_dev, double
   if (rc) return rc;
   CP_CUDA(h, cudaMemcpyAsync(h->d_red, sums_dev, sizeof(double) * (CP_SLOT_HEAD + 3 * h->nb), cudaMemcpyDeviceToDevice,
                              h->stream));
-  k_refine<<<1, 128, 0, h->stream>>>(h->d_edges, h->d_red, h->nb, n_total, alpha, h->d_iters);
+  k_refine<<<1, 128, 0, h->stream>>>(h->d_edges, h->d_red, h->nb, n_total, alpha, h->h_iters);
   CP_LAUNCH_CHECK(h, "k_refine");
-  CpIterDev r;
-  CP_CUDA(h, cudaMemcpyAsync(&r, h->d_iters, sizeof r, cudaMemcpyDeviceToHost, h->stream));
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  const CpIterDev& r = h->h_iters[0];
   if (out) fill_result(r, out);
   if (r.nbad > 0) return cp_fail(h, CP_ERR_NUMERIC, "non-finite or negative weights were zeroed");
   return CP_OK;
@@ -549,11 +543,10 @@ extern "C" int cp_weight_quantile_hist(cp_handle* h, const unsigned long long* h
 {
   CP_CHECK_HANDLE(h);
   if (!hist_dev || !(q > 0.0 && q < 1.0)) return cp_fail(h, CP_ERR_INVALID, "cp_weight_quantile_hist: bad arguments");
-  k_quantile<<<1, 1024, 0, h->stream>>>(hist_dev, q, h->d_wmax);
+  k_quantile<<<1, 1024, 0, h->stream>>>(hist_dev, q, h->d_wmax, h->mail->wq);
   CP_LAUNCH_CHECK(h, "k_quantile");
-  double v[2];
-  CP_CUDA(h, cudaMemcpyAsync(v, h->d_wmax, sizeof v, cudaMemcpyDeviceToHost, h->stream));
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  const double* v = h->mail->wq;
   h->wmax_host = v[0];
   if (w_q) *w_q = v[0];
   return CP_OK;
