@@ -338,23 +338,40 @@ CP_HD CpCteqQ cp_cteq_coef(const CpCteqPoly& c, float lnQ, float Q, float invQ, 
   return q;
 }
 
+// The terms of a parametrisation's exponent that do not depend on the scale, for both beams (lane x:
+// beam A, lane y: beam B): L (ln(1 - x) or ln(1 - x + e^ut2)) and ut1 ln(1 - x) with its FMA residual.
+struct CpCteqX {
+  CpF2 L, t6, t6l;
+};
+
+// ux = cp_cteq_uses_x1l(i)
+CP_HD CpCteqX cp_cteq_x(const CpCteqPoly& c, const CpBeamX& bA, const CpBeamX& bB, bool ux)
+{
+  CpCteqX r;
+  const CpF2 x1L = cp_f2(bA.x1L, bB.x1L);
+  r.L = ux ? x1L : cp_f2(cp_logf(bA.omx + c.eut2), cp_logf(bB.omx + c.eut2));
+  const CpF2 u1 = cp_f2s(c.ut1);
+  r.t6 = cp_mul2(u1, x1L);
+  r.t6l = cp_fma2(u1, x1L, cp_f2(-r.t6.x, -r.t6.y));
+  return r;
+}
+
 // "answer" of xfUpdate (PartonDistributions.cc:1031-1046) for one parametrisation, for both
-// beams at once (lane x: beam A, lane y: beam B): x exp(exponent) (1 - Qmin/Q), with
+// beams at once: x exp(exponent) (1 - Qmin/Q), with
 //   exponent = A + B x + C u + af1 (y^p - 1) U + part3 + ut1 ln(1-x) + af2 L,  C = af1 af8,
 // summed with the products' FMA residuals kept in a second float, and exp(hi + lo) =
 // exp(hi) (1 + lo).  Every product, residual and sum runs in two-lane arithmetic, the
-// transcendentals per lane.  ux = cp_cteq_uses_x1l(i).
-CP_HD CpF2 cp_cteq_answer2(const CpCteqPoly& c, const CpCteqQ& a, const CpBeamX& bA, const CpBeamX& bB, bool ux)
+// transcendentals per lane.
+CP_HD CpF2 cp_cteq_answer2(const CpCteqX& cx, const CpCteqQ& a, const CpBeamX& bA, const CpBeamX& bB)
 {
   const CpF2 lny = cp_f2(bA.lny, bB.lny), x = cp_f2(bA.x, bB.x), omx = cp_f2(bA.omx, bB.omx);
-  const CpF2 uh = cp_f2(bA.uh, bB.uh), ul = cp_f2(bA.ul, bB.ul), x1L = cp_f2(bA.x1L, bB.x1L);
+  const CpF2 uh = cp_f2(bA.uh, bB.uh), ul = cp_f2(bA.ul, bB.ul);
   const CpF2 p = cp_f2s(a.p);
   const CpF2 ah = cp_mul2(p, lny);
   const CpF2 ym1 = cp_expm1_2(ah);
   const CpF2 U = cp_fma2(cp_f2s(a.af8), uh, cp_f2s(1.f));
   const CpF2 xo = cp_mul2(x, omx);
   const CpF2 part3 = cp_mul2(xo, cp_fma2(cp_f2s(a.af7), xo, cp_fma2(cp_f2s(a.af6), omx, cp_f2s(a.af5))));
-  const CpF2 L = ux ? x1L : cp_f2(cp_logf(bA.omx + c.eut2), cp_logf(bB.omx + c.eut2));
   const float Ch = a.af1 * a.af8, Cl = cp_fmaf(a.af1, a.af8, -Ch);
   const CpF2 ch = cp_f2s(Ch);
   const CpF2 t3 = cp_mul2(ch, uh);
@@ -363,12 +380,10 @@ CP_HD CpF2 cp_cteq_answer2(const CpCteqPoly& c, const CpCteqQ& a, const CpBeamX&
   const CpF2 t4 = cp_mul2(qv, U), t4l = cp_fma2(qv, U, cp_f2(-t4.x, -t4.y));
   const CpF2 Bv = cp_f2s(a.B);
   const CpF2 t2 = cp_mul2(Bv, x), t2l = cp_fma2(Bv, x, cp_f2(-t2.x, -t2.y));
-  const CpF2 u1 = cp_f2s(c.ut1);
-  const CpF2 t6 = cp_mul2(u1, x1L), t6l = cp_fma2(u1, x1L, cp_f2(-t6.x, -t6.y));
   const CpF2 a2 = cp_f2s(a.af2);
-  const CpF2 t7 = cp_mul2(a2, L), t7l = cp_fma2(a2, L, cp_f2(-t7.x, -t7.y));
-  const CpF2 el = cp_add2(cp_add2(t2l, t3l), cp_add2(cp_add2(t4l, t6l), t7l));
-  const CpF2 eh = cp_add2(cp_add2(cp_add2(cp_f2s(a.A), t3), cp_add2(t4, t2)), cp_add2(part3, cp_add2(t6, t7)));
+  const CpF2 t7 = cp_mul2(a2, cx.L), t7l = cp_fma2(a2, cx.L, cp_f2(-t7.x, -t7.y));
+  const CpF2 el = cp_add2(cp_add2(t2l, t3l), cp_add2(cp_add2(t4l, cx.t6l), t7l));
+  const CpF2 eh = cp_add2(cp_add2(cp_add2(cp_f2s(a.A), t3), cp_add2(t4, t2)), cp_add2(part3, cp_add2(cx.t6, t7)));
   const CpF2 ex = cp_f2(cp_exp_cteq(eh.x), cp_exp_cteq(eh.y));
   return cp_mul2(cp_mul2(x, cp_fma2(ex, el, ex)), cp_f2s(a.qfac));
 }
@@ -389,49 +404,72 @@ CP_HD CpCteqPoly cp_load_poly(const CpCteqPoly* p)
 #endif
 }
 
-// CTEQ5L of a proton for both beams at one factorisation scale (PDF::xf + CTEQ5L::xfUpdate):
-// fa, fb = {xd, xu, xg, xubar, xdbar, xs, xc, xb}, from the coefficient records `cteq` (the
-// kernel's parameters or a shared-memory copy).  UNROLL = 8 unrolls the 8 parametrisations, so the per-i
-// structure (the ln(1 - x) and Qmin cases, the dbar/ubar ratio, which register a result lands in)
-// is resolved at compile time: about 8% fewer cycles in the integrand kernels than the rolled
-// loop.  UNROLL = 1 keeps the rolled loop where code size or registers matter more (the second
-// and third evaluations of the scale-variation path).
-template <int UNROLL = 8>
-CP_HD void cp_cteq_pair(const CpCteqPoly* cteq, float Q2, float lnxA, float lnxAL, float lnxB,
-                        float lnxBL, float fa[8], float fb[8])
+// CTEQ5L of a proton for both beams at NS factorisation scales (PDF::xf + CTEQ5L::xfUpdate):
+// fa[s], fb[s] = {xd, xu, xg, xubar, xdbar, xs, xc, xb} at Q2[s], from the coefficient records `cteq`
+// (the kernel's parameters or a shared-memory copy).  The beams' x terms and each record's loads serve
+// every scale.  UNROLL = 8 unrolls the 8 parametrisations, so the per-i structure (the ln(1 - x) and
+// Qmin cases, the dbar/ubar ratio, which register a result lands in) is resolved at compile time:
+// about 8% fewer cycles in the integrand kernels than the rolled loop.  UNROLL = 1 keeps the rolled
+// loop where code size or registers matter more.
+template <int NS, int UNROLL>
+CP_HD void cp_cteq_scales(const CpCteqPoly* cteq, const float Q2in[NS], float lnxA, float lnxAL, float lnxB,
+                          float lnxBL, float fa[NS][8], float fb[NS][8])
 {
-  // Q2 clamp of PartonDistributions.cc:925
-  if (Q2 > 1e8f) Q2 = 1e8f;
-  if (Q2 < 1.f) Q2 = 1.f;
-  const float Q = cp_sqrtf(Q2);
-  const float lnQ = 0.5f * cp_logf(Q2);
-  const float invQ = cp_rcp(Q);
+  float Q[NS], lnQ[NS], invQ[NS];
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    // Q2 clamp of PartonDistributions.cc:925
+    float Q2 = Q2in[s];
+    if (Q2 > 1e8f) Q2 = 1e8f;
+    if (Q2 < 1.f) Q2 = 1.f;
+    Q[s] = cp_sqrtf(Q2);
+    lnQ[s] = 0.5f * cp_logf(Q2);
+    invQ[s] = cp_rcp(Q[s]);
+  }
   CpBeamX A, B;
   cp_beams_x(lnxA, lnxAL, lnxB, lnxBL, A, B);
 #pragma unroll UNROLL
   for (int i = 0; i < 8; ++i) {
     const CpCteqPoly c = cp_load_poly(cteq + i);
-    const CpCteqQ a = cp_cteq_coef(c, lnQ, Q, invQ, cp_cteq_has_qmin(i));
-    const CpF2 r = cp_cteq_answer2(c, a, A, B, cp_cteq_uses_x1l(i));
-    float ra = r.x, rb = r.y;
-    // parametrisation 4 is the dbar/ubar ratio; the others are x * answer
-    if (i != 4) { ra *= A.x; rb *= B.x; }
+    const CpCteqX cx = cp_cteq_x(c, A, B, cp_cteq_uses_x1l(i));
 #pragma unroll
-    for (int k = 0; k < 8; ++k)
-      if (k == i) { fa[k] = ra; fb[k] = rb; }
-  }
-  // ubar and dbar from (ubar + dbar) and dbar/ubar: PartonDistributions.cc:1053-1054
-  const CpF2 iab = cp_rcp2(cp_f2(1.f + fa[4], 1.f + fb[4]));
-  const float ia = iab.x, ib = iab.y;
-  float sa = fa[3], sb = fb[3];
-  fa[3] = sa * ia; fa[4] = sa * fa[4] * ia;
-  fb[3] = sb * ib; fb[4] = sb * fb[4] * ib;
-  // max(0, .) of PDF::xf (PartonDistributions.cc:133-180)
+    for (int s = 0; s < NS; ++s) {
+      const CpCteqQ a = cp_cteq_coef(c, lnQ[s], Q[s], invQ[s], cp_cteq_has_qmin(i));
+      const CpF2 r = cp_cteq_answer2(cx, a, A, B);
+      float ra = r.x, rb = r.y;
+      // parametrisation 4 is the dbar/ubar ratio; the others are x * answer
+      if (i != 4) { ra *= A.x; rb *= B.x; }
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    fa[k] = fa[k] > 0.f ? fa[k] : 0.f;
-    fb[k] = fb[k] > 0.f ? fb[k] : 0.f;
+      for (int k = 0; k < 8; ++k)
+        if (k == i) { fa[s][k] = ra; fb[s][k] = rb; }
+    }
   }
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    // ubar and dbar from (ubar + dbar) and dbar/ubar: PartonDistributions.cc:1053-1054
+    const CpF2 iab = cp_rcp2(cp_f2(1.f + fa[s][4], 1.f + fb[s][4]));
+    const float ia = iab.x, ib = iab.y;
+    float sa = fa[s][3], sb = fb[s][3];
+    fa[s][3] = sa * ia; fa[s][4] = sa * fa[s][4] * ia;
+    fb[s][3] = sb * ib; fb[s][4] = sb * fb[s][4] * ib;
+    // max(0, .) of PDF::xf (PartonDistributions.cc:133-180)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      fa[s][k] = fa[s][k] > 0.f ? fa[s][k] : 0.f;
+      fb[s][k] = fb[s][k] > 0.f ? fb[s][k] : 0.f;
+    }
+  }
+}
+
+// The same at one scale.
+template <int UNROLL = 8>
+CP_HD void cp_cteq_pair(const CpCteqPoly* cteq, float Q2, float lnxA, float lnxAL, float lnxB,
+                        float lnxBL, float fa[8], float fb[8])
+{
+  float ga[1][8], gb[1][8];
+  cp_cteq_scales<1, UNROLL>(cteq, &Q2, lnxA, lnxAL, lnxB, lnxBL, ga, gb);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) { fa[k] = ga[0][k]; fb[k] = gb[0][k]; }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -563,14 +601,14 @@ CP_HD void cp_scale_ratios(const CpHadParams& P, const CpCteqPoly* cteq, const C
     return;
   }
   const float f2[2] = {4.f, 0.25f};
-  float rR[2], rF[2];
-#pragma unroll 1
+  const float Q2[2] = {P.kF * f2[0] * pt.k.pT2, P.kF * f2[1] * pt.k.pT2};
+  float rR[2], rF[2], fa[2][8], fb[2][8];
+  cp_cteq_scales<2, 1>(cteq, Q2, pt.k.lnx1, pt.k.lnx1L, pt.k.lnx2, pt.k.lnx2L, fa, fb);
+#pragma unroll
   for (int j = 0; j < 2; ++j) {
     const float a = cp_alphas(P, P.kR * f2[j] * pt.k.pT2) / pt.k.alphaS;
     rR[j] = a * a;
-    float fa[8], fb[8];
-    cp_cteq_pair<1>(cteq, P.kF * f2[j] * pt.k.pT2, pt.k.lnx1, pt.k.lnx1L, pt.k.lnx2, pt.k.lnx2L, fa, fb);
-    rF[j] = cp_channel_sum(P.mask, pt.b, fa, fb) / B0;
+    rF[j] = cp_channel_sum(P.mask, pt.b, fa[j], fb[j]) / B0;
   }
   out[0] = rR[0]; out[1] = rR[1]; out[2] = rF[0]; out[3] = rF[1];
   out[4] = rR[0] * rF[0]; out[5] = rR[1] * rF[1];
