@@ -157,6 +157,104 @@ __device__ __forceinline__ void cp_flow_mlp_tile(const uint2* __restrict__ pk, c
   o[3] = hi ? y3 : y1;
 }
 
+// Pieces of the two-tile form: a warp's 32 points are two 16-row tiles (rows = lanes 0..15 and
+// 16..31), taken together so that every weight fragment is loaded once for both and four accumulator
+// chains run side by side.  Per tile the products and their order are cp_flow_mlp_tile's.
+
+// layer-1 A fragments of both tiles from the lanes' input features
+__device__ __forceinline__ void cp_flow_in_frags(float in0, float in1, uint32_t a[2][4])
+{
+  const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const float r0a = __shfl_sync(0xffffffffu, in0, 16 * t + gid), r0b = __shfl_sync(0xffffffffu, in1, 16 * t + gid);
+    const float r8a = __shfl_sync(0xffffffffu, in0, 16 * t + gid + 8), r8b = __shfl_sync(0xffffffffu, in1, 16 * t + gid + 8);
+    a[t][0] = tig == 0 ? cp_bf2(r0a, r0b) : 0u;
+    a[t][1] = tig == 0 ? cp_bf2(r8a, r8b) : 0u;
+    a[t][2] = 0u;
+    a[t][3] = 0u;
+  }
+}
+
+// one 64-wide layer of KT k-tiles for both tiles: h = bf16(ReLU(A W + b)) as A fragments
+template <int KT>
+__device__ __forceinline__ void cp_flow_layer64(const uint32_t (&a)[2][KT][4], const uint2* __restrict__ pk,
+                                                const float* __restrict__ bias, uint32_t (&h)[2][4][4])
+{
+  const int lane = threadIdx.x & 31, tig = lane & 3;
+#pragma unroll
+  for (int k2 = 0; k2 < 4; ++k2) {   // hidden units 16 k2 .. + 15: n-tiles 2 k2 and 2 k2 + 1
+    float acc[2][2][4];              // [n-tile][tile]
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float b0 = bias[(2 * k2 + j) * 8 + 2 * tig], b1 = bias[(2 * k2 + j) * 8 + 2 * tig + 1];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) { acc[j][t][0] = b0; acc[j][t][1] = b1; acc[j][t][2] = b0; acc[j][t][3] = b1; }
+    }
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint2 w = pk[(kt * 8 + 2 * k2 + j) * 32 + lane];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) cp_mma_bf16(acc[j][t], a[t][kt], w);
+      }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        h[t][k2][2 * j] = cp_bf2(fmaxf(acc[j][t][0], 0.f), fmaxf(acc[j][t][1], 0.f));
+        h[t][k2][2 * j + 1] = cp_bf2(fmaxf(acc[j][t][2], 0.f), fmaxf(acc[j][t][3], 0.f));
+      }
+  }
+}
+
+// output layer of both tiles; o = the output columns 0..3 of this lane's own row
+__device__ __forceinline__ void cp_flow_layer_out(const uint32_t (&h)[2][4][4], const uint2* __restrict__ pk,
+                                                  const float* __restrict__ bias, float o[4])
+{
+  const int lane = threadIdx.x & 31, tig = lane & 3;
+  float c3[2][4];
+  const float b0 = bias[2 * tig], b1 = bias[2 * tig + 1];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) { c3[t][0] = b0; c3[t][1] = b1; c3[t][2] = b0; c3[t][3] = b1; }
+#pragma unroll
+  for (int kt = 0; kt < 4; ++kt) {
+    const uint2 w = pk[kt * 32 + lane];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) cp_mma_bf16(c3[t], h[t][kt], w);
+  }
+  // row r of a tile: columns 0, 1 in lane 4 (r % 8), 2, 3 in the next; rows 8..15 in the upper pair
+  const int r = lane & 15, src = 4 * (r & 7);
+  const bool hi = r >= 8, second = lane >= 16;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float x0 = __shfl_sync(0xffffffffu, c3[0][q & 1], src + (q >> 1));
+    const float x2 = __shfl_sync(0xffffffffu, c3[0][2 + (q & 1)], src + (q >> 1));
+    const float y0 = __shfl_sync(0xffffffffu, c3[1][q & 1], src + (q >> 1));
+    const float y2 = __shfl_sync(0xffffffffu, c3[1][2 + (q & 1)], src + (q >> 1));
+    o[q] = second ? (hi ? y2 : y0) : (hi ? x2 : x0);
+  }
+}
+
+// MLP of a coupling for the warp's 32 points: o = this lane's outputs
+__device__ __forceinline__ void cp_flow_mlp_warp(const uint2* __restrict__ pk, const float* __restrict__ b, float in0,
+                                                 float in1, float o[4])
+{
+  uint32_t a[2][1][4], h1[2][4][4], h2[2][4][4];
+  {
+    uint32_t f[2][4];
+    cp_flow_in_frags(in0, in1, f);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) a[t][0][q] = f[t][q];
+  }
+  cp_flow_layer64<1>(a, pk + CP_FLOW_P_W1, b, h1);
+  cp_flow_layer64<4>(h1, pk + CP_FLOW_P_W2, b + 64, h2);
+  cp_flow_layer_out(h2, pk + CP_FLOW_P_W3, b + 128, o);
+}
+
 // Flow of one point per lane (all 32 lanes active): z in, z out, logdet accumulated.  pk is the
 // packed-fragment array of all couplings (shared memory), bias arrays per coupling.
 __device__ __forceinline__ void cp_flow_couplings(const uint2* __restrict__ pk, const float* __restrict__ biases,

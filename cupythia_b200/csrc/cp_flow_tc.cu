@@ -621,7 +621,7 @@ int cp_flow_tc_status(cp_handle* h)
   const bool wgrad = h->mail->status[1] != 0;
   if (!h->mail->status[0] && !wgrad) return CP_OK;
   h->mail->status[0] = h->mail->status[1] = 0;
-  return cp_fail(h, CP_ERR_TIMEOUT, wgrad ? "k_flow_wgrad_tc: a tensor-core wait expired (this training step's gradient is invalid)"
+  return cp_fail(h, CP_ERR_TIMEOUT, wgrad ? "flow training: a tensor-core or weight-copy wait expired (this training step is invalid)"
                                             : "k_flow_fwd_tc / k_flow_accept_tc: a tensor-core wait expired (results of this pass are invalid)");
 }
 

@@ -47,33 +47,60 @@ struct FlowTrainBufs {
   float* gpart;        // [CP_WG_MAXBLK][CP_FLOW_NPARAM] per-block weight and bias gradients
 };
 
-__device__ __forceinline__ float cp_bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
-__device__ __forceinline__ float cp_bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
-
 // ------------------------------------------------------------------------------------------
 // 1. forward, saving the input z of every coupling
 // ------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(CP_THREADS, 2) k_flow_fwd_train(const uint2* __restrict__ pk_g, const float* __restrict__ bias_g,
+// One block of 16 warps per SM: the weight fragments arrive in its shared memory once, by bulk copies
+// that run while the warps draw and map their points (element copies by two blocks of 8 warps cost
+// a third of the kernel: 65,536 points 26.4 -> 17.6 us).
+#define CP_TRAIN_THREADS 512
+
+// Starts the copies of the first `count` fragments of every coupling into shared memory (one thread,
+// which has initialised the barrier), and the bounded wait for them (whole warps; on expiry the
+// status word is raised and the copies get one more bounded wait before the warp may leave).
+__device__ __forceinline__ void cp_train_weights_load(uint32_t bar, uint2* dst, const uint2* __restrict__ pk_g, int count)
+{
+  const uint32_t bytes = (uint32_t)count * (uint32_t)sizeof(uint2);
+  cp_mbar_expect_tx(bar, CP_FLOW_NC * bytes);
+  for (int c = 0; c < CP_FLOW_NC; ++c) cp_bulk_load(cp_smem_u32(dst + c * count), pk_g + c * CP_FLOW_P_PER, bytes, bar);
+}
+__device__ __forceinline__ bool cp_train_weights_wait(uint32_t bar, int* __restrict__ status)
+{
+  volatile int gave_up = 0;
+  if (__all_sync(0xffffffffu, cp_mbar_wait_bounded(bar, 0u, &gave_up))) return true;
+  *(volatile int*)status = 1;
+  gave_up = 0;
+  cp_mbar_wait_bounded(bar, 0u, &gave_up);
+  __syncwarp();
+  return false;
+}
+
+__global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_fwd_train(const uint2* __restrict__ pk_g, const float* __restrict__ bias_g,
                                                                const double* __restrict__ edges, int nb,
                                                                uint64_t seed, uint32_t iter, uint32_t stream, uint64_t point0,
-                                                               uint64_t n, float* __restrict__ zs, float4* __restrict__ vj)
+                                                               uint64_t n, float* __restrict__ zs, float4* __restrict__ vj,
+                                                               int* __restrict__ status)
 {
-  extern __shared__ uint2 sPk[];
+  extern __shared__ __align__(16) uint2 sPk[];
   float* sBias = reinterpret_cast<float*>(sPk + CP_FLOW_NC * CP_FLOW_P_FWD);
   __shared__ float2 sEdge[3][CP_MAX_BINS];
-  for (int k = threadIdx.x; k < 3 * nb; k += CP_THREADS) {
+  __shared__ __align__(8) uint64_t sBar;
+  const uint32_t bar = cp_smem_u32(&sBar);
+  if (threadIdx.x == 0) {
+    cp_mbar_init(bar, 1);
+    cp_mbar_init_fence();
+    cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_FWD);
+  }
+  for (int k = threadIdx.x; k < 3 * nb; k += CP_TRAIN_THREADS) {
     const int d = k / nb, b = k - d * nb;
     sEdge[d][b] = make_float2((float)edges[d * (nb + 1) + b], (float)(edges[d * (nb + 1) + b + 1] - edges[d * (nb + 1) + b]));
   }
-  for (int c = 0; c < CP_FLOW_NC; ++c)
-    for (int e = threadIdx.x; e < CP_FLOW_P_FWD; e += CP_THREADS) sPk[c * CP_FLOW_P_FWD + e] = pk_g[c * CP_FLOW_P_PER + e];
-  for (int j = threadIdx.x; j < CP_FLOW_NC * CP_FLOW_NB; j += CP_THREADS) sBias[j] = bias_g[j];
+  for (int j = threadIdx.x; j < CP_FLOW_NC * CP_FLOW_NB; j += CP_TRAIN_THREADS) sBias[j] = bias_g[j];
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const uint64_t stride = (uint64_t)gridDim.x * CP_THREADS;
+  const uint64_t stride = (uint64_t)gridDim.x * CP_TRAIN_THREADS;
   const uint64_t rounds = (n + stride - 1) / stride;
   for (uint64_t r = 0; r < rounds; ++r) {
-    const uint64_t p = r * stride + (uint64_t)blockIdx.x * CP_THREADS + threadIdx.x;
+    const uint64_t p = r * stride + (uint64_t)blockIdx.x * CP_TRAIN_THREADS + threadIdx.x;
     const bool active = p < n;
     float z[3], jv = 1.f, logdet = 0.f;
     uint32_t w[4] = {0x80000000u, 0x80000000u, 0x80000000u, 0u};
@@ -84,17 +111,15 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_flow_fwd_train(const uint2* _
       logdet += cp_flow_logit(cp_flow_vegas_in(sEdge[d], nb, w[d], jv, bin), z[d]);
     }
     logdet += logf(jv);
+    if (r == 0 && !cp_train_weights_wait(bar, status)) return;   // no barrier follows
 #pragma unroll 1
     for (int c = 0; c < CP_FLOW_NC; ++c) {
       if (active)
         for (int d = 0; d < 3; ++d) zs[(p * CP_FLOW_NC + c) * 3 + d] = z[d];
       const CpCoupling k = cp_coupling(c);
       const float* b = sBias + c * CP_FLOW_NB;
-      float o0[4], o1[4], o[4];
-      cp_flow_mlp_tile(sPk + c * CP_FLOW_P_FWD, b, b + 64, b + 128, z[k.cin[0]], z[k.cin[1]], k.nin, 0, o0);
-      cp_flow_mlp_tile(sPk + c * CP_FLOW_P_FWD, b, b + 64, b + 128, z[k.cin[0]], z[k.cin[1]], k.nin, 16, o1);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) o[q] = lane >= 16 ? o1[q] : o0[q];
+      float o[4];
+      cp_flow_mlp_warp(sPk + c * CP_FLOW_P_FWD, b, z[k.cin[0]], k.nin > 1 ? z[k.cin[1]] : 0.f, o);
       for (int j = 0; j < k.nt; ++j) {
         const float s = CP_FLOW_S * tanhf(o[j] / CP_FLOW_S);
         z[k.tr[j]] = fmaf(z[k.tr[j]], expf(s), o[k.nt + j]);
@@ -115,7 +140,10 @@ __global__ void __launch_bounds__(CP_THREADS, 2) k_flow_fwd_train(const uint2* _
 // ticket, after a fence) adds all slots in a fixed order (strided per-thread sums, the xor tree
 // of each warp, the warps in order) into moments[0..1], writes the batch loss <w^2>/<w>^2 over
 // n_loss points when loss != null, and re-arms the ticket.
-__global__ void __launch_bounds__(128) k_flow_igrad(const CpHadParams P, const CpCteqPoly* __restrict__ cteq_g,
+// Four blocks per SM (128 registers, some spilled): the 2048 warps of 65,536 points are then resident
+// at once; at the 190 registers it would take, eight warps per SM ran in two waves (65,536
+// points 27.5 -> 26.7 us).
+__global__ void __launch_bounds__(128, 4) k_flow_igrad(const CpHadParams P, const CpCteqPoly* __restrict__ cteq_g,
                                                     uint64_t n, float lnTauMin, const float4* __restrict__ vj,
                                                     float4* __restrict__ wg, double* __restrict__ slots,
                                                     unsigned* __restrict__ ticket, double* __restrict__ moments,
@@ -191,7 +219,7 @@ __global__ void __launch_bounds__(128) k_flow_igrad(const CpHadParams P, const C
 // writes a 16 x 64 bf16 tile held as A fragments: register (kt, 0 | 1) is the core matrix of feature
 // group 2 kt and the tile's first | second 8 points, (kt, 2 | 3) that of group 2 kt + 1.  `dst`: the
 // tile's first point group in its stage + 4 lane; ra, rb: this lane's two rows lie inside the batch
-__device__ __forceinline__ void cp_store_rowfrag(uint8_t* dst, bool ra, bool rb, const uint32_t h[4][4])
+__device__ __forceinline__ void cp_store_rowfrag(uint8_t* dst, bool ra, bool rb, const uint32_t (&h)[4][4])
 {
 #pragma unroll
   for (int kt = 0; kt < 4; ++kt) {
@@ -207,15 +235,69 @@ __device__ __forceinline__ void cp_store_rowfrag(uint8_t* dst, bool ra, bool rb,
   }
 }
 
-#define CP_BWD_THREADS 256   // 8 warps; the 92 KB of staged fragments admit two blocks per SM
-__global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __restrict__ pk_g, const float* __restrict__ bias_g, uint64_t n,
+// ReLU masks of a tile's activations (A fragments, non-negative): bit 4 nt + e for element e of
+// n-tile nt's accumulator, set where the activation is above zero
+__device__ __forceinline__ uint32_t cp_relu_mask(const uint32_t (&h)[4][4])
+{
+  uint32_t m = 0u;
+#pragma unroll
+  for (int kt = 0; kt < 4; ++kt)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int bit = 4 * (2 * kt + (q >> 1)) + 2 * (q & 1);
+      if (h[kt][q] & 0x00007fffu) m |= 1u << bit;
+      if (h[kt][q] & 0x7fff0000u) m |= 2u << bit;
+    }
+  return m;
+}
+
+// one 64-wide backward product of KT k-tiles for both tiles: d = bf16(mask (A W)) as A fragments
+template <int KT>
+__device__ __forceinline__ void cp_flow_back64(const uint32_t (&a)[2][KT][4], const uint2* __restrict__ pk,
+                                               const uint32_t (&keep)[2], uint32_t (&d)[2][4][4])
+{
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int k2 = 0; k2 < 4; ++k2) {
+    float acc[2][2][4] = {};   // [n-tile][tile]
+#pragma unroll
+    for (int kt = 0; kt < KT; ++kt)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint2 w = pk[(kt * 8 + 2 * k2 + j) * 32 + lane];
+#pragma unroll
+        for (int t = 0; t < 2; ++t) cp_mma_bf16(acc[j][t], a[t][kt], w);
+      }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float m[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) m[e] = (keep[t] >> (4 * (2 * k2 + j) + e)) & 1u ? acc[j][t][e] : 0.f;
+        d[t][k2][2 * j] = cp_bf2(m[0], m[1]);
+        d[t][k2][2 * j + 1] = cp_bf2(m[2], m[3]);
+      }
+  }
+}
+
+// One block of 16 warps per SM, the 88 KB of weight fragments by bulk copies, as in the forward
+// (65,536 points 53 -> 46.6 us).  The two tiles of a warp go together and only bit masks of the
+// activations are kept; that by itself measured no faster than a tile at a time.
+__global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_bwd(const uint2* __restrict__ pk_g, const float* __restrict__ bias_g, uint64_t n,
                                                   double n_batch, const float* __restrict__ zs, const float4* __restrict__ vj,
                                                   const float4* __restrict__ wg, const double* __restrict__ sums,
-                                                  FlowTrainBufs out, float loss_p)
+                                                  FlowTrainBufs out, float loss_p, int* __restrict__ status)
 {
-  extern __shared__ uint2 sPk[];   // all CP_FLOW_P_PER fragments of the 4 couplings, then biases
+  extern __shared__ __align__(16) uint2 sPk[];   // all CP_FLOW_P_PER fragments of the 4 couplings, then biases
   float* sBias = reinterpret_cast<float*>(sPk + CP_FLOW_NC * CP_FLOW_P_PER);
-  for (int e = threadIdx.x; e < CP_FLOW_NC * CP_FLOW_P_PER; e += blockDim.x) sPk[e] = pk_g[e];
+  __shared__ __align__(8) uint64_t sBar;
+  const uint32_t bar = cp_smem_u32(&sBar);
+  if (threadIdx.x == 0) {
+    cp_mbar_init(bar, 1);
+    cp_mbar_init_fence();
+    cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_PER);
+  }
   for (int j = threadIdx.x; j < CP_FLOW_NC * CP_FLOW_NB; j += blockDim.x) sBias[j] = bias_g[j];
   __syncthreads();
   const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
@@ -238,6 +320,7 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
       // sigmoid: dv/dz = v (1 - v); d ln(v (1 - v))/dz = 1 - 2 v
       for (int d = 0; d < 3; ++d) dz[d] = cJ * gv[d] * v[d] * (1.f - v[d]) + cJ * (1.f - 2.f * v[d]);
     }
+    if (r == 0 && !cp_train_weights_wait(bar, status)) return;   // no barrier follows
 #pragma unroll 1
     for (int c = CP_FLOW_NC - 1; c >= 0; --c) {
       const CpCoupling k = cp_coupling(c);
@@ -247,146 +330,117 @@ __global__ void __launch_bounds__(CP_BWD_THREADS, 2) k_flow_bwd(const uint2* __r
       if (active)
         for (int d = 0; d < 3; ++d) zin[d] = zs[(p * CP_FLOW_NC + c) * 3 + d];
       const float in0 = zin[k.cin[0]], in1 = k.nin > 1 ? zin[k.cin[1]] : 0.f;
-      const uint64_t st0 = (uint64_t)c * out.nst;
-#pragma unroll 1
-      for (int tile = 0; tile < 2; ++tile) {
-        const int tb = 16 * tile;
-        const uint64_t row0 = base + tb;
-        const bool rowa = row0 + gid < n, rowb = row0 + gid + 8 < n;
-        // this lane's word of the tile's first core matrix in its stage (16- and 64-wide arrays)
-        const uint64_t stage = st0 + row0 / CP_WGT_STAGE;
+      // this lane's word of each tile's first core matrix in its stage (16- and 64-wide arrays)
+      size_t at16[2], at64[2];
+      bool rowa[2], rowb[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const uint64_t row0 = base + 16 * t;
+        rowa[t] = row0 + gid < n;
+        rowb[t] = row0 + gid + 8 < n;
+        const uint64_t stage = (uint64_t)c * out.nst + row0 / CP_WGT_STAGE;
         const uint32_t inst = (uint32_t)(row0 % CP_WGT_STAGE) * 16u + 4u * lane;
-        const size_t at16 = stage * CP_WGT_BYTES(16) + inst, at64 = stage * CP_WGT_BYTES(64) + inst;
-        // ---- recompute the MLP forward of this tile (A fragments kept for the ReLU masks)
-        float r0a = __shfl_sync(0xffffffffu, in0, tb + gid), r0b = __shfl_sync(0xffffffffu, in1, tb + gid);
-        float r8a = __shfl_sync(0xffffffffu, in0, tb + gid + 8), r8b = __shfl_sync(0xffffffffu, in1, tb + gid + 8);
-        uint32_t a[4] = {tig == 0 ? cp_bf2(r0a, r0b) : 0u, tig == 0 ? cp_bf2(r8a, r8b) : 0u, 0u, 0u};
-        if (rowa) *reinterpret_cast<uint32_t*>(out.X + at16) = a[0];
-        if (rowb) *reinterpret_cast<uint32_t*>(out.X + at16 + 128) = a[1];
-        float acc[8][4];
-        uint32_t h1[4][4], h2[4][4];
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const float b0 = b[nt * 8 + 2 * tig], b1 = b[nt * 8 + 2 * tig + 1];
-          acc[nt][0] = b0; acc[nt][1] = b1; acc[nt][2] = b0; acc[nt][3] = b1;
-          cp_mma_bf16(acc[nt], a, pk[CP_FLOW_P_W1 + nt * 32 + lane]);
-        }
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          h1[kt][0] = cp_bf2(fmaxf(acc[2 * kt][0], 0.f), fmaxf(acc[2 * kt][1], 0.f));
-          h1[kt][1] = cp_bf2(fmaxf(acc[2 * kt][2], 0.f), fmaxf(acc[2 * kt][3], 0.f));
-          h1[kt][2] = cp_bf2(fmaxf(acc[2 * kt + 1][0], 0.f), fmaxf(acc[2 * kt + 1][1], 0.f));
-          h1[kt][3] = cp_bf2(fmaxf(acc[2 * kt + 1][2], 0.f), fmaxf(acc[2 * kt + 1][3], 0.f));
-        }
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const float b0 = b[64 + nt * 8 + 2 * tig], b1 = b[64 + nt * 8 + 2 * tig + 1];
-          acc[nt][0] = b0; acc[nt][1] = b1; acc[nt][2] = b0; acc[nt][3] = b1;
-#pragma unroll
-          for (int kt = 0; kt < 4; ++kt) cp_mma_bf16(acc[nt], h1[kt], pk[CP_FLOW_P_W2 + (kt * 8 + nt) * 32 + lane]);
-        }
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          h2[kt][0] = cp_bf2(fmaxf(acc[2 * kt][0], 0.f), fmaxf(acc[2 * kt][1], 0.f));
-          h2[kt][1] = cp_bf2(fmaxf(acc[2 * kt][2], 0.f), fmaxf(acc[2 * kt][3], 0.f));
-          h2[kt][2] = cp_bf2(fmaxf(acc[2 * kt + 1][0], 0.f), fmaxf(acc[2 * kt + 1][1], 0.f));
-          h2[kt][3] = cp_bf2(fmaxf(acc[2 * kt + 1][2], 0.f), fmaxf(acc[2 * kt + 1][3], 0.f));
-        }
-        cp_store_rowfrag(out.H1 + at64, rowa, rowb, h1);
-        cp_store_rowfrag(out.H2 + at64, rowa, rowb, h2);
-        float c3[4] = {b[128 + 2 * tig], b[128 + 2 * tig + 1], b[128 + 2 * tig], b[128 + 2 * tig + 1]};
-#pragma unroll
-        for (int kt = 0; kt < 4; ++kt) cp_mma_bf16(c3, h2[kt], pk[CP_FLOW_P_W3 + kt * 32 + lane]);
-        // ---- this tile's rows: outputs to the point lanes, coupling backward there
-        const int rr = (lane - tb) & 15, src = 4 * (rr & 7);
-        const bool hi = rr >= 8, mine = lane >= tb && lane < tb + 16;
-        float o[4];
+        at16[t] = stage * CP_WGT_BYTES(16) + inst;
+        at64[t] = stage * CP_WGT_BYTES(64) + inst;
+      }
+      // ---- the MLP forward again; of the activations only the ReLU masks stay
+      float o[4];
+      uint32_t keep1[2], keep2[2];
+      {
+        uint32_t a[2][1][4], h1[2][4][4], h2[2][4][4];
         {
-          float x0 = __shfl_sync(0xffffffffu, c3[0], src), x1 = __shfl_sync(0xffffffffu, c3[1], src);
-          float x2 = __shfl_sync(0xffffffffu, c3[2], src), x3 = __shfl_sync(0xffffffffu, c3[3], src);
-          float y0 = __shfl_sync(0xffffffffu, c3[0], src + 1), y1 = __shfl_sync(0xffffffffu, c3[1], src + 1);
-          float y2 = __shfl_sync(0xffffffffu, c3[2], src + 1), y3 = __shfl_sync(0xffffffffu, c3[3], src + 1);
-          o[0] = hi ? x2 : x0; o[1] = hi ? x3 : x1; o[2] = hi ? y2 : y0; o[3] = hi ? y3 : y1;
-        }
-        float dO[4] = {0.f, 0.f, 0.f, 0.f};
-        float dzT[2] = {0.f, 0.f};
-        if (mine && active) {
-          for (int j = 0; j < k.nt; ++j) {
-            const float th = tanhf(o[j] / CP_FLOW_S), s = CP_FLOW_S * th, e = expf(s);
-            const int d = k.tr[j];
-            const float dzo = dz[d];
-            const float ds = fmaf(dzo * zin[d], e, cJ);
-            dO[j] = ds * (1.f - th * th);
-            dO[k.nt + j] = dzo;
-            dzT[j] = dzo * e;
+          uint32_t f[2][4];
+          cp_flow_in_frags(in0, in1, f);
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) a[t][0][q] = f[t][q];
+            if (rowa[t]) *reinterpret_cast<uint32_t*>(out.X + at16[t]) = f[t][0];
+            if (rowb[t]) *reinterpret_cast<uint32_t*>(out.X + at16[t] + 128) = f[t][1];
           }
         }
-        // dO as an A fragment: columns 0..3, rows gid and gid + 8
-        // (a shuffle sends the value the source lane holds, so fetch all four and select here)
+        cp_flow_layer64<1>(a, pk + CP_FLOW_P_W1, b, h1);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          cp_store_rowfrag(out.H1 + at64[t], rowa[t], rowb[t], h1[t]);
+          keep1[t] = cp_relu_mask(h1[t]);
+        }
+        cp_flow_layer64<4>(h1, pk + CP_FLOW_P_W2, b + 64, h2);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          cp_store_rowfrag(out.H2 + at64[t], rowa[t], rowb[t], h2[t]);
+          keep2[t] = cp_relu_mask(h2[t]);
+        }
+        cp_flow_layer_out(h2, pk + CP_FLOW_P_W3, b + 128, o);
+      }
+      // ---- coupling backward of this lane's point
+      float dO[4] = {0.f, 0.f, 0.f, 0.f}, dzT[2] = {0.f, 0.f};
+      if (active) {
+        for (int j = 0; j < k.nt; ++j) {
+          const float th = tanhf(o[j] / CP_FLOW_S), s = CP_FLOW_S * th, e = expf(s);
+          const int d = k.tr[j];
+          const float dzo = dz[d];
+          const float ds = fmaf(dzo * zin[d], e, cJ);
+          dO[j] = ds * (1.f - th * th);
+          dO[k.nt + j] = dzo;
+          dzT[j] = dzo * e;
+        }
+      }
+      // dO as A fragments: columns 0..3, rows gid and gid + 8 of each tile
+      // (a shuffle sends the value the source lane holds, so fetch all four and select here)
+      uint32_t ad[2][4];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
         float g0[4], g8[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          g0[q] = __shfl_sync(0xffffffffu, dO[q], tb + gid);
-          g8[q] = __shfl_sync(0xffffffffu, dO[q], tb + gid + 8);
+          g0[q] = __shfl_sync(0xffffffffu, dO[q], 16 * t + gid);
+          g8[q] = __shfl_sync(0xffffffffu, dO[q], 16 * t + gid + 8);
         }
         const bool odd = tig & 1;
-        uint32_t ad[4] = {tig < 2 ? cp_bf2(odd ? g0[2] : g0[0], odd ? g0[3] : g0[1]) : 0u,
-                          tig < 2 ? cp_bf2(odd ? g8[2] : g8[0], odd ? g8[3] : g8[1]) : 0u, 0u, 0u};
-        if (rowa) *reinterpret_cast<uint32_t*>(out.DO + at16) = ad[0];
-        if (rowb) *reinterpret_cast<uint32_t*>(out.DO + at16 + 128) = ad[1];
-        // dH2 = dO W3^T, masked by the ReLU of layer 2
+        ad[t][0] = tig < 2 ? cp_bf2(odd ? g0[2] : g0[0], odd ? g0[3] : g0[1]) : 0u;
+        ad[t][1] = tig < 2 ? cp_bf2(odd ? g8[2] : g8[0], odd ? g8[3] : g8[1]) : 0u;
+        ad[t][2] = ad[t][3] = 0u;
+        if (rowa[t]) *reinterpret_cast<uint32_t*>(out.DO + at16[t]) = ad[t][0];
+        if (rowb[t]) *reinterpret_cast<uint32_t*>(out.DO + at16[t] + 128) = ad[t][1];
+      }
+      // dH2 = dO W3^T, masked by the ReLU of layer 2
+      uint32_t d2[2][4][4], d1[2][4][4];
+      {
+        uint32_t a[2][1][4];
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-          cp_mma_bf16(acc[nt], ad, pk[CP_FLOW_P_W3T + nt * 32 + lane]);
-          const uint32_t m01 = h2[nt >> 1][(nt & 1) ? 2 : 0], m23 = h2[nt >> 1][(nt & 1) ? 3 : 1];
-          if (cp_bf_lo(m01) <= 0.f) acc[nt][0] = 0.f;
-          if (cp_bf_hi(m01) <= 0.f) acc[nt][1] = 0.f;
-          if (cp_bf_lo(m23) <= 0.f) acc[nt][2] = 0.f;
-          if (cp_bf_hi(m23) <= 0.f) acc[nt][3] = 0.f;
-        }
-        uint32_t d2[4][4];
+        for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          d2[kt][0] = cp_bf2(acc[2 * kt][0], acc[2 * kt][1]);
-          d2[kt][1] = cp_bf2(acc[2 * kt][2], acc[2 * kt][3]);
-          d2[kt][2] = cp_bf2(acc[2 * kt + 1][0], acc[2 * kt + 1][1]);
-          d2[kt][3] = cp_bf2(acc[2 * kt + 1][2], acc[2 * kt + 1][3]);
-        }
-        cp_store_rowfrag(out.D2 + at64, rowa, rowb, d2);
-        // dH1 = dH2 W2^T, masked by the ReLU of layer 1
+          for (int q = 0; q < 4; ++q) a[t][0][q] = ad[t][q];
+        cp_flow_back64<1>(a, pk + CP_FLOW_P_W3T, keep2, d2);
+      }
 #pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+      for (int t = 0; t < 2; ++t) cp_store_rowfrag(out.D2 + at64[t], rowa[t], rowb[t], d2[t]);
+      // dH1 = dH2 W2^T, masked by the ReLU of layer 1
+      cp_flow_back64<4>(d2, pk + CP_FLOW_P_W2T, keep1, d1);
 #pragma unroll
-          for (int kt = 0; kt < 4; ++kt) cp_mma_bf16(acc[nt], d2[kt], pk[CP_FLOW_P_W2T + (kt * 8 + nt) * 32 + lane]);
-          const uint32_t m01 = h1[nt >> 1][(nt & 1) ? 2 : 0], m23 = h1[nt >> 1][(nt & 1) ? 3 : 1];
-          if (cp_bf_lo(m01) <= 0.f) acc[nt][0] = 0.f;
-          if (cp_bf_hi(m01) <= 0.f) acc[nt][1] = 0.f;
-          if (cp_bf_lo(m23) <= 0.f) acc[nt][2] = 0.f;
-          if (cp_bf_hi(m23) <= 0.f) acc[nt][3] = 0.f;
-        }
-        uint32_t d1[4][4];
+      for (int t = 0; t < 2; ++t) cp_store_rowfrag(out.D1 + at64[t], rowa[t], rowb[t], d1[t]);
+      // dX = dH1 W1^T: columns 0..1 are the gradients of the two input features
+      float cx[2][4] = {};
 #pragma unroll
-        for (int kt = 0; kt < 4; ++kt) {
-          d1[kt][0] = cp_bf2(acc[2 * kt][0], acc[2 * kt][1]);
-          d1[kt][1] = cp_bf2(acc[2 * kt][2], acc[2 * kt][3]);
-          d1[kt][2] = cp_bf2(acc[2 * kt + 1][0], acc[2 * kt + 1][1]);
-          d1[kt][3] = cp_bf2(acc[2 * kt + 1][2], acc[2 * kt + 1][3]);
-        }
-        cp_store_rowfrag(out.D1 + at64, rowa, rowb, d1);
-        // dX = dH1 W1^T: columns 0..1 are the gradients of the two input features
-        float cx[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int kt = 0; kt < 4; ++kt) {
+        const uint2 w = pk[CP_FLOW_P_W1T + kt * 32 + lane];
 #pragma unroll
-        for (int kt = 0; kt < 4; ++kt) cp_mma_bf16(cx, d1[kt], pk[CP_FLOW_P_W1T + kt * 32 + lane]);
-        const float e0 = __shfl_sync(0xffffffffu, cx[0], src), e1 = __shfl_sync(0xffffffffu, cx[1], src);
-        const float e2 = __shfl_sync(0xffffffffu, cx[2], src), e3 = __shfl_sync(0xffffffffu, cx[3], src);
-        if (mine && active) {
-          const float dx0 = hi ? e2 : e0, dx1 = hi ? e3 : e1;
-          for (int j = 0; j < k.nt; ++j) dz[k.tr[j]] = dzT[j];
-          dz[k.cin[0]] += dx0;
-          if (k.nin > 1) dz[k.cin[1]] += dx1;
-        }
+        for (int t = 0; t < 2; ++t) cp_mma_bf16(cx[t], d1[t][kt], w);
+      }
+      const int rr = lane & 15, src = 4 * (rr & 7);
+      const bool hi = rr >= 8, second = lane >= 16;
+      float dx[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const float e0 = __shfl_sync(0xffffffffu, cx[0][q], src), e2 = __shfl_sync(0xffffffffu, cx[0][2 + q], src);
+        const float f0 = __shfl_sync(0xffffffffu, cx[1][q], src), f2 = __shfl_sync(0xffffffffu, cx[1][2 + q], src);
+        dx[q] = second ? (hi ? f2 : f0) : (hi ? e2 : e0);
+      }
+      if (active) {
+        for (int j = 0; j < k.nt; ++j) dz[k.tr[j]] = dzT[j];
+        dz[k.cin[0]] += dx[0];
+        if (k.nin > 1) dz[k.cin[1]] += dx[1];
       }
     }
   }
@@ -742,17 +796,63 @@ __global__ void k_flow_adam(float* __restrict__ P, float* __restrict__ G, float*
   cp_flow_adam_one(i, g, P, Mo, Vo, lr, b1t, b2t);
 }
 
-// k_flow_gsum into a cleared G followed by k_flow_adam, in one pass (a single handle's training
-// loop, where no exchange of G sits between them): the same block-order sum, 0 + sum as the
-// gradient, the same update, so the same parameters bit for bit; G is not touched.
+// k_flow_gsum into a cleared G, k_flow_adam and k_flow_pack in one pass (a single handle's training
+// loop, where no exchange of G sits between them): the same block-order sum, 0 + sum as the gradient,
+// the same update, and the parameter's BF16 value into its places in the packed fragments (the
+// forward and the transposed one), which a full pack has laid out before; G is not touched.  The
+// slots are read sixteen at a time: one after the other, their latencies were the kernel (7.4 us, and
+// 3.9 us for the pack; 7.6 us together).
+__device__ __forceinline__ void cp_flow_pack_one(int i, float v, uint2* __restrict__ pk, float* __restrict__ bias)
+{
+  const int c = i / CP_FLOW_PER, o = i % CP_FLOW_PER;
+  uint16_t* q = reinterpret_cast<uint16_t*>(pk + c * CP_FLOW_P_PER);
+  const __nv_bfloat16 bv = __float2bfloat16_rn(v);
+  const uint16_t h = *reinterpret_cast<const uint16_t*>(&bv);
+  // B fragment (first fragment f0, n-tiles per k-tile nnt) of element (row k, column n): lane
+  // 4 (n % 8) + (k % 8) / 2, word k % 16 / 8, half k % 2
+  const auto put = [&](int f0, int nnt, int k, int n) {
+    const int e = f0 + ((k >> 4) * nnt + (n >> 3)) * 32 + 4 * (n & 7) + ((k & 7) >> 1);
+    q[4 * e + 2 * ((k >> 3) & 1) + (k & 1)] = h;
+  };
+  if (o < CP_FLOW_B1) {
+    const int k = o >> 6, n = o & 63;
+    put(CP_FLOW_P_W1, 8, k, n);
+    if (k < 8) put(CP_FLOW_P_W1T, 1, n, k);
+  } else if (o < CP_FLOW_W2) {
+    bias[c * CP_FLOW_NB + o - CP_FLOW_B1] = v;
+  } else if (o < CP_FLOW_B2) {
+    const int k = (o - CP_FLOW_W2) >> 6, n = (o - CP_FLOW_W2) & 63;
+    put(CP_FLOW_P_W2, 8, k, n);
+    put(CP_FLOW_P_W2T, 8, n, k);
+  } else if (o < CP_FLOW_W3) {
+    bias[c * CP_FLOW_NB + 64 + o - CP_FLOW_B2] = v;
+  } else if (o < CP_FLOW_B3) {
+    const int k = (o - CP_FLOW_W3) >> 3, n = (o - CP_FLOW_W3) & 7;
+    put(CP_FLOW_P_W3, 1, k, n);
+    put(CP_FLOW_P_W3T, 8, n, k);
+  } else {
+    bias[c * CP_FLOW_NB + 128 + o - CP_FLOW_B3] = v;
+  }
+}
+
 __global__ void k_flow_gsum_adam(float* __restrict__ P, const float* __restrict__ part, int nblk, float* __restrict__ Mo,
-                                 float* __restrict__ Vo, float lr, float b1t, float b2t)
+                                 float* __restrict__ Vo, float lr, float b1t, float b2t, uint2* __restrict__ pk,
+                                 float* __restrict__ bias)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= CP_FLOW_NPARAM) return;
   float s = 0.f;
-  for (int b = 0; b < nblk; ++b) s += part[(size_t)b * CP_FLOW_NPARAM + i];
+  int b = 0;
+  for (; b + 16 <= nblk; b += 16) {
+    float x[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) x[q] = part[(size_t)(b + q) * CP_FLOW_NPARAM + i];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) s += x[q];
+  }
+  for (; b < nblk; ++b) s += part[(size_t)b * CP_FLOW_NPARAM + i];
   cp_flow_adam_one(i, 0.f + s, P, Mo, Vo, lr, b1t, b2t);
+  cp_flow_pack_one(i, P[i], pk, bias);
 }
 
 // the batch's moments (summed over ranks) for the backward pass, and its loss <w^2> / <w>^2
@@ -848,8 +948,9 @@ static void train_buffers_done(cp_handle* h)
 static int flow_phase_moments(cp_handle* h, const FlowTrainBufs& t, uint64_t point0, uint64_t count, uint32_t iter,
                               double* moments, double* loss_dev = nullptr)
 {
-  k_flow_fwd_train<<<h->num_sms * 2, CP_THREADS, fwd_smem(), h->stream>>>(h->d_flow_pk, h->d_flow_bias, h->d_edges, h->nb,
-                                                                           h->cfg.seed, iter, 2, point0, count, t.zs, t.vj);
+  k_flow_fwd_train<<<h->num_sms, CP_TRAIN_THREADS, fwd_smem(), h->stream>>>(h->d_flow_pk, h->d_flow_bias, h->d_edges, h->nb,
+                                                                           h->cfg.seed, iter, 2, point0, count, t.zs, t.vj,
+                                                                           h->mail->status + 1);
   CP_LAUNCH_CHECK(h, "k_flow_fwd_train");
   const int gblk = h->num_sms * 4;
   int rc = cp_ensure_slots(h, (size_t)2 * gblk);
@@ -873,8 +974,8 @@ static int flow_phase_gradient(cp_handle* h, const FlowTrainBufs& t, uint64_t co
     k_flow_batch_loss<<<1, 1, 0, h->stream>>>(moments, (double)n_batch, t.sums, loss_dev);
     CP_LAUNCH_CHECK(h, "k_flow_batch_loss");
   }
-  k_flow_bwd<<<h->num_sms * 2, CP_BWD_THREADS, bwd_smem(), h->stream>>>(h->d_flow_pk, h->d_flow_bias, count, (double)n_batch, t.zs,
-                                                          t.vj, t.wg, t.sums, t, (float)h->flow_loss_p);
+  k_flow_bwd<<<h->num_sms, CP_TRAIN_THREADS, bwd_smem(), h->stream>>>(h->d_flow_pk, h->d_flow_bias, count, (double)n_batch, t.zs,
+                                                          t.vj, t.wg, t.sums, t, (float)h->flow_loss_p, h->mail->status + 1);
   CP_LAUNCH_CHECK(h, "k_flow_bwd");
   float* G = h->d_flow + CP_FLOW_NPARAM;
   // at most CP_WG_MAXBLK blocks per coupling and layer; chunks are whole multiples of the staged
@@ -924,18 +1025,17 @@ static int flow_phase_update(cp_handle* h, double lr)
   return CP_OK;
 }
 
-// Phase 3 of a single handle's step: the block-order gradient sum and the Adam step in one kernel
-// (the same parameters as k_flow_gsum + flow_phase_update), BF16 repack.
+// Phase 3 of a single handle's step: the block-order gradient sum, the Adam step and the BF16 repack in
+// one kernel (the same parameters and fragments as k_flow_gsum + flow_phase_update).
 static int flow_phase_update_local(cp_handle* h, const FlowTrainBufs& t, int nblk, double lr)
 {
   float* G = h->d_flow + CP_FLOW_NPARAM;
   const long step = h->flow_t + 1;
-  k_flow_gsum_adam<<<(CP_FLOW_NPARAM + 255) / 256, 256, 0, h->stream>>>(
+  k_flow_gsum_adam<<<(CP_FLOW_NPARAM + 127) / 128, 128, 0, h->stream>>>(
       h->d_flow, t.gpart, nblk, G + CP_FLOW_NPARAM, G + 2 * CP_FLOW_NPARAM, (float)lr, (float)pow(0.9, (double)step),
-      (float)pow(0.999, (double)step));
+      (float)pow(0.999, (double)step), h->d_flow_pk, h->d_flow_bias);
   CP_LAUNCH_CHECK(h, "k_flow_gsum_adam");
-  const int rc = cp_flow_repack(h);
-  if (rc) return rc;
+  h->flow_tc_stale = 1;
   h->flow_t = step;
   return CP_OK;
 }
