@@ -104,6 +104,36 @@ __device__ __forceinline__ float cp_logf(float x) { return __logf(x); }
 CP_HD float cp_logf(float x) { return logf(x); }
 #endif
 CP_HD float cp_expm1f(float x) { return expm1f(x); }
+// Products and sums rounded on their own: the compiler contracts none of these with a neighbour.  It
+// would otherwise choose, by the distance of definition and use in the code around, which product of
+// a b + c d an FMA takes, so that an unrelated change to a kernel moved last bits of the weights (and
+// with them accepted points).  The integrand below names every rounding: cp_mulr / cp_addr where a
+// product or sum is rounded, cp_fmaf where it is not.
+CP_HD float cp_mulr(float a, float b)
+{
+#if defined(__CUDA_ARCH__)
+  return __fmul_rn(a, b);
+#else
+  return a * b;
+#endif
+}
+CP_HD float cp_addr(float a, float b)
+{
+#if defined(__CUDA_ARCH__)
+  return __fadd_rn(a, b);
+#else
+  return a + b;
+#endif
+}
+// ln(x) + c, rounded once after the multiplication by ln 2 (ln x = ln 2 log2 x)
+CP_HD float cp_log_add(float x, float c)
+{
+#if defined(__CUDA_ARCH__)
+  return __fmaf_rn(__log2f(x), 0.693147180559945f, c);
+#else
+  return logf(x) + c;
+#endif
+}
 // exp of the CTEQ5L exponent on the device: the hardware base-2 approximation (__expf), relative
 // error about 2^-22 + |x| 2^-24 for exponents of a few units; the accept kernel a further 3%
 // faster, the largest per-point weight error 7.3e-6 (measured as above)
@@ -149,13 +179,12 @@ CP_HD float cp_cq_poly(const CpCteqPoly& c, int f, float t)
 CP_HD float cp_alphas(const CpHadParams& P, float Q2)
 {
   if (Q2 < P.scale2Min) Q2 = P.scale2Min;
-  float lnQ2 = cp_logf(Q2);
   float b0, lnL2;
   if (Q2 > P.thr2[2] && P.nfmax6) { b0 = 21.f; lnL2 = P.lnL2[3]; }
   else if (Q2 > P.thr2[1]) { b0 = 23.f; lnL2 = P.lnL2[2]; }
   else if (Q2 > P.thr2[0]) { b0 = 25.f; lnL2 = P.lnL2[1]; }
   else { b0 = 27.f; lnL2 = P.lnL2[0]; }
-  return (12.f * CP_PI_F) * cp_rcp(b0 * (lnQ2 - lnL2));
+  return (12.f * CP_PI_F) * cp_rcp(b0 * cp_log_add(Q2, -lnL2));
 }
 
 // Error-free transformations on FP32 (Knuth TwoSum, FMA TwoProd) used to carry the few
@@ -188,6 +217,16 @@ CP_HD CpF2 cp_sub2(CpF2 a, CpF2 b) { return cp_f2(a.x - b.x, a.y - b.y); }
 CP_HD CpF2 cp_mul2(CpF2 a, CpF2 b) { return cp_f2(a.x * b.x, a.y * b.y); }
 CP_HD CpF2 cp_fma2(CpF2 a, CpF2 b, CpF2 c) { return cp_f2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
 #endif
+// a product that an addition which follows is not contracted with: the compiler makes one FMA of a
+// two-lane product whose only use is a sum
+CP_HD CpF2 cp_mulr2(CpF2 a, CpF2 b)
+{
+#if defined(__CUDA_ARCH__)
+  return cp_f2(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y));
+#else
+  return cp_mul2(a, b);
+#endif
+}
 CP_HD int cp_bits(float f)
 {
 #if defined(__CUDA_ARCH__)
@@ -278,7 +317,7 @@ CP_HD CpBeamX cp_beam_x(float lnx, float lnxLo, float e1, float om)
   float omx = cp_fmaf(-x, lnxLo, om);
   if (omx < 1e-10f) { omx = 1e-10f; x = 1.f - 1e-10f; lnx = -1e-10f; lnxLo = 0.f; }
   float y = -lnx;                        // y = -ln x, correction -lnxLo
-  b.lny = cp_logf(y) - cp_div_correction(lnxLo, y);
+  b.lny = cp_log_add(y, -cp_div_correction(lnxLo, y));
   // u = ln(x / 1e-5) = ln x + ln 1e5 as a (hi, lo) pair
   const float LN1E5_HI = 11.512925148f, LN1E5_LO = 3.1696e-07f;
   cp_twosum(lnx, LN1E5_HI, b.uh, b.ul);
@@ -314,12 +353,18 @@ struct CpCteqQ {
 // cp_build_had_params checks both against the coefficient tables.
 CP_HD constexpr bool cp_cteq_uses_x1l(int i) { return i == 1 || i == 2; }
 CP_HD constexpr bool cp_cteq_has_qmin(int i) { return i >= 6; }
+// Parametrisations whose polynomial af8 (4..7) or af7 (7) is zero, so that U = 1, C = 0 and the terms
+// with them drop out of the exponent.  cp_build_had_params checks these too.  The unrolled loops leave
+// the zero terms out (and the factor (1 - Qmin/Q) where it is 1), which changes no bit of the sums: the
+// accept kernel of 2^27 points 7.00 -> 6.59 ms, ten VEGAS passes of 2^24 points 10.07 -> 9.53 ms.
+CP_HD constexpr bool cp_cteq_zero_af8(int i) { return i >= 4; }
+CP_HD constexpr bool cp_cteq_zero_af7(int i) { return i == 7; }
 
-// hq = cp_cteq_has_qmin(i)
-CP_HD CpCteqQ cp_cteq_coef(const CpCteqPoly& c, float lnQ, float Q, float invQ, bool hq)
+// hq = cp_cteq_has_qmin(i); z8: af8 is known to be zero
+CP_HD CpCteqQ cp_cteq_coef(const CpCteqPoly& c, float lnQ, float Q, float invQ, bool hq, bool z8)
 {
   CpCteqQ q;
-  float sb1 = cp_logf(lnQ - c.lnAlpha) - 1.2f;
+  float sb1 = cp_log_add(cp_addr(lnQ, -c.lnAlpha), -1.2f);
   // four pairs in two-lane FMAs (each lane rounded as the scalar FMA), af8 alone
   const CpF2 t = cp_f2s(sb1);
   CpF2 v[4];
@@ -333,8 +378,8 @@ CP_HD CpCteqQ cp_cteq_coef(const CpCteqPoly& c, float lnQ, float Q, float invQ, 
   q.af1 = v[1].x; q.af2 = v[1].y;
   q.p = v[2].x; q.af5 = v[2].y;
   q.af6 = v[3].x; q.af7 = v[3].y;
-  q.af8 = cp_cq_poly(c, CP_CQ_AF8, sb1);
-  q.qfac = hq ? ((Q > c.qlim) ? (1.f - c.qmin * invQ) : 0.f) : 1.f;
+  q.af8 = z8 ? 0.f : cp_cq_poly(c, CP_CQ_AF8, sb1);
+  q.qfac = hq ? ((Q > c.qlim) ? cp_fmaf(-c.qmin, invQ, 1.f) : 0.f) : 1.f;
   return q;
 }
 
@@ -361,31 +406,41 @@ CP_HD CpCteqX cp_cteq_x(const CpCteqPoly& c, const CpBeamX& bA, const CpBeamX& b
 //   exponent = A + B x + C u + af1 (y^p - 1) U + part3 + ut1 ln(1-x) + af2 L,  C = af1 af8,
 // summed with the products' FMA residuals kept in a second float, and exp(hi + lo) =
 // exp(hi) (1 + lo).  Every product, residual and sum runs in two-lane arithmetic, the
-// transcendentals per lane.
-CP_HD CpF2 cp_cteq_answer2(const CpCteqX& cx, const CpCteqQ& a, const CpBeamX& bA, const CpBeamX& bB)
+// transcendentals per lane.  z8, z7: af8, af7 are known to be zero; q1: the factor is known to be 1.
+CP_HD CpF2 cp_cteq_answer2(const CpCteqX& cx, const CpCteqQ& a, const CpBeamX& bA, const CpBeamX& bB, bool z8, bool z7,
+                           bool q1)
 {
   const CpF2 lny = cp_f2(bA.lny, bB.lny), x = cp_f2(bA.x, bB.x), omx = cp_f2(bA.omx, bB.omx);
   const CpF2 uh = cp_f2(bA.uh, bB.uh), ul = cp_f2(bA.ul, bB.ul);
   const CpF2 p = cp_f2s(a.p);
   const CpF2 ah = cp_mul2(p, lny);
   const CpF2 ym1 = cp_expm1_2(ah);
-  const CpF2 U = cp_fma2(cp_f2s(a.af8), uh, cp_f2s(1.f));
   const CpF2 xo = cp_mul2(x, omx);
-  const CpF2 part3 = cp_mul2(xo, cp_fma2(cp_f2s(a.af7), xo, cp_fma2(cp_f2s(a.af6), omx, cp_f2s(a.af5))));
-  const float Ch = a.af1 * a.af8, Cl = cp_fmaf(a.af1, a.af8, -Ch);
-  const CpF2 ch = cp_f2s(Ch);
-  const CpF2 t3 = cp_mul2(ch, uh);
-  const CpF2 t3l = cp_fma2(cp_f2s(Cl), uh, cp_fma2(ch, ul, cp_fma2(ch, uh, cp_f2(-t3.x, -t3.y))));
-  const CpF2 qv = cp_mul2(cp_f2s(a.af1), ym1);
-  const CpF2 t4 = cp_mul2(qv, U), t4l = cp_fma2(qv, U, cp_f2(-t4.x, -t4.y));
+  const CpF2 p56 = cp_fma2(cp_f2s(a.af6), omx, cp_f2s(a.af5));
+  const CpF2 p567 = z7 ? p56 : cp_fma2(cp_f2s(a.af7), xo, p56);   // part3 = xo p567
   const CpF2 Bv = cp_f2s(a.B);
   const CpF2 t2 = cp_mul2(Bv, x), t2l = cp_fma2(Bv, x, cp_f2(-t2.x, -t2.y));
   const CpF2 a2 = cp_f2s(a.af2);
   const CpF2 t7 = cp_mul2(a2, cx.L), t7l = cp_fma2(a2, cx.L, cp_f2(-t7.x, -t7.y));
-  const CpF2 el = cp_add2(cp_add2(t2l, t3l), cp_add2(cp_add2(t4l, cx.t6l), t7l));
-  const CpF2 eh = cp_add2(cp_add2(cp_add2(cp_f2s(a.A), t3), cp_add2(t4, t2)), cp_add2(part3, cp_add2(cx.t6, t7)));
+  const CpF2 s367 = cp_fma2(xo, p567, cp_add2(cx.t6, t7));
+  const CpF2 qv = cp_mulr2(cp_f2s(a.af1), ym1);
+  CpF2 el, eh;
+  if (z8) {   // U = 1, C = 0: the general sums without their zero terms
+    el = cp_add2(t2l, cp_add2(cx.t6l, t7l));
+    eh = cp_add2(cp_add2(cp_f2s(a.A), cp_add2(qv, t2)), s367);
+  } else {
+    const CpF2 U = cp_fma2(cp_f2s(a.af8), uh, cp_f2s(1.f));
+    const float Ch = cp_mulr(a.af1, a.af8), Cl = cp_fmaf(a.af1, a.af8, -Ch);
+    const CpF2 ch = cp_f2s(Ch);
+    const CpF2 t3 = cp_mul2(ch, uh);
+    const CpF2 t3l = cp_fma2(cp_f2s(Cl), uh, cp_fma2(ch, ul, cp_fma2(ch, uh, cp_f2(-t3.x, -t3.y))));
+    const CpF2 t4 = cp_mul2(qv, U), t4l = cp_fma2(qv, U, cp_f2(-t4.x, -t4.y));
+    el = cp_add2(cp_add2(t2l, t3l), cp_add2(cp_add2(t4l, cx.t6l), t7l));
+    eh = cp_add2(cp_add2(cp_add2(cp_f2s(a.A), t3), cp_add2(t4, t2)), s367);
+  }
   const CpF2 ex = cp_f2(cp_exp_cteq(eh.x), cp_exp_cteq(eh.y));
-  return cp_mul2(cp_mul2(x, cp_fma2(ex, el, ex)), cp_f2s(a.qfac));
+  const CpF2 r = cp_mul2(x, cp_fma2(ex, el, ex));
+  return q1 ? r : cp_mul2(r, cp_f2s(a.qfac));
 }
 
 // one coefficient record in 128-bit loads (on the device, from constant or shared memory; a
@@ -434,8 +489,11 @@ CP_HD void cp_cteq_scales(const CpCteqPoly* cteq, const float Q2in[NS], float ln
     const CpCteqX cx = cp_cteq_x(c, A, B, cp_cteq_uses_x1l(i));
 #pragma unroll
     for (int s = 0; s < NS; ++s) {
-      const CpCteqQ a = cp_cteq_coef(c, lnQ[s], Q[s], invQ[s], cp_cteq_has_qmin(i));
-      const CpF2 r = cp_cteq_answer2(cx, a, A, B);
+      // zero terms are left out where i is known at compile time
+      constexpr bool known = UNROLL == 8;
+      const bool z8 = known && cp_cteq_zero_af8(i), z7 = known && cp_cteq_zero_af7(i);
+      const CpCteqQ a = cp_cteq_coef(c, lnQ[s], Q[s], invQ[s], cp_cteq_has_qmin(i), z8);
+      const CpF2 r = cp_cteq_answer2(cx, a, A, B, z8, z7, known && !cp_cteq_has_qmin(i));
       float ra = r.x, rb = r.y;
       // parametrisation 4 is the dbar/ubar ratio; the others are x * answer
       if (i != 4) { ra *= A.x; rb *= B.x; }
@@ -478,46 +536,61 @@ CP_HD void cp_cteq_pair(const CpCteqPoly* cteq, float Q2, float lnxA, float lnxA
 // ------------------------------------------------------------------------------------------
 struct CpBrackets {
   float gg2gg, gg2qqbar, qg2qg, qqbar2gg, qqT, qqU, qqTU, qqST;
+  float qqD;   // qqU + qqTU - qqT
 };
 
 CP_HD void cp_brackets(const CpHadParams& P, float tp, float up, CpBrackets& b)
 {
   const CpF2 rtu = cp_rcp2(cp_f2(tp, up));
-  float rt = rtu.x, ru = rtu.y, tu = tp * ru, ut = up * rt;
+  const float rt = rtu.x, ru = rtu.y, tu = cp_mulr(tp, ru), rt2 = cp_mulr(rt, rt), ru2 = cp_mulr(ru, ru);
+  const float tp1 = cp_addr(tp, 1.f), rt1 = cp_addr(rt, 1.f), up1 = cp_addr(up, 1.f), ru1 = cp_addr(ru, 1.f);
+  const float tu1 = cp_addr(tu, 1.f), ut1 = cp_fmaf(up, rt, 1.f);
   // Sigma2gg2gg::sigmaKin: each 9/4 (a^2 + 2a + 3 + 2/a + 1/a^2) = 9/4 ((a+1)^2 + (1/a+1)^2 + 1)
-  float sTS = (tp + 1.f) * (tp + 1.f) + (rt + 1.f) * (rt + 1.f) + 1.f;
-  float sUS = (up + 1.f) * (up + 1.f) + (ru + 1.f) * (ru + 1.f) + 1.f;
-  float sTU = (tu + 1.f) * (tu + 1.f) + (ut + 1.f) * (ut + 1.f) + 1.f;
-  b.gg2gg = 0.5f * 2.25f * (sTS + sUS + sTU);
-  // Sigma2gg2qqbar::sigmaKin
-  b.gg2qqbar = P.nQuarkNew * ((1.f / 6.f) * (ut + tu) - (3.f / 8.f) * (up * up + tp * tp));
-  // Sigma2qg2qg::sigmaKin
-  b.qg2qg = (up * up + 1.f) * (rt * rt) - (4.f / 9.f) * (up + ru);
+  const float sTS = cp_addr(cp_fmaf(tp1, tp1, cp_mulr(rt1, rt1)), 1.f);
+  const float sUS = cp_addr(cp_fmaf(up1, up1, cp_mulr(ru1, ru1)), 1.f);
+  const float sTU = cp_addr(cp_fmaf(tu1, tu1, cp_mulr(ut1, ut1)), 1.f);
+  b.gg2gg = cp_mulr(0.5f * 2.25f, cp_addr(cp_addr(sTS, sUS), sTU));
+  // Sigma2gg2qqbar::sigmaKin: (1/6) (u/t + t/u) - (3/8) (u^2 + t^2)
+  const float uu = cp_mulr(up, up), uutt = cp_fmaf(tp, tp, uu), utu = cp_fmaf(up, rt, tu);
+  b.gg2qqbar = cp_mulr(P.nQuarkNew, cp_fmaf(1.f / 6.f, utu, cp_mulr(-(3.f / 8.f), uutt)));
+  // Sigma2qg2qg::sigmaKin: (u^2 + 1) / t^2 - (4/9) (u + 1/u)
+  const float uu1 = cp_addr(uu, 1.f);
+  b.qg2qg = cp_fmaf(uu1, rt2, cp_mulr(-(4.f / 9.f), cp_addr(up, ru)));
   // Sigma2qqbar2gg::sigmaKin
-  b.qqbar2gg = 0.5f * ((32.f / 27.f) * (ut + tu) - (8.f / 3.f) * (up * up + tp * tp));
+  b.qqbar2gg = cp_mulr(0.5f, cp_fmaf(32.f / 27.f, utu, cp_mulr(-(8.f / 3.f), uutt)));
   // Sigma2qq2qq::sigmaKin terms
-  b.qqT = (4.f / 9.f) * (1.f + up * up) * (rt * rt);
-  b.qqU = (4.f / 9.f) * (1.f + tp * tp) * (ru * ru);
-  b.qqTU = -(8.f / 27.f) * (rt * ru);
-  b.qqST = -(8.f / 27.f) * (up * up) * rt;
+  const float u4 = cp_mulr(4.f / 9.f, cp_fmaf(tp, tp, 1.f));
+  b.qqT = cp_mulr(cp_mulr(4.f / 9.f, uu1), rt2);
+  b.qqU = cp_mulr(u4, ru2);
+  b.qqTU = cp_mulr(-(8.f / 27.f), cp_mulr(rt, ru));
+  b.qqST = cp_mulr(cp_mulr(-(8.f / 27.f), uu), rt);
+  b.qqD = cp_addr(cp_fmaf(u4, ru2, b.qqTU), -b.qqT);
 }
 
+// SINGLE: the products of the opposite-flavour sum, the sea's among them, and of the q qbar -> g g
+// term are each rounded instead of fused (the nominal sum of the scale-variation ratios has them so).
+template <bool SINGLE = false>
 CP_HD float cp_channel_sum(const float mask[5], const CpBrackets& b, const float A[8], const float Bq[8])
 {
-  // flavour sums over q = +-1..+-5 (s, c, b enter twice: quark = antiquark)
+  // flavour sums over q = +-1..+-5 (s, c, b enter twice: quark = antiquark; 2 x is exact)
   float QA = A[0] + A[1] + A[3] + A[4] + 2.f * (A[5] + A[6] + A[7]);
   float QB = Bq[0] + Bq[1] + Bq[3] + Bq[4] + 2.f * (Bq[5] + Bq[6] + Bq[7]);
-  float Dsame = A[0] * Bq[0] + A[1] * Bq[1] + A[3] * Bq[3] + A[4] * Bq[4] +
-                2.f * (A[5] * Bq[5] + A[6] * Bq[6] + A[7] * Bq[7]);
-  float Dopp = A[0] * Bq[4] + A[4] * Bq[0] + A[1] * Bq[3] + A[3] * Bq[1] +
-               2.f * (A[5] * Bq[5] + A[6] * Bq[6] + A[7] * Bq[7]);
-  float G = A[2] * Bq[2];
-  float sum = G * (mask[0] * b.gg2gg + mask[1] * b.gg2qqbar);
-  sum += mask[2] * b.qg2qg * (QA * Bq[2] + A[2] * QB);
+  const float sea = 2.f * (SINGLE ? cp_addr(cp_addr(cp_mulr(A[5], Bq[5]), cp_mulr(A[6], Bq[6])), cp_mulr(A[7], Bq[7]))
+                                  : cp_fmaf(A[7], Bq[7], cp_fmaf(A[5], Bq[5], cp_mulr(A[6], Bq[6]))));
+  const float Dsame = cp_addr(cp_fmaf(A[4], Bq[4], cp_fmaf(A[3], Bq[3], cp_fmaf(A[0], Bq[0], cp_mulr(A[1], Bq[1])))), sea);
+  const float d4 = SINGLE ? cp_addr(cp_addr(cp_addr(cp_mulr(A[0], Bq[4]), cp_mulr(A[4], Bq[0])), cp_mulr(A[1], Bq[3])),
+                                    cp_mulr(A[3], Bq[1]))
+                          : cp_fmaf(A[3], Bq[1], cp_fmaf(A[1], Bq[3], cp_fmaf(A[0], Bq[4], cp_mulr(A[4], Bq[0]))));
+  const float Dopp = cp_addr(d4, sea);
+  const float G = cp_mulr(A[2], Bq[2]);
+  // the masks are 0 or 1, so their products are exact
+  const float qg = cp_mulr(cp_mulr(mask[2], b.qg2qg), cp_fmaf(QA, Bq[2], cp_mulr(A[2], QB)));
+  float sum = cp_fmaf(G, mask[0] * b.gg2gg + mask[1] * b.gg2qqbar, qg);
   // Sigma2qq2qq::sigmaHat: identical 1/2 (T + U + TU), q qbar T + ST, otherwise T
-  sum += mask[3] * (QA * QB * b.qqT + Dsame * (0.5f * (b.qqU + b.qqTU - b.qqT)) + Dopp * b.qqST);
-  sum += mask[4] * Dopp * b.qqbar2gg;
-  return sum;
+  const float qq = cp_fmaf(Dopp, b.qqST, cp_fmaf(cp_mulr(QA, QB), b.qqT, cp_mulr(Dsame, 0.5f * b.qqD)));
+  sum = cp_fmaf(mask[3], qq, sum);
+  const float m4 = cp_mulr(mask[4], Dopp);
+  return SINGLE ? cp_addr(sum, cp_mulr(m4, b.qqbar2gg)) : cp_fmaf(m4, b.qqbar2gg, sum);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -545,8 +618,8 @@ CP_HD float cp_had_eval(const CpHadParams& P, const CpCteqPoly* cteq, float x0, 
   // ln tau = (1 - x0) ln tauMin as a (hi, lo) pair: both factors carry their rounding
   float omx0, omx0l;
   cp_twosum(1.f, -x0, omx0, omx0l);
-  float lnTau = omx0 * P.lnTauMin;
-  float lnTauL = cp_fmaf(omx0, P.lnTauMin, -lnTau) + omx0 * P.lnTauMinLo + omx0l * P.lnTauMin;
+  float lnTau = cp_mulr(omx0, P.lnTauMin);
+  float lnTauL = cp_fmaf(omx0l, P.lnTauMin, cp_fmaf(omx0, P.lnTauMinLo, cp_fmaf(omx0, P.lnTauMin, -lnTau)));
   float eT = cp_expf(lnTau);
   float tau = cp_fmaf(eT, lnTauL, eT);
   float eI = cp_expf(-lnTau);
@@ -566,10 +639,10 @@ CP_HD float cp_had_eval(const CpHadParams& P, const CpCteqPoly* cteq, float x0, 
   // ln x1 = ln tau (1 - v), ln x2 = ln tau v, each as (hi, lo)
   float omv, omvl;
   cp_twosum(1.f, -x1, omv, omvl);
-  float lnx1 = lnTau * omv;
-  float lnx1L = cp_fmaf(lnTau, omv, -lnx1) + lnTauL * omv + lnTau * omvl;
-  float lnx2 = lnTau * x1;
-  float lnx2L = cp_fmaf(lnTau, x1, -lnx2) + lnTauL * x1;
+  float lnx1 = cp_mulr(lnTau, omv);
+  float lnx1L = cp_fmaf(lnTau, omvl, cp_fmaf(lnTauL, omv, cp_fmaf(lnTau, omv, -lnx1)));
+  float lnx2 = cp_mulr(lnTau, x1);
+  float lnx2L = cp_fmaf(lnTauL, x1, cp_fmaf(lnTau, x1, -lnx2));
   float alphaS = cp_alphas(P, P.kR * pT2);
   if (pdf) {
 #pragma unroll
@@ -594,7 +667,7 @@ CP_HD float cp_had_eval(const CpHadParams& P, const CpCteqPoly* cteq, float x0, 
 // with CTEQ5L at the varied scale over the nominal one; the combined points are the products.
 CP_HD void cp_scale_ratios(const CpHadParams& P, const CpCteqPoly* cteq, const CpPoint& pt, float out[6])
 {
-  const float B0 = cp_channel_sum(P.mask, pt.b, pt.fa, pt.fb);
+  const float B0 = cp_channel_sum<true>(P.mask, pt.b, pt.fa, pt.fb);
   if (!(B0 > 0.f) || !(pt.k.alphaS > 0.f)) {
 #pragma unroll
     for (int j = 0; j < 6; ++j) out[j] = 1.f;

@@ -107,6 +107,9 @@ static inline int cp_build_had_params(const CpHadConfig& c, CpHadParams& P)
     if (q.useX1L != (cp_cteq_uses_x1l(i) ? 1 : 0) || (QMIN[i] > 0.0) != cp_cteq_has_qmin(i) ||
         (!cp_cteq_has_qmin(i) && !(ALPHA[i] < 1.0)))
       return 1;
+    // and leave out the terms of these zero polynomials
+    for (int k = 0; k < 3; ++k)
+      if ((cp_cteq_zero_af8(i) && q.co[k][CP_CQ_AF8] != 0.f) || (cp_cteq_zero_af7(i) && q.co[k][CP_CQ_AF7] != 0.f)) return 1;
   }
   double s = c.sqrtS * c.sqrtS;
   double tauMin = 4.0 * c.pTmin * c.pTmin / s;
