@@ -169,14 +169,13 @@ extern "C" int cp_destroy(cp_handle* h)
     if (h->gen_copied[k]) cudaEventDestroy(h->gen_copied[k]);
   }
   if (h->gen_copy) cudaStreamDestroy(h->gen_copy);
-  void* pinned[] = {h->h_gen_cnt, h->h_gen_red, h->h_unw_red, h->h_iters, h->h_losses, h->mail};
+  void* pinned[] = {h->h_gen_cnt, h->h_gen_red, h->h_iters, h->h_losses, h->mail};
   for (void* b : pinned)
     if (b) cudaFreeHost(b);
   void* bufs[] = {h->d_edges, h->d_slots, h->d_red, h->d_x1, h->d_x2, h->d_sH,
                   h->d_tH, h->d_uH, h->d_as, h->d_q2r, h->d_q2f, h->d_qhist, h->d_wmax, h->d_counter, h->d_cteq, h->d_flow, h->d_flow_pk,
-                  h->d_flow_bias, h->d_flow_buf, h->d_flow_tc, h->d_flow_ticket, h->d_pdfbuf,
-                  h->d_gen_stage, h->d_ftrain, h->d_tails, h->d_bmask,
-                  h->d_rsum, h->d_roff, h->d_ticket, h->d_adj};
+                  h->d_flow_bias, h->d_flow_buf, h->d_flow_tc, h->d_flow_ticket, h->d_staging,
+                  h->d_gen_stage, h->d_ftrain, h->d_ticket, h->d_adj};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete h;

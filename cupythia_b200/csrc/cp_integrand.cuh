@@ -665,6 +665,8 @@ CP_HD float cp_had_eval(const CpHadParams& P, const CpCteqPoly* cteq, float x0, 
 // (1, 2), (1, 1/2), (2, 2), (1/2, 1/2).  The brackets carry no scale, alpha_s^2 carries mu_R and
 // the two PDFs mu_F, so a mu_R ratio is (alpha_s' / alpha_s)^2 and a mu_F ratio the channel sum
 // with CTEQ5L at the varied scale over the nominal one; the combined points are the products.
+// Both scales' CTEQ5L run in one loop over the parametrisations: the beams' x terms, the coefficient
+// loads and ln(1 - x + e^ut2) once instead of twice.
 CP_HD void cp_scale_ratios(const CpHadParams& P, const CpCteqPoly* cteq, const CpPoint& pt, float out[6])
 {
   const float B0 = cp_channel_sum<true>(P.mask, pt.b, pt.fa, pt.fb);
@@ -676,7 +678,7 @@ CP_HD void cp_scale_ratios(const CpHadParams& P, const CpCteqPoly* cteq, const C
   const float f2[2] = {4.f, 0.25f};
   const float Q2[2] = {P.kF * f2[0] * pt.k.pT2, P.kF * f2[1] * pt.k.pT2};
   float rR[2], rF[2], fa[2][8], fb[2][8];
-  cp_cteq_scales<2, 1>(cteq, Q2, pt.k.lnx1, pt.k.lnx1L, pt.k.lnx2, pt.k.lnx2L, fa, fb);
+  cp_cteq_scales<2, 8>(cteq, Q2, pt.k.lnx1, pt.k.lnx1L, pt.k.lnx2, pt.k.lnx2L, fa, fb);
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const float a = cp_alphas(P, P.kR * f2[j] * pt.k.pT2) / pt.k.alphaS;

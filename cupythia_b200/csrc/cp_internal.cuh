@@ -87,6 +87,9 @@ struct CpIterDev {
   double sumw, sumw2, wmax, nbad, n, sigma, err, pad;
 };
 
+// chunks of a production pass: at most 2^32 points, 2^24 a chunk
+#define CP_UNW_MAXCHUNKS 256
+
 // What a call's kernels hand back to the host: in mapped pinned memory, which they write themselves,
 // so a call ends with one stream synchronisation instead of device-to-host copies into pageable
 // memory (each of which waits for the device by itself; 50,021 points of production: 54 -> 38 us).
@@ -96,6 +99,7 @@ struct CpMail {
   double wq[2];                               // threshold quantile, q
   double sums[4];                             // partonic: sum w, sum w^2, max w, unused
   unsigned long long count;                   // accepted events of a production pass
+  double unw[8 * CP_UNW_MAXCHUNKS];           // sums of a production pass's chunks
   double adj[10 + 6 * (CP_MAX_BINS + 1)];     // adjoint record and edge gradients
 };
 
@@ -125,7 +129,7 @@ struct cp_handle {
   // launch shapes (resident blocks per SM on this handle's device; -1 until first use)
   int had_blocks = 0;
   int adj_per_sm_nt[2] = {-1, -1}, flow_per_sm = -1;   // adjoint: x tangents only / all six
-  int build_per_sm[2] = {-1, -1};   // record builder without / with scale weights
+  int build_per_sm = -1;            // record builder
   // weight histogram of the last iteration and the unweighting threshold (device)
   unsigned long long* d_qhist = nullptr;   // CP_QBINS
   double wmax_host = 0.0;                  // the unweighting threshold d_wmax[0], as last set
@@ -134,14 +138,13 @@ struct cp_handle {
   unsigned* d_ticket = nullptr;            // last-block ticket of the iteration's finish (0 between launches)
   // production staging for pdfbuf_cap points (K1 -> K2): PDFs and record tails per point, accept
   // masks per 32-point block, totals and output offsets per 1024-point range; per-chunk sums
+  void* d_staging = nullptr;               // one allocation for the arrays below
   float4* d_pdfbuf = nullptr;
   uint4* d_tails = nullptr;
   unsigned* d_bmask = nullptr;
   unsigned* d_rsum = nullptr;
   unsigned long long* d_roff = nullptr;
   uint64_t pdfbuf_cap = 0;
-  double* h_unw_red = nullptr;             // mapped pinned memory
-  uint64_t unw_red_cap = 0;
   float* scalew = nullptr;                 // caller's scale-variation weights (6 per record), or null
   uint64_t scalew_cap = 0;
   // cp_generate_host pipeline, kept between calls: CP_GEN_BUFS record staging buffers of gen_cap

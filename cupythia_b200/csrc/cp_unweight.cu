@@ -13,8 +13,8 @@
 // range per warp, spreads its accepted points over the lanes (every lane busy), takes each one's
 // point index from its block's mask, recomputes the points' kinematics and brackets from the
 // staged coordinates (the PDFs come from K1 too), picks process, flavours and colour
-// flow, and writes the 64-byte records as four 16-byte stores (and, on request, the 7-point
-// scale-variation ratios).  Keeping the record builder out of K1 keeps K1's code small and its
+// flow, and writes the 64-byte records as four 16-byte stores; on request K3 adds the 7-point
+// scale-variation ratios.  Keeping the record builder out of K1 keeps K1's code small and its
 // lanes converged.  Staging grows with the points of a pass, so passes run in chunks of at most
 // CP_UNW_CHUNK points.
 //
@@ -26,6 +26,7 @@
 #include "cp_unweight.cuh"
 
 static_assert(sizeof(CpEventRec) == 64, "event record must be 64 bytes");
+static_assert(CP_UNW_CHUNK * CP_UNW_MAXCHUNKS == 1ull << 32, "chunks of the largest production call");
 static_assert(sizeof(CpEventRec) == sizeof(cp_event), "C ABI record layout");
 
 struct CpMapped {
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(CP_UNW_THREADS, CP_UNW_RESIDENT)
 // accept blocks' sums (fixed order: thread t takes column t % 8 of slots t / 8, t / 8 + 128, ...,
 // then the xor tree of a warp, then the warps in order), block 1 turns the range totals into output
 // offsets: roff[r] = *base_io (0 for `first`) + the records of the ranges before r; then
-// *base_io = the records so far, also handed to the host (as the sums are, through `red`).  Sixteen ranges a thread, so the 16,384 ranges of a full chunk are
+// base_io[0] = the records so far, base_io[1] = those before the chunk; the former also handed to the host (as the sums are, through `red`).  Sixteen ranges a thread, so the 16,384 ranges of a full chunk are
 // one tile: one scan over the block (warp shuffles, a warp over the warps' sums) instead of sixteen
 // (18 us of every chunk, 13 of them saved).  The totals are cleared as they are read, for the next chunk.
 #define CP_SCAN_PER 16
@@ -210,7 +211,10 @@ __global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ 
     carry += wsum[31];
     __syncthreads();   // wsum is rewritten by the next tile
   }
-  if (t == 0) *host_count = *base_io = carry;   // every thread has read it: the loop's barriers (nrange >= 1)
+  if (t == 0) {   // every thread has read *base_io: the loop's barriers (nrange >= 1)
+    base_io[1] = first ? 0ull : *base_io;
+    *host_count = *base_io = carry;
+  }
 }
 
 // K2: work units of a quarter range (8 blocks, 256 points: 65,536 per 2^24-point chunk, so the
@@ -220,10 +224,9 @@ __global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ 
 // kinematics from the staged coordinates (the PDFs come from K1's staging too), picks process,
 // flavours and colour flow, builds the lab-frame kinematics and stores the full 64-byte record
 // at its output index.
-// 4 resident blocks per SM without scale weights (64 registers), 2 with them
-template <bool SCALEW>
-__global__ void __launch_bounds__(CP_THREADS, SCALEW ? 2 : 4) k_unw_build(const __grid_constant__ CpHadParams P,
-                                                                          const __grid_constant__ UnwLaunch L)
+// 4 resident blocks per SM (64 registers)
+__global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_constant__ CpHadParams P,
+                                                             const __grid_constant__ UnwLaunch L)
 {
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = (uint64_t)gridDim.x * (CP_THREADS / 32);
@@ -279,19 +282,45 @@ __global__ void __launch_bounds__(CP_THREADS, SCALEW ? 2 : 4) k_unw_build(const 
       CpEventRec ev;
       cp_make_event(P, pt, cp_u24(w2[0]), cp_u24(w2[1]), cp_u24(w2[2]), cp_u24(w2[3]), cp_colour_rc(w2),
                     cp_colour_rs(w2), __uint_as_float(tail.x), (uint32_t)point, ev);
-      if (SCALEW) {
-        float r[6];
-        cp_scale_ratios(P, P.cteq, pt, r);
-        float2* sw = reinterpret_cast<float2*>(L.scalew + 6 * k);
-        sw[0] = make_float2(r[0], r[1]);
-        sw[1] = make_float2(r[2], r[3]);
-        sw[2] = make_float2(r[4], r[5]);
-      }
       const uint4* src = reinterpret_cast<const uint4*>(&ev);
       uint4* dst = reinterpret_cast<uint4*>(L.out + k);
 #pragma unroll
       for (int f = 0; f < 4; ++f) dst[f] = src[f];
     }
+  }
+}
+
+// K3, on request: the scale-variation ratios of the chunk's records, one record a lane in output
+// order, so every lane works (the record builder's lanes follow the accepted points of a quarter
+// range, 3 of 4 busy in the plain form) and the builder keeps its 64 registers.  A record's point gives
+// its staging slot through its block's accept mask; the kinematics and brackets come from the staged
+// coordinates and PDFs, as the record's did, and CTEQ5L runs at both varied scales together.  With the
+// ratios inside the builder (128 registers, a rolled CTEQ5L loop) the two took
+// 252 us per 1.15e6 records of a 6e6-point pass, now 169.
+__global__ void __launch_bounds__(CP_UNW_THREADS, CP_UNW_RESIDENT)
+    k_unw_scales(const __grid_constant__ CpHadParams P, const __grid_constant__ UnwLaunch L,
+                 const unsigned long long* __restrict__ range)   // records [range[1], range[0])
+{
+  const uint64_t end = range[0] < L.capacity ? range[0] : L.capacity;
+  const uint64_t stride = (uint64_t)gridDim.x * CP_UNW_THREADS;
+  for (uint64_t k = range[1] + (uint64_t)blockIdx.x * CP_UNW_THREADS + threadIdx.x; k < end; k += stride) {
+    const uint32_t p = L.out[k].point - (uint32_t)L.point0;   // in the chunk, of at most 2^24 points
+    const uint64_t q = (p & ~31u) + (uint64_t)__popc(L.bmask[p >> 5] & ((1u << (p & 31u)) - 1u));
+    const uint4 tail = L.tails[q];
+    float pdf[16];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+      const float4 v = L.pdf[4 * q + f];
+      pdf[4 * f] = v.x; pdf[4 * f + 1] = v.y; pdf[4 * f + 2] = v.z; pdf[4 * f + 3] = v.w;
+    }
+    CpPoint pt;
+    cp_had_eval(P, P.cteq, __uint_as_float(tail.y), __uint_as_float(tail.z), __uint_as_float(tail.w), pt, pdf);
+    float r[6];
+    cp_scale_ratios(P, P.cteq, pt, r);
+    float2* sw = reinterpret_cast<float2*>(L.scalew + 6 * k);
+    sw[0] = make_float2(r[0], r[1]);
+    sw[1] = make_float2(r[2], r[3]);
+    sw[2] = make_float2(r[4], r[5]);
   }
 }
 
@@ -313,16 +342,14 @@ static unsigned accept_rounds(const cp_handle* h, uint64_t n)
 
 // The record builder loops grid-stride over the records: its grid is exactly the blocks that
 // are resident at once, so no second wave runs after the first.
-static int build_blocks(cp_handle* h, bool scalew)
+static int build_blocks(cp_handle* h)
 {
-  int& c = h->build_per_sm[scalew ? 1 : 0];
-  if (c < 0) {
+  if (h->build_per_sm < 0) {
     int per_sm = 1;
-    const cudaError_t e = scalew ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_unw_build<true>, CP_THREADS, 0)
-                                 : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_unw_build<false>, CP_THREADS, 0);
-    c = (e != cudaSuccess || per_sm < 1) ? 1 : per_sm;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_unw_build, CP_THREADS, 0);
+    h->build_per_sm = (e != cudaSuccess || per_sm < 1) ? 1 : per_sm;
   }
-  return h->num_sms * c;
+  return h->num_sms * h->build_per_sm;
 }
 
 // Staging of a production chunk of n points: record tails and PDFs per point, accept masks per
@@ -331,19 +358,24 @@ static int unw_staging(cp_handle* h, uint64_t n)
 {
   if (n <= h->pdfbuf_cap) return CP_OK;
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
-  void* old[] = {h->d_pdfbuf, h->d_tails, h->d_bmask, h->d_roff, h->d_rsum};
-  for (void* b : old)
-    if (b) CP_CUDA(h, cudaFree(b));
-  h->d_pdfbuf = nullptr; h->d_tails = nullptr; h->d_bmask = nullptr; h->d_roff = nullptr; h->d_rsum = nullptr;
+  if (h->d_staging) CP_CUDA(h, cudaFree(h->d_staging));
+  h->d_staging = nullptr;
   h->pdfbuf_cap = 0;
   const uint64_t nblk = (n + 31) / 32, nrange = (nblk + CP_UNW_RANGE - 1) / CP_UNW_RANGE;
-  CP_CUDA(h, cudaMalloc(&h->d_pdfbuf, sizeof(float4) * 4 * n));
-  CP_CUDA(h, cudaMalloc(&h->d_tails, sizeof(uint4) * n));
-  CP_CUDA(h, cudaMalloc(&h->d_bmask, sizeof(unsigned) * nblk));
   const uint64_t nscan = (nrange + CP_SCAN_PER - 1) / CP_SCAN_PER * CP_SCAN_PER;   // whole threads of k_unw_finish
-  CP_CUDA(h, cudaMalloc(&h->d_roff, sizeof(unsigned long long) * nscan));
-  CP_CUDA(h, cudaMalloc(&h->d_rsum, sizeof(unsigned) * nscan));
-  CP_CUDA(h, cudaMemsetAsync(h->d_rsum, 0, sizeof(unsigned) * nscan, h->stream));   // k_unw_finish leaves it zero
+  // one allocation, each array at a multiple of 256 bytes
+  const size_t bytes[5] = {sizeof(float4) * 4 * n, sizeof(uint4) * n, sizeof(unsigned) * nblk,
+                           sizeof(unsigned long long) * nscan, sizeof(unsigned) * nscan};
+  size_t at[6] = {0};
+  for (int k = 0; k < 5; ++k) at[k + 1] = at[k] + ((bytes[k] + 255) & ~(size_t)255);
+  CP_CUDA(h, cudaMalloc(&h->d_staging, at[5]));
+  uint8_t* q = static_cast<uint8_t*>(h->d_staging);
+  h->d_pdfbuf = reinterpret_cast<float4*>(q + at[0]);
+  h->d_tails = reinterpret_cast<uint4*>(q + at[1]);
+  h->d_bmask = reinterpret_cast<unsigned*>(q + at[2]);
+  h->d_roff = reinterpret_cast<unsigned long long*>(q + at[3]);
+  h->d_rsum = reinterpret_cast<unsigned*>(q + at[4]);
+  CP_CUDA(h, cudaMemsetAsync(h->d_rsum, 0, bytes[4], h->stream));   // k_unw_finish leaves it zero
   h->pdfbuf_cap = n;
   return CP_OK;
 }
@@ -455,9 +487,15 @@ static int unweight_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t 
     return cp_fail_cuda(h, fe, "k_unw_finish");
   }
   if (capacity) {
-    if (L.scalew) k_unw_build<true><<<build_blocks(h, true), CP_THREADS, 0, h->stream>>>(h->P, L);
-    else k_unw_build<false><<<build_blocks(h, false), CP_THREADS, 0, h->stream>>>(h->P, L);
+    k_unw_build<<<build_blocks(h), CP_THREADS, 0, h->stream>>>(h->P, L);
     CP_LAUNCH_CHECK(h, "k_unw_build");
+    if (L.scalew) {
+      // the host does not know the chunk's record count: eight waves of resident blocks, at most as
+      // many blocks as the points could fill
+      const uint64_t want = (n + CP_UNW_THREADS - 1) / CP_UNW_THREADS, most = (uint64_t)h->num_sms * CP_UNW_RESIDENT * 8;
+      k_unw_scales<<<(unsigned)(want < most ? want : most), CP_UNW_THREADS, 0, h->stream>>>(h->P, L, base_dev);
+      CP_LAUNCH_CHECK(h, "k_unw_scales");
+    }
   }
   if (ev) cudaEventRecord(ev[2], h->stream);
   return CP_OK;
@@ -514,14 +552,6 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   // chunks of at most CP_UNW_CHUNK points; the running record count (d_counter) places each
   // chunk's records after the previous chunk's
   const uint64_t nsub = (n_points + CP_UNW_CHUNK - 1) / CP_UNW_CHUNK;
-  if (nsub > h->unw_red_cap) {
-    CP_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (h->h_unw_red) CP_CUDA(h, cudaFreeHost(h->h_unw_red));
-    h->h_unw_red = nullptr;
-    h->unw_red_cap = 0;
-    CP_CUDA(h, cudaHostAlloc(&h->h_unw_red, sizeof(double) * 8 * nsub, cudaHostAllocMapped | cudaHostAllocPortable));
-    h->unw_red_cap = nsub;
-  }
   int rc = timing_reserve(h, nsub);
   if (rc) return rc;
   h->mail->count = 0;   // without records no kernel writes it
@@ -539,7 +569,7 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   }
   for (uint64_t c = 0; c < nsub; ++c) {
     const uint64_t p0 = c * CP_UNW_CHUNK, n = p0 + CP_UNW_CHUNK <= n_points ? CP_UNW_CHUNK : n_points - p0;
-    rc = unweight_enqueue(h, p0, n, iter, records_dev, capacity, h->h_unw_red + 8 * c, h->scalew, h->d_counter, c == 0, &h->mail->count,
+    rc = unweight_enqueue(h, p0, n, iter, records_dev, capacity, h->mail->unw + 8 * c, h->scalew, h->d_counter, c == 0, &h->mail->count,
                           (h->flow_on && !fused) ? h->d_flow_buf + p0 : nullptr,
                           (h->flow_on && !fused && cp_flow_writes_u(h)) ? h->d_flow_u + p0 : nullptr, (int)c);
     if (rc) return rc;
@@ -549,7 +579,7 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   timing_collect(h, nsub, h->flow_on && !fused, capacity > 0);
   if (h->flow_on && (rc = cp_flow_tc_status(h)) != CP_OK) return rc;
   double red[8];
-  combine_chunks(h->h_unw_red, nsub, red);
+  combine_chunks(h->mail->unw, nsub, red);
   if (out) fill_unw(red, (double)n_points, wm0, out);
   if (cnt > capacity) return cp_fail(h, CP_ERR_CAPACITY, "cp_unweight: record buffer too small (n_accepted reported)");
   if (red[3] > 0) return cp_fail(h, CP_ERR_NUMERIC, "non-finite or negative weights were zeroed");
