@@ -385,6 +385,29 @@ __device__ __forceinline__ void cp_warp_hist_add(float* const (&h)[ND], int ld, 
     }
 }
 
+// Chained launches (programmatic dependent launch): the next kernel's blocks may take their places
+// while this kernel's still run, and wait there until every earlier kernel of the stream has completed
+// with its writes visible.  A chained kernel calls cp_wait_previous before it reads or writes anything
+// that an earlier kernel writes or reads; without the launch attribute both are no-ops.
+__device__ __forceinline__ void cp_next_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... K, class... A>
+static cudaError_t cp_launch_chained(void (*kernel)(K...), unsigned blocks, unsigned threads, cudaStream_t stream,
+                                     const A&... args)
+{
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+
 // out[k] = sum over blocks of slots[b][k], or their max for k == max_col; fixed order, FP64.
 // One warp per output element.
 __device__ __forceinline__ void cp_reduce_column(const double* __restrict__ slots, int nblocks, int width, double* out,

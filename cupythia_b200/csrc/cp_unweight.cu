@@ -91,6 +91,8 @@ __global__ void __launch_bounds__(CP_UNW_THREADS, CP_UNW_RESIDENT)
   __shared__ float2 sEdge[3][CP_MAX_BINS];
   __shared__ double sRed[CP_UNW_THREADS / 32][7];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  cp_next_may_launch();
+  cp_wait_previous();
   if (!L.flow) cp_stage_edges(sEdge, L.edges, L.nb);
   __syncthreads();
   const float wmax = (float)L.wmax[0];
@@ -145,6 +147,8 @@ __global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ 
   __shared__ double sRed[32][CP_UNW_SLOT];
   __shared__ unsigned long long wsum[32];
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  cp_next_may_launch();
+  cp_wait_previous();
   if (blockIdx.x == 0) {
     const int c = t & 7;
     double a = 0.0;
@@ -217,9 +221,9 @@ __global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ 
   }
 }
 
-// K2: work units of a quarter range (8 blocks, 256 points: 65,536 per 2^24-point chunk, so the
-// warps' shares differ by about 1%).  A warp loads its range's 32 block masks, scans their
-// popcounts with shuffles and spreads the accepted points of its quarter over the lanes in point
+// K2: work units of 2^-L.unit_log2 of a range: a quarter (8 blocks, 256 points: 65,536 per 2^24-point
+// chunk, so the warps' shares differ by about 1%), smaller ones for chunks that leave warps idle.  A warp loads its range's 32 block masks, scans their
+// popcounts with shuffles and spreads the accepted points of its unit over the lanes in point
 // order; each lane takes its point index from its block's mask, re-evaluates the point's
 // kinematics from the staged coordinates (the PDFs come from K1's staging too), picks process,
 // flavours and colour flow, builds the lab-frame kinematics and stores the full 64-byte record
@@ -230,9 +234,12 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_consta
 {
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = (uint64_t)gridDim.x * (CP_THREADS / 32);
-  for (uint64_t U = ((uint64_t)blockIdx.x * CP_THREADS + threadIdx.x) >> 5; U < 4 * L.nrange; U += nwarps) {
-    const uint64_t R = U >> 2;
-    const int quarter = (int)(U & 3);
+  const int ul = L.unit_log2, span = CP_UNW_RANGE >> ul;   // span: blocks per unit
+  cp_next_may_launch();
+  cp_wait_previous();
+  for (uint64_t U = ((uint64_t)blockIdx.x * CP_THREADS + threadIdx.x) >> 5; U < (L.nrange << ul); U += nwarps) {
+    const uint64_t R = U >> ul;
+    const int unit = (int)U & ((1 << ul) - 1);
     const uint64_t blk = R * CP_UNW_RANGE + lane;
     const unsigned mk = blk < L.nblk ? L.bmask[blk] : 0u;
     const unsigned c = __popc(mk);
@@ -243,9 +250,9 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_consta
       if (lane >= o) incl += v;
     }
     const unsigned excl = incl - c;
-    // this quarter's entries of the range: [first, total)
-    const unsigned first = __shfl_sync(0xffffffffu, excl, 8 * quarter);
-    const unsigned total = __shfl_sync(0xffffffffu, incl, 8 * quarter + 7);
+    // this unit's entries of the range: [first, total)
+    const unsigned first = __shfl_sync(0xffffffffu, excl, span * unit);
+    const unsigned total = __shfl_sync(0xffffffffu, incl, span * unit + span - 1);
     const unsigned long long base = L.roff[R];
     for (unsigned j0 = first; j0 < total; j0 += 32) {
       const unsigned j = j0 + lane;
@@ -301,6 +308,8 @@ __global__ void __launch_bounds__(CP_UNW_THREADS, CP_UNW_RESIDENT)
     k_unw_scales(const __grid_constant__ CpHadParams P, const __grid_constant__ UnwLaunch L,
                  const unsigned long long* __restrict__ range)   // records [range[1], range[0])
 {
+  cp_next_may_launch();
+  cp_wait_previous();
   const uint64_t end = range[0] < L.capacity ? range[0] : L.capacity;
   const uint64_t stride = (uint64_t)gridDim.x * CP_UNW_THREADS;
   for (uint64_t k = range[1] + (uint64_t)blockIdx.x * CP_UNW_THREADS + threadIdx.x; k < end; k += stride) {
@@ -340,8 +349,11 @@ static unsigned accept_rounds(const cp_handle* h, uint64_t n)
   return r < 1 ? 1u : (r > CP_UNW_MAXROUNDS ? (unsigned)CP_UNW_MAXROUNDS : (unsigned)r);
 }
 
-// The record builder loops grid-stride over the records: its grid is exactly the blocks that
-// are resident at once, so no second wave runs after the first.
+// The record builder loops grid-stride over its units: its grid is the blocks that are resident at
+// once, so no second wave runs after the first, and no more than there are units.  A range is four
+// units, or as many more (up to its 32 blocks) as still leave a unit for every resident warp: with a
+// quarter a unit a chunk of 50,021 points kept 196 of 4,736 warps busy, each for two rounds of
+// records (11.5 us for its 9,500 records, the chained launches aside).
 static int build_blocks(cp_handle* h)
 {
   if (h->build_per_sm < 0) {
@@ -350,6 +362,14 @@ static int build_blocks(cp_handle* h)
     h->build_per_sm = (e != cudaSuccess || per_sm < 1) ? 1 : per_sm;
   }
   return h->num_sms * h->build_per_sm;
+}
+static unsigned build_grid(cp_handle* h, UnwLaunch& L)
+{
+  const uint64_t resident = (uint64_t)build_blocks(h) * (CP_THREADS / 32);
+  L.unit_log2 = 2;
+  while ((1 << L.unit_log2) < CP_UNW_RANGE && (L.nrange << (L.unit_log2 + 1)) <= resident) ++L.unit_log2;
+  const uint64_t blocks = ((L.nrange << L.unit_log2) + CP_THREADS / 32 - 1) / (CP_THREADS / 32);
+  return (unsigned)(blocks < (uint64_t)build_blocks(h) ? blocks : (uint64_t)build_blocks(h));
 }
 
 // Staging of a production chunk of n points: record tails and PDFs per point, accept masks per
@@ -472,29 +492,26 @@ static int unweight_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t 
     rc = cp_flow_tc_accept_enqueue(h, L, &red_blocks);
     if (rc) return rc;
   } else {
-    if (L.flow_u) k_unw_accept<true><<<blocks, CP_UNW_THREADS, 0, h->stream>>>(h->P, L);
-    else k_unw_accept<false><<<blocks, CP_UNW_THREADS, 0, h->stream>>>(h->P, L);
-    CP_LAUNCH_CHECK(h, "k_unw_accept");
+    if (L.flow_u) CP_CUDA(h, cp_launch_chained(k_unw_accept<true>, blocks, CP_UNW_THREADS, h->stream, h->P, L));
+    else CP_CUDA(h, cp_launch_chained(k_unw_accept<false>, blocks, CP_UNW_THREADS, h->stream, h->P, L));
   }
   if (ev) cudaEventRecord(ev[1], h->stream);
   // without records there are no offsets to form: the sums' block alone
-  k_unw_finish<<<capacity ? 2 : 1, 1024, 0, h->stream>>>(h->d_slots, red_blocks, red_dst,
-                                                         reinterpret_cast<uint4*>(L.rsum), L.nrange, first, base_dev,
-                                                         h->d_roff, host_count);
-  const cudaError_t fe = cudaGetLastError();
+  const cudaError_t fe = cp_launch_chained(k_unw_finish, capacity ? 2 : 1, 1024, h->stream, h->d_slots, red_blocks, red_dst,
+                                           reinterpret_cast<uint4*>(L.rsum), L.nrange, first, base_dev, h->d_roff,
+                                           host_count);
   if (fe != cudaSuccess) {
     h->pdfbuf_cap = 0;   // the range totals were not cleared: the next pass allocates them anew
     return cp_fail_cuda(h, fe, "k_unw_finish");
   }
   if (capacity) {
-    k_unw_build<<<build_blocks(h), CP_THREADS, 0, h->stream>>>(h->P, L);
-    CP_LAUNCH_CHECK(h, "k_unw_build");
+    CP_CUDA(h, cp_launch_chained(k_unw_build, build_grid(h, L), CP_THREADS, h->stream, h->P, L));
     if (L.scalew) {
       // the host does not know the chunk's record count: eight waves of resident blocks, at most as
       // many blocks as the points could fill
       const uint64_t want = (n + CP_UNW_THREADS - 1) / CP_UNW_THREADS, most = (uint64_t)h->num_sms * CP_UNW_RESIDENT * 8;
-      k_unw_scales<<<(unsigned)(want < most ? want : most), CP_UNW_THREADS, 0, h->stream>>>(h->P, L, base_dev);
-      CP_LAUNCH_CHECK(h, "k_unw_scales");
+      CP_CUDA(h, cp_launch_chained(k_unw_scales, (unsigned)(want < most ? want : most), CP_UNW_THREADS, h->stream, h->P, L,
+                                   base_dev));
     }
   }
   if (ev) cudaEventRecord(ev[2], h->stream);

@@ -35,15 +35,17 @@ __global__ void __launch_bounds__(CP_THREADS, CP_MIN_BLOCKS) k_had_accum(const _
   __shared__ unsigned sQ[CP_QBINS];
   const int nb = L.nb;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  cp_next_may_launch();
+  for (int k = threadIdx.x; k < CP_WARPS * 3 * CP_MAX_BINS; k += CP_THREADS)
+    (&sHist[0][0][0])[k] = 0.f;
+  for (int k = threadIdx.x; k < CP_QBINS; k += CP_THREADS) sQ[k] = 0u;
+  cp_wait_previous();   // the grid, and the slots and histogram that the pass before may still read
   for (int k = threadIdx.x; k < 3 * nb; k += CP_THREADS) {
     int d = k / nb, b = k - d * nb;
     const double* e = L.edges + d * (nb + 1);
     double lo = e[b], hi = e[b + 1];
     sEdge[d][b] = make_float2((float)lo, (float)(hi - lo));
   }
-  for (int k = threadIdx.x; k < CP_WARPS * 3 * CP_MAX_BINS; k += CP_THREADS)
-    (&sHist[0][0][0])[k] = 0.f;
-  for (int k = threadIdx.x; k < CP_QBINS; k += CP_THREADS) sQ[k] = 0u;
   __syncthreads();
 
   const float nbf = (float)nb;
@@ -185,51 +187,58 @@ __global__ void __launch_bounds__(1024) k_quantile(const unsigned long long* __r
 
 // Shared-memory working set of one dimension's refinement.
 struct CpRefineDim {
-  double h[CP_MAX_BINS], sm[CP_MAX_BINS], r[CP_MAX_BINS], cum[CP_MAX_BINS + 1], e[CP_MAX_BINS + 1];
+  double h[CP_MAX_BINS], sm[CP_MAX_BINS], r[CP_MAX_BINS], cum[CP_MAX_BINS + 1], e[CP_MAX_BINS + 1], tot;
 };
 
-// Lepage's refinement of one dimension (FP64) by one warp: smooth (1,1)/(1,1,1)/(1,1), normalise,
+// the two warps of a dimension
+#define CP_REFINE_WARPS 2
+__device__ __forceinline__ void cp_refine_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+
+// Lepage's refinement of one dimension (FP64) by two warps (so 50 bins are one round): smooth (1,1)/(1,1,1)/(1,1), normalise,
 // compress r = ((d - 1) / ln d)^alpha, and rebin to equal shares of sum r.  The bins' divisions,
-// logarithms and powers and the new edges run over the lanes; the two sums over the bins (their
-// terms' order decides the last bits) run on lane 0, in bin order, so the edges are those of a
+// logarithms and powers and the new edges run over the threads; the two sums over the bins (their
+// terms' order decides the last bits) run on one thread, in bin order, so the edges are those of a
 // serial refinement.  The new edge k lies in the first bin j with cum[j + 1] >= k rsum / nb, cum the
 // running sum of r: a binary search, since r >= 0.
 __device__ __forceinline__ void cp_refine_dim(CpRefineDim& S, double* __restrict__ edges, const double* __restrict__ hist,
-                                              int nb, double alpha)
+                                              int nb, double alpha, int bar)
 {
-  const int lane = threadIdx.x & 31;
-  for (int i = lane; i < nb; i += 32) S.h[i] = __ldcg(hist + i);
-  for (int i = lane; i <= nb; i += 32) S.e[i] = edges[i];
-  __syncwarp();
-  for (int i = lane; i < nb; i += 32) {
+  const int t = threadIdx.x % (32 * CP_REFINE_WARPS), n = 32 * CP_REFINE_WARPS;
+  for (int i = t; i < nb; i += n) S.h[i] = __ldcg(hist + i);
+  for (int i = t; i <= nb; i += n) S.e[i] = edges[i];
+  cp_refine_sync(bar);
+  for (int i = t; i < nb; i += n) {
     double s;
     if (i == 0) s = (S.h[0] + S.h[1]) / 2.0;
     else if (i == nb - 1) s = (S.h[nb - 2] + S.h[nb - 1]) / 2.0;
     else s = (S.h[i - 1] + S.h[i] + S.h[i + 1]) / 3.0;
     S.sm[i] = s;
   }
-  __syncwarp();
-  double tot = 0.0;
-  if (lane == 0)
-    for (int i = 0; i < nb; ++i) tot += S.sm[i];
-  tot = __shfl_sync(0xffffffffu, tot, 0);
+  cp_refine_sync(bar);
+  if (t == 0) {
+    double a = 0.0;
+    for (int i = 0; i < nb; ++i) a += S.sm[i];
+    S.tot = a;
+  }
+  cp_refine_sync(bar);
+  const double tot = S.tot;
   if (!(tot > 0.0)) return;
-  for (int i = lane; i < nb; i += 32) {
+  for (int i = t; i < nb; i += n) {
     const double di = S.sm[i] / tot;
     double ri = 0.0;
     if (di >= 1.0) ri = 1.0;
     else if (di > 0.0) ri = pow((di - 1.0) / log(di), alpha);
     S.r[i] = ri;
   }
-  __syncwarp();
-  if (lane == 0) {
+  cp_refine_sync(bar);
+  if (t == 0) {
     double acc = 0.0;
     S.cum[0] = 0.0;
     for (int i = 0; i < nb; ++i) S.cum[i + 1] = acc += S.r[i];
   }
-  __syncwarp();
+  cp_refine_sync(bar);
   const double step = S.cum[nb] / (double)nb;
-  for (int k = 1 + lane; k < nb; k += 32) {
+  for (int k = 1 + t; k < nb; k += n) {
     const double need = step * (double)k;
     int j = 0, hi = nb - 1;
     while (j < hi) {
@@ -243,24 +252,24 @@ __device__ __forceinline__ void cp_refine_dim(CpRefineDim& S, double* __restrict
   }
 }
 
-// Iteration record (one thread) and, if alpha > 0, the grid refinement (warps 0..2, one dimension
-// each) from the reduced sums of a pass.
+// Iteration record (one thread) and, if alpha > 0, the grid refinement (two warps a dimension) from
+// the reduced sums of a pass; blocks of 256 threads.
 __device__ __forceinline__ void cp_pass_record_refine(CpRefineDim (&S)[3], double* edges, const double* red, int nb,
                                                       double n, double alpha, CpIterDev* rec)
 {
-  const int w = threadIdx.x >> 5;
-  if (threadIdx.x == 96 && rec) {
+  const int d = threadIdx.x / (32 * CP_REFINE_WARPS);
+  if (threadIdx.x == 255 && rec) {
     const double sumw = __ldcg(red), sumw2 = __ldcg(red + 1);
     const double mean = sumw / n;
     const double var = (sumw2 / n - mean * mean) / (n - 1.0);
     rec->sumw = sumw; rec->sumw2 = sumw2; rec->wmax = __ldcg(red + 2); rec->nbad = __ldcg(red + 3); rec->n = n;
     rec->sigma = mean; rec->err = sqrt(var > 0.0 ? var : 0.0);
   }
-  if (alpha > 0.0 && w < 3) cp_refine_dim(S[w], edges + w * (nb + 1), red + CP_SLOT_HEAD + w * nb, nb, alpha);
+  if (alpha > 0.0 && d < 3) cp_refine_dim(S[d], edges + d * (nb + 1), red + CP_SLOT_HEAD + d * nb, nb, alpha, 1 + d);
 }
 
 // The record and refinement from sums already reduced (over ranks).
-__global__ void __launch_bounds__(128) k_refine(double* edges, const double* red, int nb, double n, double alpha,
+__global__ void __launch_bounds__(256) k_refine(double* edges, const double* red, int nb, double n, double alpha,
                                                 CpIterDev* rec)
 {
   __shared__ CpRefineDim S[3];
@@ -280,6 +289,8 @@ __global__ void __launch_bounds__(256) k_pass_finish(const double* __restrict__ 
 {
   __shared__ CpRefineDim S[3];
   __shared__ int sLast;
+  cp_next_may_launch();
+  cp_wait_previous();
   cp_reduce_column(slots, nblocks, width, red, 2);
   if (qclear)
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < CP_QBINS; k += gridDim.x * blockDim.x) qclear[k] = 0ull;
@@ -338,9 +349,8 @@ static int had_pass(cp_handle* h, uint64_t point0, uint64_t n, uint32_t iter, ui
   }
   if (clear) CP_CUDA(h, cudaMemsetAsync(h->d_qhist, 0, sizeof(unsigned long long) * CP_QBINS, h->stream));
   h->last_n = n;
-  if (w_out || x_out) k_had_accum<true><<<blocks, CP_THREADS, 0, h->stream>>>(h->P, L);
-  else k_had_accum<false><<<blocks, CP_THREADS, 0, h->stream>>>(h->P, L);
-  CP_LAUNCH_CHECK(h, "k_had_accum");
+  if (w_out || x_out) CP_CUDA(h, cp_launch_chained(k_had_accum<true>, blocks, CP_THREADS, h->stream, h->P, L));
+  else CP_CUDA(h, cp_launch_chained(k_had_accum<false>, blocks, CP_THREADS, h->stream, h->P, L));
   return CP_OK;
 }
 
@@ -364,10 +374,9 @@ static int had_iteration(cp_handle* h, uint64_t n, uint32_t iter, double alpha, 
   int rc = had_pass(h, 0, n, iter, 0, nullptr, nullptr, clear_before);
   if (rc) return rc;
   const int wpb = 8, width = CP_SLOT_HEAD + 3 * h->nb;
-  k_pass_finish<<<(width + wpb - 1) / wpb, wpb * 32, 0, h->stream>>>(h->d_slots, had_blocks_for(h, n), width, h->d_red,
-                                                                     h->d_edges, h->nb, (double)n, alpha, rec,
-                                                                     clear_after ? h->d_qhist : nullptr, h->d_ticket);
-  CP_LAUNCH_CHECK(h, "k_pass_finish");
+  CP_CUDA(h, cp_launch_chained(k_pass_finish, (width + wpb - 1) / wpb, wpb * 32, h->stream, h->d_slots,
+                               had_blocks_for(h, n), width, h->d_red, h->d_edges, h->nb, (double)n, alpha, rec,
+                               clear_after ? h->d_qhist : nullptr, h->d_ticket));
   return CP_OK;
 }
 
@@ -519,7 +528,7 @@ extern "C" int cp_vegas_refine_sums(cp_handle* h, const double* sums_dev, double
   if (rc) return rc;
   CP_CUDA(h, cudaMemcpyAsync(h->d_red, sums_dev, sizeof(double) * (CP_SLOT_HEAD + 3 * h->nb), cudaMemcpyDeviceToDevice,
                              h->stream));
-  k_refine<<<1, 128, 0, h->stream>>>(h->d_edges, h->d_red, h->nb, n_total, alpha, h->h_iters);
+  k_refine<<<1, 256, 0, h->stream>>>(h->d_edges, h->d_red, h->nb, n_total, alpha, h->h_iters);
   CP_LAUNCH_CHECK(h, "k_refine");
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
   const CpIterDev& r = h->h_iters[0];
