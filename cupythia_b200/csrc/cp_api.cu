@@ -142,8 +142,6 @@ extern "C" int cp_create(const cp_config* cfg, cp_handle** out)
             cudaMalloc(&h->d_wmax, sizeof(double) * 2) == cudaSuccess &&
             cudaMalloc(&h->d_counter, sizeof(unsigned long long) * 2) == cudaSuccess &&
             cudaMemset(h->d_wmax, 0, sizeof(double) * 2) == cudaSuccess &&
-            cudaMalloc(&h->d_ticket, sizeof(unsigned)) == cudaSuccess &&
-            cudaMemset(h->d_ticket, 0, sizeof(unsigned)) == cudaSuccess &&
             cudaMalloc(&h->d_cteq, sizeof(CpCteqPoly) * 8) == cudaSuccess &&
             cudaMemcpy(h->d_cteq, h->P.cteq, sizeof(CpCteqPoly) * 8, cudaMemcpyHostToDevice) == cudaSuccess;
   if (h->mail) memset(h->mail, 0, sizeof(CpMail));
@@ -175,7 +173,7 @@ extern "C" int cp_destroy(cp_handle* h)
   void* bufs[] = {h->d_edges, h->d_slots, h->d_red, h->d_x1, h->d_x2, h->d_sH,
                   h->d_tH, h->d_uH, h->d_as, h->d_q2r, h->d_q2f, h->d_qhist, h->d_wmax, h->d_counter, h->d_cteq, h->d_flow, h->d_flow_pk,
                   h->d_flow_bias, h->d_flow_buf, h->d_flow_tc, h->d_flow_ticket, h->d_staging,
-                  h->d_gen_stage, h->d_ftrain, h->d_ticket, h->d_adj};
+                  h->d_gen_stage, h->d_ftrain, h->d_adj};
   for (void* b : bufs)
     if (b) cudaFree(b);
   delete h;

@@ -135,7 +135,6 @@ struct cp_handle {
   double wmax_host = 0.0;                  // the unweighting threshold d_wmax[0], as last set
   double* d_wmax = nullptr;                // [0] threshold used by cp_unweight, [1] quantile q
   unsigned long long* d_counter = nullptr; // accepted-event counter
-  unsigned* d_ticket = nullptr;            // last-block ticket of the iteration's finish (0 between launches)
   // production staging for pdfbuf_cap points (K1 -> K2): PDFs and record tails per point, accept
   // masks per 32-point block, totals and output offsets per 1024-point range; per-chunk sums
   void* d_staging = nullptr;               // one allocation for the arrays below

@@ -10,7 +10,10 @@
 // and its last block refines the grid in FP64, so iterations chain on the stream
 // without host round trips (the reference round-trips through the host every iteration:
 // cuPythia/11_vegas_importance/vegas.cu:107-124).
+#include <cooperative_groups.h>
+
 #include <mutex>
+
 #include "cp_internal.cuh"
 
 struct HadLaunch {
@@ -185,56 +188,66 @@ __global__ void __launch_bounds__(1024) k_quantile(const unsigned long long* __r
   }
 }
 
-// Shared-memory working set of one dimension's refinement.
+// Shared-memory working set of one dimension's refinement: the histogram, the old edges, the
+// smoothed histogram, the bins' shares and their running sum, and the two warps' parts of a sum.
 struct CpRefineDim {
-  double h[CP_MAX_BINS], sm[CP_MAX_BINS], r[CP_MAX_BINS], cum[CP_MAX_BINS + 1], e[CP_MAX_BINS + 1], tot;
+  double h[CP_MAX_BINS], e[CP_MAX_BINS + 1], r[CP_MAX_BINS], cum[CP_MAX_BINS + 1], part[2];
 };
 
 // the two warps of a dimension
 #define CP_REFINE_WARPS 2
 __device__ __forceinline__ void cp_refine_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
-// Lepage's refinement of one dimension (FP64) by two warps (so 50 bins are one round): smooth (1,1)/(1,1,1)/(1,1), normalise,
-// compress r = ((d - 1) / ln d)^alpha, and rebin to equal shares of sum r.  The bins' divisions,
-// logarithms and powers and the new edges run over the threads; the two sums over the bins (their
-// terms' order decides the last bits) run on one thread, in bin order, so the edges are those of a
-// serial refinement.  The new edge k lies in the first bin j with cum[j + 1] >= k rsum / nb, cum the
-// running sum of r: a binary search, since r >= 0.
-__device__ __forceinline__ void cp_refine_dim(CpRefineDim& S, double* __restrict__ edges, const double* __restrict__ hist,
-                                              int nb, double alpha, int bar)
+// Lepage's refinement of one dimension (FP64) by two warps (so 50 bins are one round), from S.h and S.e:
+// smooth (1,1)/(1,1,1)/(1,1), normalise, compress r = ((d - 1) / ln d)^alpha, and rebin to equal shares of
+// sum r.  The new edge k lies in the first bin j with cum[j + 1] >= k rsum / nb, cum the
+// running sum of r: a binary search, since r >= 0.  It is all latency: the two sums over the bins are
+// warp trees (serial on one thread: 2,200 of 6,500 cycles for 50 bins, now 700), and the usual
+// alpha of 3/2 is a product and a square root instead of a power.
+__device__ __forceinline__ void cp_refine_dim(CpRefineDim& S, double* __restrict__ edges, int nb, double alpha, int bar)
 {
-  const int t = threadIdx.x % (32 * CP_REFINE_WARPS), n = 32 * CP_REFINE_WARPS;
-  for (int i = t; i < nb; i += n) S.h[i] = __ldcg(hist + i);
-  for (int i = t; i <= nb; i += n) S.e[i] = edges[i];
-  cp_refine_sync(bar);
+  const int t = threadIdx.x % (32 * CP_REFINE_WARPS), n = 32 * CP_REFINE_WARPS, lane = t & 31, w = t >> 5;
+  double a = 0.0;
   for (int i = t; i < nb; i += n) {
     double s;
     if (i == 0) s = (S.h[0] + S.h[1]) / 2.0;
     else if (i == nb - 1) s = (S.h[nb - 2] + S.h[nb - 1]) / 2.0;
     else s = (S.h[i - 1] + S.h[i] + S.h[i + 1]) / 3.0;
-    S.sm[i] = s;
+    S.r[i] = s;
+    a += s;
   }
+  a = cp_warp_sum_d(a);
+  if (lane == 0) S.part[w] = a;
   cp_refine_sync(bar);
-  if (t == 0) {
-    double a = 0.0;
-    for (int i = 0; i < nb; ++i) a += S.sm[i];
-    S.tot = a;
-  }
-  cp_refine_sync(bar);
-  const double tot = S.tot;
+  const double tot = S.part[0] + S.part[1];
   if (!(tot > 0.0)) return;
-  for (int i = t; i < nb; i += n) {
-    const double di = S.sm[i] / tot;
+  double carry = 0.0;
+  if (t == 0) S.cum[0] = 0.0;
+  for (int i0 = 0; i0 < nb; i0 += n) {
+    const int i = i0 + t;
     double ri = 0.0;
-    if (di >= 1.0) ri = 1.0;
-    else if (di > 0.0) ri = pow((di - 1.0) / log(di), alpha);
-    S.r[i] = ri;
-  }
-  cp_refine_sync(bar);
-  if (t == 0) {
-    double acc = 0.0;
-    S.cum[0] = 0.0;
-    for (int i = 0; i < nb; ++i) S.cum[i + 1] = acc += S.r[i];
+    if (i < nb) {
+      const double di = S.r[i] / tot;
+      if (di >= 1.0) {
+        ri = 1.0;
+      } else if (di > 0.0) {
+        const double x = (di - 1.0) / log(di);
+        ri = alpha == 1.5 ? x * sqrt(x) : pow(x, alpha);
+      }
+      S.r[i] = ri;
+    }
+    double c = ri;   // inclusive sum over the warp's bins
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double y = __shfl_up_sync(0xffffffffu, c, o);
+      if (lane >= o) c += y;
+    }
+    cp_refine_sync(bar);   // the parts read before
+    if (lane == 31) S.part[w] = c;
+    cp_refine_sync(bar);
+    if (w) c += S.part[0];
+    if (i < nb) S.cum[i + 1] = carry + c;
+    carry += S.part[0] + S.part[1];
   }
   cp_refine_sync(bar);
   const double step = S.cum[nb] / (double)nb;
@@ -252,20 +265,25 @@ __device__ __forceinline__ void cp_refine_dim(CpRefineDim& S, double* __restrict
   }
 }
 
-// Iteration record (one thread) and, if alpha > 0, the grid refinement (two warps a dimension) from
-// the reduced sums of a pass; blocks of 256 threads.
-__device__ __forceinline__ void cp_pass_record_refine(CpRefineDim (&S)[3], double* edges, const double* red, int nb,
+// Iteration record (one thread) and, if alpha > 0, the grid refinement (two warps a dimension, from
+// S[d].h and S[d].e) of a pass with the sums head; blocks of at least 256 threads.
+__device__ __forceinline__ void cp_pass_record_refine(CpRefineDim (&S)[3], const double* head, double* edges, int nb,
                                                       double n, double alpha, CpIterDev* rec)
 {
   const int d = threadIdx.x / (32 * CP_REFINE_WARPS);
   if (threadIdx.x == 255 && rec) {
-    const double sumw = __ldcg(red), sumw2 = __ldcg(red + 1);
+    const double sumw = head[0], sumw2 = head[1];
     const double mean = sumw / n;
     const double var = (sumw2 / n - mean * mean) / (n - 1.0);
-    rec->sumw = sumw; rec->sumw2 = sumw2; rec->wmax = __ldcg(red + 2); rec->nbad = __ldcg(red + 3); rec->n = n;
+    rec->sumw = sumw; rec->sumw2 = sumw2; rec->wmax = head[2]; rec->nbad = head[3]; rec->n = n;
     rec->sigma = mean; rec->err = sqrt(var > 0.0 ? var : 0.0);
   }
-  if (alpha > 0.0 && d < 3) cp_refine_dim(S[d], edges + d * (nb + 1), red + CP_SLOT_HEAD + d * nb, nb, alpha, 1 + d);
+  if (alpha > 0.0 && d < 3) cp_refine_dim(S[d], edges + d * (nb + 1), nb, alpha, 1 + d);
+}
+
+__device__ __forceinline__ void cp_refine_load_edges(CpRefineDim (&S)[3], const double* __restrict__ edges, int nb)
+{
+  for (int k = threadIdx.x; k < 3 * (nb + 1); k += blockDim.x) S[k / (nb + 1)].e[k % (nb + 1)] = edges[k];
 }
 
 // The record and refinement from sums already reduced (over ranks).
@@ -273,35 +291,72 @@ __global__ void __launch_bounds__(256) k_refine(double* edges, const double* red
                                                 CpIterDev* rec)
 {
   __shared__ CpRefineDim S[3];
-  cp_pass_record_refine(S, edges, red, nb, n, alpha, rec);
+  cp_refine_load_edges(S, edges, nb);
+  for (int k = threadIdx.x; k < 3 * nb; k += blockDim.x) S[k / nb].h[k % nb] = red[CP_SLOT_HEAD + k];
+  __syncthreads();
+  cp_pass_record_refine(S, red, edges, nb, n, alpha, rec);
 }
 
-// The end of an iteration in one launch: the fixed-order reduction of the block slots (one warp
-// per column, as k_reduce_slots), then, in the block that finishes last (an integer ticket, which
-// it re-arms), the iteration record and the refinement; on the way the weight histogram is cleared
-// for the iteration that follows, if qclear is given.  With the refinement as three serial threads
-// in a launch of its own (54 us) and a clear before each pass, ten iterations of a million points
-// and the threshold's quantile took 1.65 ms, now 0.92 ms; five of 4,099 points 0.60, now 0.18 ms,
-// where the pass kernel's own latency and the host's round trips are what is left.
-__global__ void __launch_bounds__(256) k_pass_finish(const double* __restrict__ slots, int nblocks, int width, double* red,
-                                                     double* edges, int nb, double n, double alpha, CpIterDev* rec,
-                                                     unsigned long long* qclear, unsigned* ticket)
+// The end of an iteration in one launch, by one cluster: the fixed-order reduction of the block slots, the
+// sums of k_reduce_slots bit for bit, with the partial sums stored to the first block's shared memory, then
+// there the iteration record and the refinement; on the way the weight histogram is cleared
+// for the iteration that follows, if qclear is given.  Four warps take four columns: lane 4 o + c
+// of warp w adds column c of the slots b = w + 4 o (mod 32), so a load of the warp covers whole sectors
+// and 296 slots are two batches of loads.  It is latency from end to end, and a pass of a few thousand points waits
+// for it longer than for its own kernel.  With a grid of 20 blocks, a ticket for the last of them, the sums read
+// back through L2 and serial sums in the refinement, five iterations of 4,099 points took 137 us, now 128, and ten
+// of a million 818, now 803.  The block is as small as that because the pass kernels on either side leave room for
+// it, and it for them, so that chained launches take their places early (640 threads: 125 and 816 us).
+#define CP_FINISH_BLOCKS 8
+#define CP_FINISH_THREADS 320
+#define CP_FINISH_LOADS 5
+__global__ void __cluster_dims__(CP_FINISH_BLOCKS, 1, 1) __launch_bounds__(CP_FINISH_THREADS, 4)
+    k_pass_finish(const double* __restrict__ slots, int nblocks, int width, double* red, double* edges, int nb, double n,
+                  double alpha, CpIterDev* rec, unsigned long long* qclear)
 {
   __shared__ CpRefineDim S[3];
-  __shared__ int sLast;
+  __shared__ double sPart[4][CP_SLOT_HEAD + 3 * CP_MAX_BINS], sHead[CP_SLOT_HEAD];
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int rank = (int)cluster.block_rank(), lane = threadIdx.x & 31;
   cp_next_may_launch();
   cp_wait_previous();
-  cp_reduce_column(slots, nblocks, width, red, 2);
+  if (rank == 0) cp_refine_load_edges(S, edges, nb);
+  double* const part0 = cluster.map_shared_rank(&sPart[0][0], 0);
+  const int groups = (width + 3) / 4;
+  for (int v = rank + CP_FINISH_BLOCKS * (threadIdx.x >> 5); v < 4 * groups; v += CP_FINISH_BLOCKS * (CP_FINISH_THREADS / 32)) {
+    const int w = v & 3, k = 4 * (v >> 2) + (lane & 3);
+    double acc = 0.0;
+    if (k < width) {
+      const double* col = slots + k;
+      for (int b0 = w + 4 * (lane >> 2); b0 < nblocks; b0 += 32 * CP_FINISH_LOADS) {
+        double x[CP_FINISH_LOADS];   // in flight at once, added in slot order (a slot past the last adds nothing)
+#pragma unroll
+        for (int i = 0; i < CP_FINISH_LOADS; ++i) x[i] = b0 + 32 * i < nblocks ? col[(size_t)(b0 + 32 * i) * width] : 0.0;
+#pragma unroll
+        for (int i = 0; i < CP_FINISH_LOADS; ++i) acc = k == 2 ? fmax(acc, x[i]) : acc + x[i];
+      }
+    }
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) {
+      const double y = __shfl_xor_sync(0xffffffffu, acc, o);
+      acc = k == 2 ? fmax(acc, y) : acc + y;
+    }
+    if (lane < 4 && k < width) part0[w * (CP_SLOT_HEAD + 3 * CP_MAX_BINS) + k] = acc;
+  }
   if (qclear)
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < CP_QBINS; k += gridDim.x * blockDim.x) qclear[k] = 0ull;
-  __threadfence();
+    for (int k = rank * CP_FINISH_THREADS + threadIdx.x; k < CP_QBINS; k += CP_FINISH_BLOCKS * CP_FINISH_THREADS) qclear[k] = 0ull;
+  cluster.sync();
+  if (rank != 0) return;
+  for (int k = threadIdx.x; k < width; k += CP_FINISH_THREADS) {
+    const double v = k == 2 ? fmax(fmax(sPart[0][k], sPart[2][k]), fmax(sPart[1][k], sPart[3][k]))
+                            : (sPart[0][k] + sPart[2][k]) + (sPart[1][k] + sPart[3][k]);
+    red[k] = v;
+    const int q = k - CP_SLOT_HEAD;
+    if (q < 0) sHead[k] = v;
+    else S[q / nb].h[q % nb] = v;
+  }
   __syncthreads();
-  if (threadIdx.x == 0) sLast = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!sLast) return;
-  __threadfence();
-  cp_pass_record_refine(S, edges, red, nb, n, alpha, rec);
-  if (threadIdx.x == 0) *ticket = 0u;
+  cp_pass_record_refine(S, sHead, edges, nb, n, alpha, rec);
 }
 
 // FP32 integrand at caller-supplied x
@@ -373,10 +428,9 @@ static int had_iteration(cp_handle* h, uint64_t n, uint32_t iter, double alpha, 
 {
   int rc = had_pass(h, 0, n, iter, 0, nullptr, nullptr, clear_before);
   if (rc) return rc;
-  const int wpb = 8, width = CP_SLOT_HEAD + 3 * h->nb;
-  CP_CUDA(h, cp_launch_chained(k_pass_finish, (width + wpb - 1) / wpb, wpb * 32, h->stream, h->d_slots,
-                               had_blocks_for(h, n), width, h->d_red, h->d_edges, h->nb, (double)n, alpha, rec,
-                               clear_after ? h->d_qhist : nullptr, h->d_ticket));
+  CP_CUDA(h, cp_launch_chained(k_pass_finish, CP_FINISH_BLOCKS, CP_FINISH_THREADS, h->stream, h->d_slots, had_blocks_for(h, n),
+                               CP_SLOT_HEAD + 3 * h->nb, h->d_red, h->d_edges, h->nb, (double)n, alpha, rec,
+                               clear_after ? h->d_qhist : nullptr));
   return CP_OK;
 }
 
