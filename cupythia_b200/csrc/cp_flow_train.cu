@@ -89,8 +89,10 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_fwd_train(const uint2
   if (threadIdx.x == 0) {
     cp_mbar_init(bar, 1);
     cp_mbar_init_fence();
-    cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_FWD);
   }
+  cp_wait_previous();
+  cp_next_may_launch();
+  if (threadIdx.x == 0) cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_FWD);
   for (int k = threadIdx.x; k < 3 * nb; k += CP_TRAIN_THREADS) {
     const int d = k / nb, b = k - d * nb;
     sEdge[d][b] = make_float2((float)edges[d * (nb + 1) + b], (float)(edges[d * (nb + 1) + b + 1] - edges[d * (nb + 1) + b]));
@@ -154,6 +156,8 @@ __global__ void __launch_bounds__(128, 4) k_flow_igrad(const CpHadParams P, cons
   __shared__ int sLast;
   cp_stage_cteq(sCteq, cteq_g);
   __syncthreads();
+  cp_wait_previous();
+  cp_next_may_launch();
   typedef CpDual<3> D3;
   CpHadParamsT<D3> Q;
   Q.lnTauMin = cp_dconst<3>(lnTauMin);
@@ -300,6 +304,10 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_bwd(const uint2* __re
   }
   for (int j = threadIdx.x; j < CP_FLOW_NC * CP_FLOW_NB; j += blockDim.x) sBias[j] = bias_g[j];
   __syncthreads();
+  // the weights above are older than the forward pass, which every chained kernel before this one has
+  // waited for; what follows is theirs
+  cp_wait_previous();
+  cp_next_may_launch();
   const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   // the batch's moments and size (all ranks' points when the batch is sharded)
   const double sig = sums[0] / n_batch;
@@ -731,6 +739,8 @@ __global__ void __launch_bounds__(128) k_flow_wgrad_tc(FlowTrainBufs t, uint64_t
   cp_tc_fence_before();
   __syncthreads();
   cp_tc_fence_after();
+  cp_wait_previous();
+  cp_next_may_launch();
   const uint32_t tmem = tmem_slot;
   // chunk is a whole number of stages; rows beyond n of the last one are zero
   const uint64_t sb = (uint64_t)blockIdx.x * (chunk / CP_WGT_STAGE);
@@ -839,6 +849,8 @@ __global__ void k_flow_gsum_adam(float* __restrict__ P, const float* __restrict_
                                  float* __restrict__ Vo, float lr, float b1t, float b2t, uint2* __restrict__ pk,
                                  float* __restrict__ bias)
 {
+  cp_wait_previous();
+  cp_next_may_launch();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= CP_FLOW_NPARAM) return;
   float s = 0.f;
@@ -943,22 +955,25 @@ static void train_buffers_done(cp_handle* h)
   h->ftrain_cap = h->ftrain_zeroed = 0;
 }
 
+// The kernels of a step are chained launches: each starts its blocks, barriers and constants while the one
+// before it drains, and triggers the next only after its own wait, so whatever an earlier kernel than the
+// last has written (the weights, for the backward pass) is complete as well.  100 steps of 65,536 points:
+// 13.55 -> 12.75 ms.
+//
 // Phase 1 of a step: forward and integrand over the batch points [point0, point0 + count) at
 // counter iteration `iter` (Philox stream 2); moments[0..1] = (sum w, sum w^2) over them.
 static int flow_phase_moments(cp_handle* h, const FlowTrainBufs& t, uint64_t point0, uint64_t count, uint32_t iter,
                               double* moments, double* loss_dev = nullptr)
 {
-  k_flow_fwd_train<<<h->num_sms, CP_TRAIN_THREADS, fwd_smem(), h->stream>>>(h->d_flow_pk, h->d_flow_bias, h->d_edges, h->nb,
-                                                                           h->cfg.seed, iter, 2, point0, count, t.zs, t.vj,
-                                                                           h->mail->status + 1);
-  CP_LAUNCH_CHECK(h, "k_flow_fwd_train");
+  CP_CUDA(h, cp_launch_chained_smem(k_flow_fwd_train, h->num_sms, CP_TRAIN_THREADS, fwd_smem(), h->stream, h->d_flow_pk,
+                                    h->d_flow_bias, h->d_edges, h->nb, h->cfg.seed, iter, 2u, point0, count, t.zs, t.vj,
+                                    h->mail->status + 1));
   const int gblk = h->num_sms * 4;
   int rc = cp_ensure_slots(h, (size_t)2 * gblk);
   if (rc) return rc;
   const float lnTauMin = (float)log(4.0 * h->cfg.pt_hat_min * h->cfg.pt_hat_min / (h->cfg.sqrt_s * h->cfg.sqrt_s));
-  k_flow_igrad<<<gblk, 128, 0, h->stream>>>(h->P, h->d_cteq, count, lnTauMin, t.vj, t.wg, h->d_slots,
-                                            h->d_flow_ticket, moments, (double)count, loss_dev);
-  CP_LAUNCH_CHECK(h, "k_flow_igrad");
+  CP_CUDA(h, cp_launch_chained(k_flow_igrad, gblk, 128, h->stream, h->P, h->d_cteq, count, lnTauMin, t.vj, t.wg, h->d_slots,
+                               h->d_flow_ticket, moments, (double)count, loss_dev));
   return CP_OK;
 }
 
@@ -974,9 +989,9 @@ static int flow_phase_gradient(cp_handle* h, const FlowTrainBufs& t, uint64_t co
     k_flow_batch_loss<<<1, 1, 0, h->stream>>>(moments, (double)n_batch, t.sums, loss_dev);
     CP_LAUNCH_CHECK(h, "k_flow_batch_loss");
   }
-  k_flow_bwd<<<h->num_sms, CP_TRAIN_THREADS, bwd_smem(), h->stream>>>(h->d_flow_pk, h->d_flow_bias, count, (double)n_batch, t.zs,
-                                                          t.vj, t.wg, t.sums, t, (float)h->flow_loss_p, h->mail->status + 1);
-  CP_LAUNCH_CHECK(h, "k_flow_bwd");
+  CP_CUDA(h, cp_launch_chained_smem(k_flow_bwd, h->num_sms, CP_TRAIN_THREADS, bwd_smem(), h->stream, h->d_flow_pk, h->d_flow_bias,
+                                    count, (double)n_batch, t.zs, t.vj, t.wg, t.sums, t, (float)h->flow_loss_p,
+                                    h->mail->status + 1));
   float* G = h->d_flow + CP_FLOW_NPARAM;
   // at most CP_WG_MAXBLK blocks per coupling and layer; chunks are whole multiples of the staged
   // rows.  The three launches share the grid, so together they write every entry of the
@@ -985,9 +1000,8 @@ static int flow_phase_gradient(cp_handle* h, const FlowTrainBufs& t, uint64_t co
   const int nblk = (int)((count + chunk - 1) / chunk);
   if (h->flow_kernel == 0) {
     // tensor cores (tcgen05): every coupling and layer shape in one launch
-    k_flow_wgrad_tc<<<dim3((unsigned)nblk, CP_FLOW_NC, 3), 128, 0, h->stream>>>(t, count, (int)chunk,
-                                                                             h->mail->status + 1);
-    CP_LAUNCH_CHECK(h, "k_flow_wgrad_tc");
+    CP_CUDA(h, cp_launch_chained_smem(k_flow_wgrad_tc, dim3((unsigned)nblk, CP_FLOW_NC, 3), 128, 0, h->stream, t, count, (int)chunk,
+                                      h->mail->status + 1));
   } else {
     // warp-level mma.sync, one launch per layer shape (the cross-check path)
     const dim3 grid((unsigned)nblk, CP_FLOW_NC);
@@ -1031,10 +1045,9 @@ static int flow_phase_update_local(cp_handle* h, const FlowTrainBufs& t, int nbl
 {
   float* G = h->d_flow + CP_FLOW_NPARAM;
   const long step = h->flow_t + 1;
-  k_flow_gsum_adam<<<(CP_FLOW_NPARAM + 127) / 128, 128, 0, h->stream>>>(
-      h->d_flow, t.gpart, nblk, G + CP_FLOW_NPARAM, G + 2 * CP_FLOW_NPARAM, (float)lr, (float)pow(0.9, (double)step),
-      (float)pow(0.999, (double)step), h->d_flow_pk, h->d_flow_bias);
-  CP_LAUNCH_CHECK(h, "k_flow_gsum_adam");
+  CP_CUDA(h, cp_launch_chained(k_flow_gsum_adam, (CP_FLOW_NPARAM + 127) / 128, 128, h->stream, h->d_flow, t.gpart, nblk,
+                               G + CP_FLOW_NPARAM, G + 2 * CP_FLOW_NPARAM, (float)lr, (float)pow(0.9, (double)step),
+                               (float)pow(0.999, (double)step), h->d_flow_pk, h->d_flow_bias));
   h->flow_tc_stale = 1;
   h->flow_t = step;
   return CP_OK;

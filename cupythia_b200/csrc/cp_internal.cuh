@@ -392,12 +392,13 @@ __device__ __forceinline__ void cp_next_may_launch() { asm volatile("griddepcont
 __device__ __forceinline__ void cp_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... K, class... A>
-static cudaError_t cp_launch_chained(void (*kernel)(K...), unsigned blocks, unsigned threads, cudaStream_t stream,
-                                     const A&... args)
+static cudaError_t cp_launch_chained_smem(void (*kernel)(K...), dim3 blocks, unsigned threads, size_t smem, cudaStream_t stream,
+                                          const A&... args)
 {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks);
+  cfg.gridDim = blocks;
   cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr = {};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -405,6 +406,12 @@ static cudaError_t cp_launch_chained(void (*kernel)(K...), unsigned blocks, unsi
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+template <class... K, class... A>
+static cudaError_t cp_launch_chained(void (*kernel)(K...), unsigned blocks, unsigned threads, cudaStream_t stream,
+                                     const A&... args)
+{
+  return cp_launch_chained_smem(kernel, dim3(blocks), threads, 0, stream, args...);
 }
 
 // out[k] = sum over blocks of slots[b][k], or their max for k == max_col; fixed order, FP64.
