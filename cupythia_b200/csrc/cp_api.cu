@@ -590,7 +590,7 @@ struct PartonicArgs {
 // are sums without cancellation, and p is the FMA 1 - c c, rounded once, so the form is within a
 // few 1e-16 of the exact value at its c (the bracket form: 1.1e-15 over |cos theta| < 0.9).
 // Twelve FP64 operations a draw with the sums, against 27 and an IEEE division in terms of t and u
-// (1.05e9 SplitMix64 draws: 3.03 ms there, 1.86 ms here); the prefactor
+// (1.05e9 SplitMix64 draws: 3.03 ms there, 1.68 ms here); the prefactor
 // (pi / s^2) alpha_s^2 / 2 (9/2) is the same for every draw and multiplies the sums.
 __device__ __forceinline__ double cp_gg2gg_form(double c)
 {
@@ -623,10 +623,29 @@ struct CpPartonicSums {
     s2 = fma(v, v, s2);
     if (v > wm) wm = v;
   }
+  // The same for several draws.  A draw seldom raises the largest one, so the upper words (order-preserving:
+  // the values are positive) decide whether any can: one compare and a branch for eight draws instead of a
+  // compare and two selects each (1.05e9 draws: 1.78 -> 1.72 ms).
+  template <int N>
+  __device__ __forceinline__ void add(const double (&v)[N])
+  {
+    int top = __double2hiint(v[0]);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      s1 += v[j];
+      s2 = fma(v[j], v[j], s2);
+      top = max(top, __double2hiint(v[j]));
+    }
+    if (top >= __double2hiint(wm)) {
+#pragma unroll
+      for (int j = 0; j < N; ++j)
+        if (v[j] > wm) wm = v[j];
+    }
+  }
 };
 
-// MODE 0: Philox sums over points; 1: SplitMix64 sums over the reference's (thread, draw) pairs;
-// 2: Philox per-point weights.  Sums are of the bare form above; each block scales its slot.
+// MODE 0: Philox sums over points; 1 and 3: SplitMix64 sums over the reference's (thread, draw) pairs, for
+// many and for few threads; 2: Philox per-point weights.  Sums are of the bare form above; each block scales its slot.
 // Bound by instruction issue: about 20 integer operations (SplitMix64) and 12 FP64 a draw.
 template <int MODE>
 __global__ void __launch_bounds__(CP_THREADS, 5) k_partonic(const PartonicArgs a)
@@ -636,33 +655,65 @@ __global__ void __launch_bounds__(CP_THREADS, 5) k_partonic(const PartonicArgs a
   CpPartonicSums S;
   const uint64_t nthr = (uint64_t)gridDim.x * CP_THREADS;
   const uint64_t t = (uint64_t)blockIdx.x * CP_THREADS + threadIdx.x;
-  if (MODE == 1) {
+  if (MODE == 1 || MODE == 3) {
     // the reference's thread i makes draws k = 0 .. kper-1 from counter seed + i 0x100000001B3 + k
-    // (cuPythia/03_fused_resident_me/fused_gg2gg.cu:43-50); the n kper pairs are split into
-    // equal contiguous shares, so every thread here does the same number of draws (the first
-    // total % nthr threads one more).  Within a reference thread the counters are consecutive; a
-    // warp advances by the draws that all of its lanes have left in theirs, so its lanes stay
-    // converged (lanes that loop over their own runs were 59% active at 1000 draws a thread).
-    const uint64_t total = a.n * a.kper, q = total / nthr, rem = total % nthr;
-    const uint64_t w0 = q * t + (t < rem ? t : rem);
-    uint64_t left = q, i = w0 / a.kper, k = w0 - i * a.kper;
-    uint64_t ctr = a.seed + i * 0x100000001B3ULL + k;
+    // (cuPythia/03_fused_resident_me/fused_gg2gg.cu:43-50)
     const auto draw = [&](uint64_t c) {
       const uint64_t v = cp_splitmix64(c);
-      S.add(cp_gg2gg_form(cp_partonic_cos((uint32_t)(v >> 32), (uint32_t)v, a.cMax)));
+      return cp_gg2gg_form(cp_partonic_cos((uint32_t)(v >> 32), (uint32_t)v, a.cMax));
     };
-    while (left) {
-      uint64_t run = a.kper - k;
-      run = run < left ? run : left;
-      const uint32_t m = __reduce_min_sync(0xffffffffu, run < (1u << 30) ? (uint32_t)run : (1u << 30));
-#pragma unroll 4
-      for (uint32_t j = 0; j < m; ++j) draw(ctr + j);
-      left -= m;
-      k += m;
-      ctr += m;
-      if (k == a.kper) { k = 0; ++i; ctr = a.seed + i * 0x100000001B3ULL; }
+    const auto draws = [&](uint64_t ctr, uint32_t m) {
+      uint32_t j = 0;
+      for (; j + 8 <= m; j += 8) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = draw(ctr + j + q);
+        S.add(v);
+      }
+      for (; j < m; ++j) S.add(draw(ctr + j));
+    };
+    if (MODE == 1) {
+      // A warp's lanes take 32 consecutive reference threads at the same k, and the warps equal contiguous
+      // shares of the (group of 32, k) pairs, so the lanes are converged over runs of up to kper draws (shares
+      // of single lanes cross their threads' ends at different draws: 2^20 threads x 1000 draws 1.72 -> 1.68 ms,
+      // x 100 draws 268 -> 206 us).
+      const int lane = threadIdx.x & 31;
+      const uint64_t warps = nthr / 32, wi = t / 32;
+      const uint64_t total = (a.n + 31) / 32 * a.kper, q = total / warps, rem = total % warps;
+      const uint64_t w0 = q * wi + (wi < rem ? wi : rem);
+      uint64_t left = q + (wi < rem ? 1 : 0), g = w0 / a.kper, k = w0 - g * a.kper;
+      while (left) {
+        uint64_t run = a.kper - k;
+        run = run < left ? run : left;
+        const uint32_t m = run < (1u << 30) ? (uint32_t)run : (1u << 30);
+        const uint64_t i = 32 * g + lane;
+        if (i < a.n) draws(a.seed + i * 0x100000001B3ULL + k, m);
+        left -= m;
+        k += m;
+        if (k == a.kper) { k = 0; ++g; }
+      }
+    } else {
+      // Few reference threads: the n kper pairs are split into
+      // equal contiguous shares, so every thread here does the same number of draws (the first
+      // total % nthr threads one more).  Within a reference thread the counters are consecutive; a
+      // warp advances by the draws that all of its lanes have left in theirs, so its lanes stay
+      // converged (lanes that loop over their own runs were 59% active at 1000 draws a thread).
+      const uint64_t total = a.n * a.kper, q = total / nthr, rem = total % nthr;
+      const uint64_t w0 = q * t + (t < rem ? t : rem);
+      uint64_t left = q, i = w0 / a.kper, k = w0 - i * a.kper;
+      uint64_t ctr = a.seed + i * 0x100000001B3ULL + k;
+      while (left) {
+        uint64_t run = a.kper - k;
+        run = run < left ? run : left;
+        const uint32_t m = __reduce_min_sync(0xffffffffu, run < (1u << 30) ? (uint32_t)run : (1u << 30));
+        draws(ctr, m);
+        left -= m;
+        k += m;
+        ctr += m;
+        if (k == a.kper) { k = 0; ++i; ctr = a.seed + i * 0x100000001B3ULL; }
+      }
+      if (t < rem) S.add(draw(ctr));
     }
-    if (t < rem) draw(ctr);
   } else {
     for (uint64_t i = t; i < a.n; i += nthr) {
       uint32_t wd[4];
@@ -688,17 +739,22 @@ __global__ void __launch_bounds__(CP_THREADS, 5) k_partonic(const PartonicArgs a
 static int partonic_run(cp_handle* h, int mode, PartonicArgs a, uint64_t npoints, cp_result* out)
 {
   if (!(a.s > 0) || !(a.cMax > 0) || !(a.cMax < 1)) return cp_fail(h, CP_ERR_INVALID, "partonic: bad kinematics");
-  // one wave of resident blocks: the per-thread shares are equal, so nothing waits on a tail
+  // Equal shares for one wave of resident blocks, or for four waves once that leaves a thread 64 draws: the
+  // warps of a wave finish far apart (at 75% of the issue slots some are served less), and the later blocks fill
+  // what the early ones leave (1.05e9 draws: one wave 1.86 ms, 4 waves 1.78, 40 waves 1.88).
   int per_sm = 0;
   const cudaError_t oe = mode == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_partonic<0>, CP_THREADS, 0)
-                                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_partonic<1>, CP_THREADS, 0);
+                       : mode == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_partonic<1>, CP_THREADS, 0)
+                                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_partonic<3>, CP_THREADS, 0);
   if (oe != cudaSuccess || per_sm < 1) per_sm = 4;
-  const int blocks = h->num_sms * per_sm;
+  const int wave = h->num_sms * per_sm;
+  const int blocks = npoints / ((uint64_t)wave * CP_THREADS) >= 4 * 64 ? 4 * wave : wave;
   int rc = cp_ensure_slots(h, (size_t)blocks * 4);
   if (rc) return rc;
   a.slots = h->d_slots;
   if (mode == 0) k_partonic<0><<<blocks, CP_THREADS, 0, h->stream>>>(a);
-  else k_partonic<1><<<blocks, CP_THREADS, 0, h->stream>>>(a);
+  else if (mode == 1) k_partonic<1><<<blocks, CP_THREADS, 0, h->stream>>>(a);
+  else k_partonic<3><<<blocks, CP_THREADS, 0, h->stream>>>(a);
   CP_LAUNCH_CHECK(h, "k_partonic");
   k_reduce_slots<0><<<1, 4 * 32, 0, h->stream>>>(h->d_slots, blocks, 4, h->mail->sums);
   CP_LAUNCH_CHECK(h, "k_reduce_slots");
@@ -734,7 +790,8 @@ extern "C" int cp_partonic_splitmix(cp_handle* h, double sqrt_shat, double alpha
   if (nthr * kper < 2) return cp_fail(h, CP_ERR_INVALID, "too few draws");
   double s = sqrt_shat * sqrt_shat;
   PartonicArgs a{s, alphas, cmax, (2.0 * cmax) * (s / 2.0) * conv, seed, 0, nthr, kper, nullptr, nullptr};
-  return partonic_run(h, 1, a, nthr * kper, out);
+  // groups of 32 reference threads, the last one possibly short, once that idles at most 3% of the lanes
+  return partonic_run(h, nthr >= 1024 ? 1 : 3, a, nthr * kper, out);
 }
 
 extern "C" int cp_partonic_weights(cp_handle* h, double sqrt_shat, double alphas, double cmax,
