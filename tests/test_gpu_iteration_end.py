@@ -19,3 +19,19 @@ def test_iteration_matches_accumulate_and_refine(nb, n):
             rb = b.refine(b.accumulate(n, k), n, alpha)
             assert ra == rb
             assert np.asarray(a.grid).tobytes() == np.asarray(b.grid).tobytes()
+
+
+@pytest.mark.parametrize("n_iter", [1, 2, 3])
+def test_weight_histogram_is_the_last_pass_s(n_iter):
+    import cupythia_b200 as cp
+
+    n = 70_001
+    with cp.Integrator() as a, cp.Integrator() as b:
+        a.iteration(5000, 9)     # leaves a histogram behind
+        a.grid = b.grid
+        a.integrate(n_iter, n)
+        for k in range(n_iter):
+            b.iteration(n, k)
+        assert np.asarray(a.grid).tobytes() == np.asarray(b.grid).tobytes()
+        h = a.weight_histogram().cpu().numpy()
+        assert (h == b.weight_histogram().cpu().numpy()).all() and 0 < h.sum() <= n
