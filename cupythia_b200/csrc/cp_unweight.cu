@@ -221,28 +221,39 @@ __global__ void __launch_bounds__(1024) k_unw_finish(const double* __restrict__ 
   }
 }
 
-// K2: work units of 2^-L.unit_log2 of a range: a quarter (8 blocks, 256 points: 65,536 per 2^24-point
-// chunk, so the warps' shares differ by about 1%), smaller ones for chunks that leave warps idle.  A warp loads its range's 32 block masks, scans their
-// popcounts with shuffles and spreads the accepted points of its unit over the lanes in point
-// order; each lane takes its point index from its block's mask, re-evaluates the point's
+// K2: every warp takes an equal run of 32-point blocks.  It loads the masks of a window of 32 blocks, scans their
+// popcounts with shuffles and spreads the accepted points over the lanes in point
+// order, whole warps of them at a time (the next window starts at the first one left), so that all lanes
+// work until the run's end; each lane takes its point index from its block's mask, re-evaluates the point's
 // kinematics from the staged coordinates (the PDFs come from K1's staging too), picks process,
 // flavours and colour flow, builds the lab-frame kinematics and stores the full 64-byte record
-// at its output index.
+// at its output index.  Bound by instruction issue (74% of the slots).  Over quarter ranges of 256 points 5 of 6
+// lanes were busy: plain production of 2^27 points
+// 1.34 -> 1.12 ms, flow of 2^26 1.47 -> 1.33.
 // 4 resident blocks per SM (64 registers)
 __global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_constant__ CpHadParams P,
                                                              const __grid_constant__ UnwLaunch L)
 {
   const int lane = threadIdx.x & 31;
   const uint64_t nwarps = (uint64_t)gridDim.x * (CP_THREADS / 32);
-  const int ul = L.unit_log2, span = CP_UNW_RANGE >> ul;   // span: blocks per unit
   cp_next_may_launch();
   cp_wait_previous();
-  for (uint64_t U = ((uint64_t)blockIdx.x * CP_THREADS + threadIdx.x) >> 5; U < (L.nrange << ul); U += nwarps) {
-    const uint64_t R = U >> ul;
-    const int unit = (int)U & ((1 << ul) - 1);
-    const uint64_t blk = R * CP_UNW_RANGE + lane;
-    const unsigned mk = blk < L.nblk ? L.bmask[blk] : 0u;
-    const unsigned c = __popc(mk);
+  // this warp's run of blocks
+  const uint64_t W = ((uint64_t)blockIdx.x * CP_THREADS + threadIdx.x) >> 5;
+  uint64_t B = L.nblk * W / nwarps;
+  const uint64_t Bend = L.nblk * (W + 1) / nwarps;
+  if (B >= Bend) return;
+  // a window of 32 blocks; the output position of its first entry is the range's offset and the
+  // accepted points of the range's blocks before it
+  unsigned mk = B + lane < Bend ? L.bmask[B + lane] : 0u;
+  const int before = (int)(B % CP_UNW_RANGE);
+  const unsigned mp = lane < before ? L.bmask[B - before + lane] : 0u;
+  unsigned long long base = L.roff[B / CP_UNW_RANGE];
+  base += __reduce_add_sync(0xffffffffu, (unsigned)__popc(mp));
+  unsigned skip = 0;   // entries of block B already built
+  for (;;) {
+    // all of the window's entries in the end, before that whole warps of them
+    const unsigned c = __popc(mk) - (lane == 0 ? skip : 0u);
     unsigned incl = c;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -250,11 +261,10 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_consta
       if (lane >= o) incl += v;
     }
     const unsigned excl = incl - c;
-    // this unit's entries of the range: [first, total)
-    const unsigned first = __shfl_sync(0xffffffffu, excl, span * unit);
-    const unsigned total = __shfl_sync(0xffffffffu, incl, span * unit + span - 1);
-    const unsigned long long base = L.roff[R];
-    for (unsigned j0 = first; j0 < total; j0 += 32) {
+    const unsigned all = __shfl_sync(0xffffffffu, incl, 31);
+    const bool last = B + 32 >= Bend;
+    const unsigned total = last || all < 32u ? all : all & ~31u;
+    for (unsigned j0 = 0; j0 < total; j0 += 32) {
       const unsigned j = j0 + lane;
       // this lane's entry lies in the first block whose inclusive count exceeds j
       int b = 0;
@@ -267,12 +277,12 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_consta
       if (j >= total || k >= L.capacity) continue;
       // the entry is the block's accepted point of rank r; its lane is the position of the
       // r-th set bit of the block's mask: the largest x with fewer than r + 1 set bits below x
-      const unsigned r = j - ex;
+      const unsigned r = j - ex + (b == 0 ? skip : 0u);
       int x = 0;
 #pragma unroll
       for (int st = 16; st > 0; st >>= 1)
         if ((unsigned)__popc(mb & ((1u << (x + st)) - 1u)) <= r) x += st;
-      const uint64_t blkq = (R * CP_UNW_RANGE + b) * 32;
+      const uint64_t blkq = (B + b) * 32;
       const uint64_t q = blkq + r;   // staging slot
       const uint4 tail = L.tails[q];
       const uint64_t point = L.point0 + blkq + (uint64_t)x;
@@ -294,6 +304,20 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_consta
 #pragma unroll
       for (int f = 0; f < 4; ++f) dst[f] = src[f];
     }
+    if (last) break;
+    base += total;
+    if (total < all) {   // on from the block of the first entry left
+      int b = 0;
+#pragma unroll
+      for (int st = 16; st > 0; st >>= 1)
+        if (__shfl_sync(0xffffffffu, incl, b + st - 1) <= total) b += st;
+      skip = total - __shfl_sync(0xffffffffu, excl, b) + (b == 0 ? skip : 0u);
+      B += b;
+    } else {
+      B += 32;
+      skip = 0;
+    }
+    mk = B + lane < Bend ? L.bmask[B + lane] : 0u;
   }
 }
 
@@ -349,11 +373,8 @@ static unsigned accept_rounds(const cp_handle* h, uint64_t n)
   return r < 1 ? 1u : (r > CP_UNW_MAXROUNDS ? (unsigned)CP_UNW_MAXROUNDS : (unsigned)r);
 }
 
-// The record builder loops grid-stride over its units: its grid is the blocks that are resident at
-// once, so no second wave runs after the first, and no more than there are units.  A range is four
-// units, or as many more (up to its 32 blocks) as still leave a unit for every resident warp: with a
-// quarter a unit a chunk of 50,021 points kept 196 of 4,736 warps busy, each for two rounds of
-// records (11.5 us for its 9,500 records, the chained launches aside).
+// The record builder's grid: the blocks that are resident at once, so no second wave runs after the first, and
+// no more than leave every warp a 32-point block.
 static int build_blocks(cp_handle* h)
 {
   if (h->build_per_sm < 0) {
@@ -363,12 +384,9 @@ static int build_blocks(cp_handle* h)
   }
   return h->num_sms * h->build_per_sm;
 }
-static unsigned build_grid(cp_handle* h, UnwLaunch& L)
+static unsigned build_grid(cp_handle* h, const UnwLaunch& L)
 {
-  const uint64_t resident = (uint64_t)build_blocks(h) * (CP_THREADS / 32);
-  L.unit_log2 = 2;
-  while ((1 << L.unit_log2) < CP_UNW_RANGE && (L.nrange << (L.unit_log2 + 1)) <= resident) ++L.unit_log2;
-  const uint64_t blocks = ((L.nrange << L.unit_log2) + CP_THREADS / 32 - 1) / (CP_THREADS / 32);
+  const uint64_t blocks = (L.nblk + CP_THREADS / 32 - 1) / (CP_THREADS / 32);
   return (unsigned)(blocks < (uint64_t)build_blocks(h) ? blocks : (uint64_t)build_blocks(h));
 }
 

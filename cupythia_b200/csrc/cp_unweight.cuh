@@ -31,7 +31,6 @@ struct UnwLaunch {
   uint64_t capacity;
   double* slots;
   unsigned rounds;             // points per thread of an accept block (k_unw_accept)
-  int unit_log2;               // work units per range of the record builder, as a power of two: 2 .. 5
   const float4* flow;          // flow output (v, ln J) per in-call point, or null (K1 only)
   const float* flow_u;         // the flow forward's accept draw per in-call point, or null: K1 draws it
 };
