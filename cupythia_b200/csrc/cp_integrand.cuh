@@ -536,7 +536,7 @@ CP_HD void cp_cteq_pair(const CpCteqPoly* cteq, float Q2, float lnxA, float lnxA
 // ------------------------------------------------------------------------------------------
 struct CpBrackets {
   float gg2gg, gg2qqbar, qg2qg, qqbar2gg, qqT, qqU, qqTU, qqST;
-  float qqD;   // qqU + qqTU - qqT
+  float qqUTU, qqD;   // qqU + qqTU with one rounding, and that less qqT
 };
 
 CP_HD void cp_brackets(const CpHadParams& P, float tp, float up, CpBrackets& b)
@@ -564,7 +564,8 @@ CP_HD void cp_brackets(const CpHadParams& P, float tp, float up, CpBrackets& b)
   b.qqU = cp_mulr(u4, ru2);
   b.qqTU = cp_mulr(-(8.f / 27.f), cp_mulr(rt, ru));
   b.qqST = cp_mulr(cp_mulr(-(8.f / 27.f), uu), rt);
-  b.qqD = cp_addr(cp_fmaf(u4, ru2, b.qqTU), -b.qqT);
+  b.qqUTU = cp_fmaf(u4, ru2, b.qqTU);
+  b.qqD = cp_addr(b.qqUTU, -b.qqT);
 }
 
 // SINGLE: the products of the opposite-flavour sum, the sea's among them, and of the q qbar -> g g
@@ -796,7 +797,7 @@ CP_HD void cp_process_shares(const float mask[5], const CpBrackets& b, const flo
   c[0] = mask[0] * G * b.gg2gg;
   c[1] = mask[1] * G * b.gg2qqbar;
   c[2] = mask[2] * b.qg2qg * (QA * Bq[2] + A[2] * QB);
-  c[3] = mask[3] * (QA * QB * b.qqT + Dsame * (0.5f * (b.qqU + b.qqTU - b.qqT)) + Dopp * b.qqST);
+  c[3] = mask[3] * (QA * QB * b.qqT + Dsame * (0.5f * b.qqD) + Dopp * b.qqST);
   c[4] = mask[4] * Dopp * b.qqbar2gg;
 }
 
@@ -829,7 +830,7 @@ CP_HD void cp_pick_pair(const CpHadParams& P, int k, const CpPoint& pt, float r1
     // pickInState over the 100 (q1, q2) pairs in initFlux order, walked row by row: the row
     // total A(q1) sum_q2 B(q2) br(q1, q2) from the three bracket classes first, then the pair
     // inside the chosen row
-    const float brS = 0.5f * (pt.b.qqU + pt.b.qqTU + pt.b.qqT), brO = pt.b.qqT + pt.b.qqST, brT = pt.b.qqT;
+    const float brS = 0.5f * cp_addr(pt.b.qqUTU, pt.b.qqT), brO = pt.b.qqT + pt.b.qqST, brT = pt.b.qqT;
     const float SB = B[0] + B[1] + B[3] + B[4] + 2.f * (B[5] + B[6] + B[7]);
     float row[10], tot2 = 0.f;
 #pragma unroll

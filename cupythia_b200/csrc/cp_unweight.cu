@@ -322,8 +322,7 @@ __global__ void __launch_bounds__(CP_THREADS, 4) k_unw_build(const __grid_consta
 }
 
 // K3, on request: the scale-variation ratios of the chunk's records, one record a lane in output
-// order, so every lane works (the record builder's lanes follow the accepted points of a quarter
-// range, 3 of 4 busy in the plain form) and the builder keeps its 64 registers.  A record's point gives
+// order, and the builder keeps its 64 registers.  A record's point gives
 // its staging slot through its block's accept mask; the kinematics and brackets come from the staged
 // coordinates and PDFs, as the record's did, and CTEQ5L runs at both varied scales together.  With the
 // ratios inside the builder (128 registers, a rolled CTEQ5L loop) the two took
