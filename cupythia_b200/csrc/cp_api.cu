@@ -393,6 +393,7 @@ __global__ void k_sigma(const CpHadParams P, const CpCteqPoly* cteq_g, int64_t n
       for (int k = 0; k < 5; ++k) m[k] = (mask >> k) & 1 ? 1.f : 0.f;
       float fa[8], fb[8];
       cp_cteq_pair<1>(cteq, q2f[i], logf(x1[i]), 0.f, logf(x2[i]), 0.f, fa, fb);
+      b.qqD = cp_addr(cp_addr(b.qqU, b.qqTU), -b.qqT);   // each term rounded, as in sigmaHat
       v = P.conv * pref * cp_channel_sum(m, b, fa, fb);
     } else {
       float br = 0.f;
