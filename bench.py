@@ -180,15 +180,15 @@ UNW_CHUNK = 1 << 24               # points per production chunk of the library (
 ALG_FP32_OPS_PER_POINT = 795
 ALG_MUFU_OPS_PER_POINT = 72
 # k_unw_accept, executed: FADD + FMUL + 2 FFMA lane operations per point from the ncu per-opcode
-# counters of a flow-form launch (profiles/k_unw_accept_production_2e24.md; packed two-lane
+# counters of a flow-form launch (profiles/counters_production_2e24.md; packed two-lane
 # forms counted per lane), i.e. the algorithm plus the FP32 precision bookkeeping (FMA residuals,
 # (hi, lo) logarithms) and the transcendentals' own arithmetic (the exp reduction's polynomial)
-EXEC_FLOP_PER_POINT = 1866.7
+EXEC_FLOP_PER_POINT = 1692.5
 FLOW_FLOP_PER_POINT = 35072.0     # k_flow_fwd: 2 x sum over couplings of (n_in*64 + 64*64 + 64*n_out) MACs
 # DRAM bytes (read + write) per point of the flow-form launches, from ncu captures of 2^24-point
-# launches of the same workload (profiles/traffic_flow_form_2e24.md); scaled to a launch's points
-TRAFFIC_PER_POINT = {"k_unw_accept": (343450880 + 688227584) / 2 ** 24,
-                     "k_flow_fwd_tc": (158976 + 275642624) / 2 ** 24}
+# launches of the same workload (profiles/counters_production_2e24.md); scaled to a launch's points
+TRAFFIC_PER_POINT = {"k_unw_accept": (343463168 + 671472384) / 2 ** 24,
+                     "k_flow_fwd_tc": (98048 + 275129344) / 2 ** 24}
 
 
 def production(it, n, records, k0, warmup, steps, pg, dev, stream, clocks=None):

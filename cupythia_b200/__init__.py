@@ -304,7 +304,7 @@ class Integrator:
     def flow_fuse_production(self, on=True):
         """Production passes in the flow form: flow forward, integrand and accept step in one
         tcgen05 kernel (on), or the forward over the pass followed by the accept kernel (off, the
-        default and the faster of the two)."""
+        default; about as fast, with the flow's output in memory)."""
         self._check(self.lib.cp_flow_fuse_production(self.h, 1 if on else 0))
 
     def flow_objective(self, p=2.0):

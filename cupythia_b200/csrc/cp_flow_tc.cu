@@ -553,7 +553,7 @@ int cp_flow_tc_status(cp_handle* h)
                                             : "k_flow_fwd_tc / k_flow_accept_tc: a tensor-core wait expired (results of this pass are invalid)");
 }
 
-// Test hook of the failure path: with on != 0 the issuing warps issue nothing, so every bounded
+// Test hook of the failure path: with on != 0 no layer is issued, so every bounded
 // wait of the epilogue expires (about one second of clock), the kernel raises its status word and
 // releases its TMEM, and the call returns CP_ERR_TIMEOUT with the context still usable.
 extern "C" int cp_flow_test_stall(cp_handle* h, int on)

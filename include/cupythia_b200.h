@@ -346,8 +346,8 @@ int cp_flow_select_kernel(cp_handle* h, int which);
 /* Production passes in the flow form (cp_unweight, cp_generate_host) with the tcgen05 forward:
  * on != 0 runs the flow forward, the integrand and the accept step as one kernel per chunk, the
  * flow's output never leaving the SM (no 20-byte-per-point flow buffer); 0 (default) runs the
- * forward over the pass first and the accept kernel on its stored output, which is faster on
- * B200 (17.9 ms against 19.3 ms per 2^27-point pass of the two kernels' work).  Both give the
+ * forward over the pass first and the accept kernel on its stored output, which is about as fast on
+ * B200 (2^26 points: 6.3 ms of the two kernels' work against 6.4 ms).  Both give the
  * same records, byte for byte, and the same counts; the sums of w and w^2 differ by their FP64
  * addition order. */
 int cp_flow_fuse_production(cp_handle* h, int on);
