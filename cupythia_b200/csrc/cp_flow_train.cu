@@ -102,7 +102,9 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_fwd_train(const uint2
   const uint64_t stride = (uint64_t)gridDim.x * CP_TRAIN_THREADS;
   const uint64_t rounds = (n + stride - 1) / stride;
   for (uint64_t r = 0; r < rounds; ++r) {
-    const uint64_t p = r * stride + (uint64_t)blockIdx.x * CP_TRAIN_THREADS + threadIdx.x;
+    // consecutive warps' points to consecutive blocks: a batch that is not whole blocks loads every SM alike (the
+    // same in k_flow_bwd; 65,536 points are 128 of 148 blocks; 100 steps 12.68 -> 12.50 ms)
+    const uint64_t p = r * stride + ((uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
     const bool active = p < n;
     float z[3], jv = 1.f, logdet = 0.f;
     uint32_t w[4] = {0x80000000u, 0x80000000u, 0x80000000u, 0u};
@@ -317,7 +319,7 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_bwd(const uint2* __re
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   const uint64_t rounds = (n + 32 * warps - 1) / (32 * warps);
   for (uint64_t r = 0; r < rounds; ++r) {
-    const uint64_t base = (r * warps + (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
+    const uint64_t base = (r * warps + (uint64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32;
     const uint64_t p = base + lane;
     const bool active = p < n;
     float dz[3] = {0.f, 0.f, 0.f}, cJ = 0.f;
