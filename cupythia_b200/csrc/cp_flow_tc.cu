@@ -28,20 +28,20 @@
 // TMEM, and the epilogues' stores share that bandwidth.  TMEM then holds 5 tiles of 96 columns, against 8
 // of 64 with A in shared memory.  2^26 points on a B200: 5.22 ms with two tiles per warpgroup, A in shared
 // memory and issuing warps of their own; 4.66 with those warps' operands uniform; 3.63 with 8 tiles in 8
-// warpgroups and no issuing warps; 3.19 with A in TMEM (4 tiles in flight: 3.42; 6 with half of A in
+// warpgroups and no issuing warps; 3.15 with A in TMEM (4 tiles in flight: 3.42; 6 with half of A in
 // shared memory: 3.19, and 3.61 with 5 of those).
 //
 // A production form (k_flow_accept_tc, opt-in through cp_flow_fuse_production) instantiates the
 // same body and takes each finished tile on, from registers, through the integrand and the
 // accept step of the production pass (the code of k_unw_accept, shared through cp_unweight.cuh),
 // so no flow output is stored.  Its records equal the two-kernel path's byte for byte; the time is about
-// the same (2^26 points: 6.4 ms, against 3.2 + 3.1 for the two kernels; 9.6 before this layout).
+// the same (2^26 points: 6.4 ms, against 3.1 + 3.1 for the two kernels; 9.6 before this layout).
 //
 // Synchronisation: rows written by tcgen05.st (waited for) are ordered before the MMAs by the
 // warpgroup's barrier; the issuing warp commits to the tile's mbarrier, which the warpgroup waits on before
 // reading TMEM.  Every wait on it is bounded (about 1 s of clock without progress); on expiry the waiting
-// warp raises its warpgroup's abort flag and issues no more, the warpgroup finishes its tile without
-// waiting and stops, the issuing warp waits (bounded) for the MMAs it still has in flight, and the kernel
+// warp raises its warpgroup's abort flag and issues no more, the warpgroup runs through its tiles without
+// waiting or touching TMEM, the issuing warp waits (bounded) for the MMAs it still has in flight, and the kernel
 // sets *status and releases its TMEM.
 #include "cp_flow.cuh"
 #include "cp_internal.cuh"
@@ -219,10 +219,11 @@ __device__ __forceinline__ void cp_tc_issue_l3(uint32_t d, uint32_t a, uint64_t 
     cp_tc_mma_ts(d, a + 8 * j, b16 + bw + ((CP_TC_B3 + j * 512) >> 4), CP_TC_IDESC16, j > 0 ? 1u : 0u);
 }
 
-// waits for the tile's MMAs; live turns false (for the whole warp) when the wait gives up
+// waits for the tile's MMAs; live turns false (for the whole warp) when the wait gives up, and then nothing is
+// waited for any more: the warpgroup's tiles run out at once, with their results invalid
 __device__ __forceinline__ void cp_tc_wait(uint32_t mbar, uint32_t& phase, volatile int* abort, bool& live)
 {
-  if (!__all_sync(0xffffffffu, cp_mbar_try(mbar, phase)))
+  if (live && !__all_sync(0xffffffffu, cp_mbar_try(mbar, phase)))
     live = __all_sync(0xffffffffu, cp_mbar_wait_bounded(mbar, phase, abort)) && live;
   phase ^= 1u;
   cp_tc_fence_after();
@@ -314,7 +315,8 @@ __device__ __forceinline__ void cp_flow_tc_body(const uint4* __restrict__ img_g,
   const uint64_t b64 = cp_tc_desc(sbase, 1024, 128), b16 = cp_tc_desc(sbase, 256, 128);
   const uint32_t td = tmem + (uint32_t)(wg * CP_TC_COLS), ta = td + CP_TC_A, mb = cp_smem_u32(&mbar[wg]);
   uint32_t ph = 0;
-  bool live = !stall;     // stall: test hook, no MMA is ever issued
+  bool live = !stall;     // MMAs are issued, and no wait of this warp has given up
+  if (stall) cp_mbar_wait_bounded(mb, 0u, abort);     // test hook: nothing is issued, so the wait expires
   // the warpgroup's rows of a step are written: its warps meet, one of them issues the next layer
   // (lay of coupling c) from warp-uniform operands
   auto publish = [&](int lay, int c) {
@@ -425,7 +427,6 @@ __device__ __forceinline__ void cp_flow_tc_body(const uint4* __restrict__ img_g,
         }
       }
     }
-    if (cp_bar_wg_or(bar_id, *abort != 0)) break;
   }
   // After an abort MMAs may still be in flight: every one this warpgroup issued has completed (bounded
   // wait) before the CTA releases its TMEM.
@@ -553,7 +554,7 @@ int cp_flow_tc_status(cp_handle* h)
                                             : "k_flow_fwd_tc / k_flow_accept_tc: a tensor-core wait expired (results of this pass are invalid)");
 }
 
-// Test hook of the failure path: with on != 0 no layer is issued, so every bounded
+// Test hook of the failure path: with on != 0 no layer is issued, so the first bounded
 // wait of the epilogue expires (about one second of clock), the kernel raises its status word and
 // releases its TMEM, and the call returns CP_ERR_TIMEOUT with the context still usable.
 extern "C" int cp_flow_test_stall(cp_handle* h, int on)

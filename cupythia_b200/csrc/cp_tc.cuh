@@ -240,18 +240,4 @@ __device__ __forceinline__ void cp_bar_wg(uint32_t id)
 {
   asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory");
 }
-// the same barrier with an OR-reduction of a predicate over the warpgroup
-__device__ __forceinline__ bool cp_bar_wg_or(uint32_t id, bool v)
-{
-  uint32_t out;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.u32 p, %2, 0;\n\t"
-      "bar.red.or.pred q, %1, 128, p;\n\t"
-      "selp.u32 %0, 1, 0, q;\n\t}\n"
-      : "=r"(out)
-      : "r"(id), "r"((uint32_t)v)
-      : "memory");
-  return out != 0;
-}
 #endif
