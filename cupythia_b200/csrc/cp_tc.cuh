@@ -164,11 +164,6 @@ __device__ __forceinline__ uint32_t cp_relu_bf2(float lo, float hi)
   return d;
 }
 
-__device__ __forceinline__ void cp_sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
-{
-  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
 __device__ __forceinline__ void cp_mbar_init(uint32_t mbar, uint32_t count)
 {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
@@ -190,19 +185,6 @@ __device__ __forceinline__ void cp_bulk_load(uint32_t dst, const void* src, uint
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(mbar)
                : "memory");
-}
-// non-blocking test of the phase `parity` of an mbarrier
-__device__ __forceinline__ bool cp_mbar_test(uint32_t mbar, uint32_t parity)
-{
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}\n"
-      : "=r"(ok)
-      : "r"(mbar), "r"(parity)
-      : "memory");
-  return ok != 0;
 }
 // Bounded wait for the phase `parity` of an mbarrier (try_wait suspends the thread in hardware
 // until the phase completes or a short time limit): gives up after CP_TC_WAIT_CYCLES clock cycles
