@@ -321,10 +321,14 @@ __global__ void __cluster_dims__(CP_FINISH_BLOCKS, 1, 1) __launch_bounds__(CP_FI
   __shared__ double sPart[4][CP_SLOT_HEAD + 3 * CP_MAX_BINS], sHead[CP_SLOT_HEAD];
   const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int rank = (int)cluster.block_rank(), lane = threadIdx.x & 31;
+  cluster.barrier_arrive();
   cp_next_may_launch();
   cp_wait_previous();
   if (rank == 0) cp_refine_load_edges(S, edges, nb);
   double* const part0 = cluster.map_shared_rank(&sPart[0][0], 0);
+  // the blocks of a cluster are placed together but need not have started together, and a block's shared memory
+  // may be written only once it runs: a pass of one slot leaves most blocks nothing to load before they store
+  cluster.barrier_wait();
   const int groups = (width + 3) / 4;
   for (int v = rank + CP_FINISH_BLOCKS * (threadIdx.x >> 5); v < 4 * groups; v += CP_FINISH_BLOCKS * (CP_FINISH_THREADS / 32)) {
     const int w = v & 3, k = 4 * (v >> 2) + (lane & 3);
