@@ -302,14 +302,12 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_bwd(const uint2* __re
   if (threadIdx.x == 0) {
     cp_mbar_init(bar, 1);
     cp_mbar_init_fence();
-    cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_PER);
   }
-  for (int j = threadIdx.x; j < CP_FLOW_NC * CP_FLOW_NB; j += blockDim.x) sBias[j] = bias_g[j];
-  __syncthreads();
-  // the weights above are older than the forward pass, which every chained kernel before this one has
-  // waited for; what follows is theirs
   cp_wait_previous();
   cp_next_may_launch();
+  if (threadIdx.x == 0) cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_PER);
+  for (int j = threadIdx.x; j < CP_FLOW_NC * CP_FLOW_NB; j += blockDim.x) sBias[j] = bias_g[j];
+  __syncthreads();
   const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
   // the batch's moments and size (all ranks' points when the batch is sharded)
   const double sig = sums[0] / n_batch;
@@ -958,9 +956,8 @@ static void train_buffers_done(cp_handle* h)
 }
 
 // The kernels of a step are chained launches: each starts its blocks, barriers and constants while the one
-// before it drains, and triggers the next only after its own wait, so whatever an earlier kernel than the
-// last has written (the weights, for the backward pass) is complete as well.  100 steps of 65,536 points:
-// 13.55 -> 12.75 ms.
+// before it drains, and reads what earlier kernels wrote only after its own wait (which alone promises that their
+// writes are visible, the weights of the step before among them).  100 steps of 65,536 points: 13.55 -> 12.75 ms.
 //
 // Phase 1 of a step: forward and integrand over the batch points [point0, point0 + count) at
 // counter iteration `iter` (Philox stream 2); moments[0..1] = (sum w, sum w^2) over them.

@@ -1,5 +1,5 @@
 """Orders in the kernels' sources that no run on one GPU shows to be missing: what has to have happened before another
-block's shared memory is touched."""
+block's shared memory is touched, and before a chained kernel reads what an earlier kernel writes."""
 import glob
 import os
 import re
@@ -60,3 +60,28 @@ def test_no_block_touches_another_s_shared_memory_before_the_cluster_runs(name):
         use = re.search(r"\b%s\b" % m.group(1), body[m.end():])
         assert use, m.group(1)
         assert re.search(r"\.(barrier_wait|sync)\(\)", body[:m.end() + use.start()]), (name, m.group(1))
+
+
+# written once, when the handle is created
+CONSTANT = {"cteq_g"}
+CHAINED = sorted(k for k, (_, b) in KERNELS.items() if "cp_wait_previous()" in b)
+
+
+@pytest.mark.parametrize("name", CHAINED)
+def test_no_chained_kernel_touches_global_memory_before_its_wait(name):
+    """Ahead of cp_wait_previous a kernel names none of its pointer parameters, and of a launch record's members only
+    whether a pointer is null."""
+    params, body = KERNELS[name]
+    head = body[:body.index("cp_wait_previous()")]
+    names = set(re.findall(r"\*\s*(?:__restrict__\s*)?(\w+)\s*(?:,|$)", params)) - CONSTANT
+    assert not {n for n in names if re.search(r"\b%s\b" % n, head)}
+    for rec in re.findall(r"(?:HadLaunch|UnwLaunch|FlowTrainBufs)\s+(\w+)", params):
+        used = set(re.findall(r"(?<!if \()\b%s\.(\w+)" % rec, head))
+        assert used <= {"nb", "n"}, (name, used)
+
+
+def test_chained_kernels_are_launched_as_such():
+    """Every kernel that a chained launch starts has the wait."""
+    for f in glob.glob(os.path.join(CSRC, "*.cu")):
+        for n in re.findall(r"cp_launch_chained(?:_smem)?\((k_\w+)", open(f).read()):
+            assert n in CHAINED
