@@ -21,6 +21,8 @@ int cp_fail_cuda(cp_handle* h, cudaError_t e, const char* what)
   return e == cudaErrorMemoryAllocation ? CP_ERR_NOMEM : CP_ERR_CUDA;
 }
 
+// Workspaces that grow: the capacity is zero from the moment the old block goes until the new one is there, so a
+// growth that fails leaves a workspace that the next call allocates, not one that counts as large and is null.
 int cp_ensure_slots(cp_handle* h, size_t doubles)
 {
   if (doubles <= h->slots_cap) return CP_OK;
@@ -28,6 +30,7 @@ int cp_ensure_slots(cp_handle* h, size_t doubles)
     CP_CUDA(h, cudaStreamSynchronize(h->stream));
     CP_CUDA(h, cudaFree(h->d_slots));
     h->d_slots = nullptr;
+    h->slots_cap = 0;
   }
   CP_CUDA(h, cudaMalloc(&h->d_slots, doubles * sizeof(double)));
   h->slots_cap = doubles;
@@ -67,6 +70,7 @@ static int ensure_kin(cp_handle* h, int64_t n)
   if (n <= h->kin_cap) return CP_OK;
   float** bufs[8] = {&h->d_x1, &h->d_x2, &h->d_sH, &h->d_tH, &h->d_uH, &h->d_as, &h->d_q2r, &h->d_q2f};
   CP_CUDA(h, cudaStreamSynchronize(h->stream));
+  h->kin_cap = h->kin_n = 0;   // the batch goes with its arrays
   for (auto b : bufs) {
     if (*b) CP_CUDA(h, cudaFree(*b));
     *b = nullptr;

@@ -120,17 +120,22 @@ __global__ void __launch_bounds__(CP_THREADS) k_flow_fwd(const uint2* __restrict
 // ------------------------------------------------------------------------------------------
 static size_t flow_fwd_smem() { return sizeof(uint2) * CP_FLOW_NC * CP_FLOW_P_FWD + sizeof(float) * CP_FLOW_NC * CP_FLOW_NB; }
 
+// The flow's arrays; d_flow comes last, so that it says the others are there.
 int cp_flow_ensure(cp_handle* h)
 {
   if (h->d_flow) return CP_OK;
-  CP_CUDA(h, cudaMalloc(&h->d_flow, sizeof(float) * CP_FLOW_NPARAM * 4));   // master, grad, m, v
-  CP_CUDA(h, cudaMemsetAsync(h->d_flow, 0, sizeof(float) * CP_FLOW_NPARAM * 4, h->stream));
-  CP_CUDA(h, cudaMalloc(&h->d_flow_pk, sizeof(uint2) * CP_FLOW_NC * CP_FLOW_P_PER));
-  CP_CUDA(h, cudaMalloc(&h->d_flow_bias, sizeof(float) * CP_FLOW_NC * CP_FLOW_NB));
-  CP_CUDA(h, cudaMalloc(&h->d_flow_ticket, sizeof(unsigned)));
+  if (!h->d_flow_pk) CP_CUDA(h, cudaMalloc(&h->d_flow_pk, sizeof(uint2) * CP_FLOW_NC * CP_FLOW_P_PER));
+  if (!h->d_flow_bias) CP_CUDA(h, cudaMalloc(&h->d_flow_bias, sizeof(float) * CP_FLOW_NC * CP_FLOW_NB));
+  if (!h->d_flow_ticket) CP_CUDA(h, cudaMalloc(&h->d_flow_ticket, sizeof(unsigned)));
   CP_CUDA(h, cudaMemsetAsync(h->d_flow_ticket, 0, sizeof(unsigned), h->stream));
   CP_CUDA(h, cudaFuncSetAttribute(k_flow_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)flow_fwd_smem()));
-  return cp_flow_tc_alloc(h);
+  const int rc = cp_flow_tc_alloc(h);
+  if (rc) return rc;
+  float* flow = nullptr;
+  CP_CUDA(h, cudaMalloc(&flow, sizeof(float) * CP_FLOW_NPARAM * 4));   // master, grad, m, v
+  h->d_flow = flow;
+  CP_CUDA(h, cudaMemsetAsync(h->d_flow, 0, sizeof(float) * CP_FLOW_NPARAM * 4, h->stream));
+  return CP_OK;
 }
 
 // The warp-level fragments (used by training and the mma.sync forward) are repacked at once; the
@@ -152,6 +157,7 @@ int cp_flow_buffer(cp_handle* h, uint64_t n)
     CP_CUDA(h, cudaFree(h->d_flow_buf));
     h->d_flow_buf = nullptr;
     h->d_flow_u = nullptr;
+    h->flow_buf_cap = 0;
   }
   // the points' (v, ln J), then their accept draws
   CP_CUDA(h, cudaMalloc(&h->d_flow_buf, (sizeof(float4) + sizeof(float)) * n));

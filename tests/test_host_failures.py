@@ -1,0 +1,91 @@
+"""What the host code does when an allocation fails, against a CUDA runtime without a GPU.
+
+A workspace that could not grow must not count as grown: the next, smaller call allocates again instead of
+launching a kernel on a null pointer."""
+import ctypes as C
+
+import pytest
+
+import host_runtime
+from cupythia_b200 import _lib
+
+OK, NOMEM = _lib.CP_OK, _lib.CP_ERR_NOMEM
+NONE = 1 << 62
+
+
+@pytest.fixture(scope="module")
+def rt(tmp_path_factory):
+    return host_runtime.load(host_runtime.build(str(tmp_path_factory.mktemp("host"))))
+
+
+@pytest.fixture
+def h(rt):
+    rt.fake_fail_above(NONE)
+    rt.fake_fail_nth(-1)
+    cfg, p = _lib.cp_config(), C.c_void_p()
+    assert rt.cp_config_default(C.byref(cfg)) == OK
+    assert rt.cp_create(C.byref(cfg), C.byref(p)) == OK
+    yield p
+    rt.fake_fail_above(NONE)
+    rt.fake_fail_nth(-1)
+    assert rt.cp_destroy(p) == OK
+    assert rt.fake_device_allocations() == rt.fake_pinned_allocations() == 0
+
+
+def _iterate(rt, h, n):
+    return rt.cp_vegas_iteration(h, n, 0, 1.5, C.byref(_lib.cp_result()))
+
+
+def test_flow_buffer_after_a_failed_growth(rt, h):
+    assert rt.cp_flow_init(h, 7) == OK and rt.cp_flow_enable(h, 1) == OK
+    assert _iterate(rt, h, 1 << 20) == OK
+    rt.fake_fail_above(1 << 30)
+    assert _iterate(rt, h, 1 << 28) == NOMEM
+    rt.fake_watch(b"k_flow_fwd_tc", 9)
+    assert _iterate(rt, h, 1 << 18) == OK
+    assert rt.fake_is_device(rt.fake_watched(), 16 << 18)
+
+
+def test_slots_after_a_failed_growth(rt, h):
+    assert rt.cp_set_wmax(h, 1.0) == OK
+    r = _lib.cp_unweight_result()
+    assert rt.cp_unweight(h, 300, 0, None, 0, C.byref(r)) == OK
+    rt.fake_fail_nth(0)
+    assert _iterate(rt, h, 1 << 20) == NOMEM
+    rt.fake_watch(b"k_unw_finish", 0)
+    assert rt.cp_unweight(h, 300, 0, None, 0, C.byref(r)) == OK
+    assert rt.fake_is_device(rt.fake_watched(), 64)
+
+
+@pytest.mark.parametrize("nth", range(8))
+def test_kinematics_after_a_failed_growth(rt, h, nth):
+    def set2kin(n):
+        return rt.cp_set2kin_batch(h, *[(C.c_float * n)() for _ in range(4)], n)
+
+    assert set2kin(100) == OK
+    rt.fake_fail_nth(nth)
+    assert set2kin(1000) == NOMEM
+    rt.fake_clear()
+    assert rt.cp_sigma_hat_batch(h, 111, 21, 21, (C.c_float * 1000)()) == OK   # no batch is set
+    assert rt.fake_count(b"launch") == 0
+    assert set2kin(50) == OK
+    assert rt.fake_count(b"malloc 200") == 8
+
+
+@pytest.mark.parametrize("nth", range(5))
+def test_flow_set_up_after_a_failed_allocation(rt, h, nth):
+    """Every array of the flow is there once a call on the flow succeeds."""
+    before = rt.fake_device_allocations()
+    rt.fake_fail_nth(nth)
+    assert rt.cp_flow_init(h, 7) == NOMEM
+    rt.fake_watch(b"k_flow_pack", 1)
+    assert rt.cp_flow_init(h, 7) == OK
+    assert rt.fake_is_device(rt.fake_watched(), 64)
+    assert rt.fake_device_allocations() == before + 5
+
+
+def test_pinned_records_after_a_failed_growth(rt, h):
+    per = (_lib.cp_result * 1000)()
+    rt.fake_fail_nth(0)
+    assert rt.cp_integrate(h, 1000, 64, 1.5, 0, per, C.byref(_lib.cp_result())) == NOMEM
+    assert rt.cp_integrate(h, 1, 64, 1.5, 0, per, C.byref(_lib.cp_result())) == OK
