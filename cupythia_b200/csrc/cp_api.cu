@@ -163,7 +163,8 @@ extern "C" int cp_destroy(cp_handle* h)
 {
   if (!h) return CP_OK;
   CpDeviceGuard guard(h->device);
-  if (h->stream) cudaStreamSynchronize(h->stream);
+  // kernels in flight write to the pinned memory below (a null stream is the default one, and can be busy as well)
+  cudaStreamSynchronize(h->stream);
   if (h->gen_copy) cudaStreamSynchronize(h->gen_copy);
   for (cudaEvent_t e : h->tpool) cudaEventDestroy(e);
   for (int k = 0; k < CP_GEN_BUFS; ++k) {

@@ -1,4 +1,5 @@
-"""What the host code does when an allocation fails, against a CUDA runtime without a GPU.
+"""What the host code allocates, waits for and gives back, and what it does when an allocation fails, against a CUDA
+runtime without a GPU.
 
 A workspace that could not grow must not count as grown: the next, smaller call allocates again instead of
 launching a kernel on a null pointer."""
@@ -89,3 +90,18 @@ def test_pinned_records_after_a_failed_growth(rt, h):
     rt.fake_fail_nth(0)
     assert rt.cp_integrate(h, 1000, 64, 1.5, 0, per, C.byref(_lib.cp_result())) == NOMEM
     assert rt.cp_integrate(h, 1, 64, 1.5, 0, per, C.byref(_lib.cp_result())) == OK
+
+
+def test_a_handle_s_work_ends_before_its_memory_goes(rt, h):
+    """The step calls return with their kernels in flight; on the default stream, too, nothing is unpinned or freed
+    before they are done."""
+    cfg, p = _lib.cp_config(), C.c_void_p()
+    assert rt.cp_config_default(C.byref(cfg)) == OK and rt.cp_create(C.byref(cfg), C.byref(p)) == OK
+    assert rt.cp_flow_init(p, 7) == OK
+    rt.fake_clear()
+    assert rt.cp_flow_step_moments(p, 0, 64, (C.c_double * 2)()) == OK
+    last = rt.fake_count(b"")
+    assert rt.fake_first(b"sync") == -1
+    assert rt.cp_destroy(p) == OK
+    gone = [rt.fake_first(e) for e in (b"unpin", b"unregister", b"free")]
+    assert last <= rt.fake_first(b"sync") < min(k for k in gone if k >= 0)
