@@ -40,9 +40,9 @@
 // Synchronisation: rows written by tcgen05.st (waited for) are ordered before the MMAs by the
 // warpgroup's barrier; the issuing warp commits to the tile's mbarrier, which the warpgroup waits on before
 // reading TMEM.  Every wait on it is bounded (about 1 s of clock without progress); on expiry the waiting
-// warp raises its warpgroup's abort flag and issues no more, the warpgroup runs through its tiles without
-// waiting or touching TMEM, the issuing warp waits (bounded) for the MMAs it still has in flight, and the kernel
-// sets *status and releases its TMEM.
+// warp raises its warpgroup's abort flag and issues no more, the warpgroup's warps run through their tiles without
+// waiting or touching TMEM, the issuing warp waits (bounded) for the MMAs it still has in flight, every warp
+// that gave up sets *status, and the kernel releases its TMEM.
 #include "cp_flow.cuh"
 #include "cp_internal.cuh"
 #include "cp_tc.cuh"
@@ -315,8 +315,8 @@ __device__ __forceinline__ void cp_flow_tc_body(const uint4* __restrict__ img_g,
   const uint64_t b64 = cp_tc_desc(sbase, 1024, 128), b16 = cp_tc_desc(sbase, 256, 128);
   const uint32_t td = tmem + (uint32_t)(wg * CP_TC_COLS), ta = td + CP_TC_A, mb = cp_smem_u32(&mbar[wg]);
   uint32_t ph = 0;
-  bool live = !stall;     // MMAs are issued, and no wait of this warp has given up
-  if (stall) cp_mbar_wait_bounded(mb, 0u, abort);     // test hook: nothing is issued, so the wait expires
+  bool live = stall != 1;     // MMAs are issued, and no wait of this warp has given up
+  if (stall == 1) cp_mbar_wait_bounded(mb, 0u, abort);     // test hook: nothing is issued, so the wait expires
   // the warpgroup's rows of a step are written: its warps meet, one of them issues the next layer
   // (lay of coupling c) from warp-uniform operands
   auto publish = [&](int lay, int c) {
@@ -428,16 +428,19 @@ __device__ __forceinline__ void cp_flow_tc_body(const uint4* __restrict__ img_g,
       }
     }
   }
+  // test hook: the last warp of a warpgroup gives up when the others are through (no arrival comes on this barrier)
+  if (stall == 2 && (warp & 3) == 3) live = __all_sync(0xffffffffu, cp_mbar_wait_bounded(cp_smem_u32(&mbar[CP_TC_WG]), 0u, abort));
   // After an abort MMAs may still be in flight: every one this warpgroup issued has completed (bounded
   // wait) before the CTA releases its TMEM.
-  if ((warp & 3) == 0 && !stall) {
+  if ((warp & 3) == 0 && stall != 1) {
     const uint32_t fin = cp_smem_u32(&mbar[8 + wg]);
     if (cp_elect()) cp_tc_commit(fin);
     __syncwarp();
     volatile int fin_abort = 0;
-    if (!cp_mbar_wait_bounded(fin, 0u, &fin_abort)) *abort = 1;
+    live = __all_sync(0xffffffffu, cp_mbar_wait_bounded(fin, 0u, &fin_abort)) && live;
   }
-  if (row == 0 && *abort) *(volatile int*)status = 1;
+  // every warp reports its own: no barrier follows its last wait, so another warp's flag may come too late to be seen
+  if (!live && (tid & 31) == 0) *(volatile int*)status = 1;
   if constexpr (ACCEPT) {
     double v[7];
     cp_unw_warp_sums(S, v);
@@ -556,10 +559,11 @@ int cp_flow_tc_status(cp_handle* h)
 
 // Test hook of the failure path: with on != 0 no layer is issued, so the first bounded
 // wait of the epilogue expires (about one second of clock), the kernel raises its status word and
-// releases its TMEM, and the call returns CP_ERR_TIMEOUT with the context still usable.
+// releases its TMEM, and the call returns CP_ERR_TIMEOUT with the context still usable.  With on = 2 the layers
+// are issued and the last warp of each warpgroup waits in vain after its last tile.
 extern "C" int cp_flow_test_stall(cp_handle* h, int on)
 {
   CP_CHECK_HANDLE(h);
-  h->flow_stall = on ? 1 : 0;
+  h->flow_stall = on == 2 ? 2 : on != 0;
   return CP_OK;
 }
