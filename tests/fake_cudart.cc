@@ -17,7 +17,7 @@ std::map<const void*, std::string> kernels;     // host stub -> kernel name
 std::map<void*, size_t> device, pinned;         // live allocations
 size_t fail_above = SIZE_MAX;                   // a larger allocation fails ...
 long fail_nth = -1;                             // ... and so does the n-th from now (0: the next)
-std::vector<std::string> events;                // "malloc 123", "free", "pin 123", "unpin", "sync", "launch name"
+std::vector<std::string> events;                // "malloc 123", "free", "pin 123", "unpin", "chunk", "sync", "launch name"
 std::string watch_name;
 int watch_arg = -1;
 void* watched = nullptr;
@@ -126,6 +126,7 @@ cudaError_t cudaFree(void* p)
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned)
 {
   if (refused(n)) return cudaErrorMemoryAllocation;
+  if (pinned.empty()) events.push_back("chunk");   // the driver maps one for the first and keeps it to the last
   *p = map(n);
   pinned[*p] = n;
   events.push_back("pin " + std::to_string(n));
@@ -139,18 +140,6 @@ cudaError_t cudaFreeHost(void* p)
   pinned.erase(a);
   events.push_back("unpin");
   return cudaSuccess;
-}
-cudaError_t cudaHostRegister(void* p, size_t n, unsigned)
-{
-  if (refused(n)) return cudaErrorMemoryAllocation;
-  pinned[p] = n;
-  events.push_back("register " + std::to_string(n));
-  return cudaSuccess;
-}
-cudaError_t cudaHostUnregister(void* p)
-{
-  events.push_back("unregister");
-  return pinned.erase(p) ? cudaSuccess : cudaErrorInvalidValue;
 }
 cudaError_t cudaMemset(void* p, int v, size_t n)
 {
