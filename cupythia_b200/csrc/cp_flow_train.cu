@@ -921,6 +921,7 @@ static size_t fwd_smem() { return sizeof(uint2) * CP_FLOW_NC * CP_FLOW_P_FWD + s
 // padding of the 16-wide operands) must read as zero.
 static int train_buffers(cp_handle* h, uint64_t count, FlowTrainBufs& t)
 {
+  h->ftrain_idle = 0;
   if (!h->d_ftrain || count > h->ftrain_cap) {
     if (h->d_ftrain) {
       CP_CUDA(h, cudaStreamSynchronize(h->stream));
@@ -941,18 +942,34 @@ static int train_buffers(cp_handle* h, uint64_t count, FlowTrainBufs& t)
   return CP_OK;
 }
 
-// Ends a call's use of the training buffers: no step is pending any more, and buffers above
-// CP_TRAIN_KEEP bytes go back to the device.  Smaller ones stay in the handle until it is destroyed
-// (batches of 65,536 points: 160 MB), since allocating and freeing them took up to 3 ms of a call.
-#define CP_TRAIN_KEEP ((size_t)1 << 30)
-static void train_buffers_done(cp_handle* h)
+// Gives the training buffers back, unless a step is pending in them.
+static void train_release(cp_handle* h)
 {
-  h->ftrain_count = 0;
-  if (!h->d_ftrain || train_bytes(h->ftrain_cap) <= CP_TRAIN_KEEP) return;
+  if (!h->d_ftrain || h->ftrain_count) return;
   cudaStreamSynchronize(h->stream);
   cudaFree(h->d_ftrain);
   h->d_ftrain = nullptr;
   h->ftrain_cap = h->ftrain_zeroed = 0;
+}
+
+// A production pass begins: the CP_TRAIN_IDLE-th since the buffers were last used gives them back.  Freeing and
+// allocating them again takes 0.8 ms (a pass of 50,021 points: 0.04), so a program that trains and produces in
+// turn keeps them, and one that has trained and now produces loses that time once.
+#define CP_TRAIN_IDLE 8
+void cp_train_idle(cp_handle* h)
+{
+  if (h->d_ftrain && ++h->ftrain_idle >= CP_TRAIN_IDLE) train_release(h);
+}
+
+// Ends a call's use of the training buffers: no step is pending any more, and buffers above
+// CP_TRAIN_KEEP bytes go back to the device.  Smaller ones stay in the handle for the next training call
+// (batches of 65,536 points: 160 MB), since allocating and freeing them took up to 3 ms of a call, until production
+// passes give them back.
+#define CP_TRAIN_KEEP ((size_t)1 << 30)
+static void train_buffers_done(cp_handle* h)
+{
+  h->ftrain_count = 0;
+  if (train_bytes(h->ftrain_cap) > CP_TRAIN_KEEP) train_release(h);
 }
 
 // The kernels of a step are chained launches: each starts its blocks, barriers and constants while the one

@@ -176,6 +176,7 @@ struct cp_handle {
   // ftrain_count points), kept between the phases of a data-parallel step
   void* d_ftrain = nullptr;
   uint64_t ftrain_cap = 0, ftrain_count = 0;
+  int ftrain_idle = 0;                     // production passes since they were last used
   uint64_t ftrain_zeroed = 0;              // the layout (count) whose never-written parts are zero
   double* h_losses = nullptr;              // batch losses of a training run, mapped pinned memory
   int losses_cap = 0;
@@ -213,6 +214,7 @@ int cp_flow_tc_repack(cp_handle* h);
 int cp_flow_tc_enqueue(cp_handle* h, uint64_t point0, uint64_t n, uint32_t iter, uint32_t stream, float4* out,
                        float* uout);
 int cp_flow_tc_status(cp_handle* h);
+void cp_train_idle(cp_handle* h);
 
 // Makes `dev` the calling thread's current device for the rest of the scope and restores the
 // caller's device at its end, so one host thread can drive handles on several GPUs.

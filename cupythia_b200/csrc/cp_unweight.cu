@@ -583,6 +583,7 @@ extern "C" int cp_unweight(cp_handle* h, uint64_t n_points, uint32_t iter, cp_ev
   if (n_points > (1ull << 32)) return cp_fail(h, CP_ERR_INVALID, "at most 2^32 points per production call");
   if (h->scalew && capacity > h->scalew_cap)
     return cp_fail(h, CP_ERR_INVALID, "cp_unweight: record capacity exceeds the scale-weight buffer (cp_set_scale_weights)");
+  cp_train_idle(h);
   // chunks of at most CP_UNW_CHUNK points; the running record count (d_counter) places each
   // chunk's records after the previous chunk's
   const uint64_t nsub = (n_points + CP_UNW_CHUNK - 1) / CP_UNW_CHUNK;
@@ -669,6 +670,7 @@ extern "C" int cp_generate_host(cp_handle* h, uint64_t n_points, uint32_t iter, 
   if (capacity && !records_host) return cp_fail(h, CP_ERR_INVALID, "cp_generate_host: null records");
   const double wm0 = h->wmax_host;
   if (!(wm0 > 0)) return cp_fail(h, CP_ERR_INVALID, "cp_generate_host: no threshold");
+  cp_train_idle(h);
   if (chunk > n_points) chunk = n_points;
   if (chunk > CP_UNW_CHUNK) chunk = CP_UNW_CHUNK;
   const uint64_t nchunks = (n_points + chunk - 1) / chunk;

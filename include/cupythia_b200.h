@@ -362,7 +362,8 @@ int cp_flow_enable(cp_handle* h, int on);
 /* n_steps Adam steps (learning rate lr) on batches of `batch` points (counter stream 2) drawn
  * through the current flow and VEGAS grid, minimising <w^2>/<w>^2; loss_host (n_steps doubles,
  * may be NULL) receives each batch's value before its update.  The training buffers (2.4 KB per
- * point) stay in the handle for the next call up to 1 GiB; larger ones are freed on return. */
+ * point) stay in the handle for the next call up to 1 GiB, until eight production passes (cp_unweight,
+ * cp_generate_host) have run without another; larger ones are freed on return. */
 int cp_flow_train(cp_handle* h, int n_steps, uint64_t batch, double lr, double* loss_host);
 /* Training objective of cp_flow_train and the data-parallel steps: the relative p-th moment of
  * the weights <w^p>/<w>^p, 2 <= p <= 8 (default 2: <w^2>/<w>^2 = 1 + Var[w]/sigma^2, the weight

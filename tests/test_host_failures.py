@@ -135,3 +135,35 @@ def test_a_handle_that_cannot_be_made_leaves_nothing(rt, h, nth):
     else:
         assert rc == NOMEM and not p.value
     assert (rt.fake_device_allocations(), rt.fake_pinned_allocations()) == (dev, pin)
+
+
+@pytest.mark.parametrize("produce", ["unweight", "generate_host"])
+def test_production_gives_the_training_buffers_back(rt, h, produce):
+    """Training keeps its buffers for the next call and over a few production passes; the eighth in a row frees
+    them, but not those of a step that is not finished."""
+    n, chunk = 300, (C.c_uint8 * (300 * 64 + 16))()
+    at = (C.addressof(chunk) + 15) & ~15
+
+    def pass_():
+        r = _lib.cp_unweight_result()
+        if produce == "unweight":
+            return rt.cp_unweight(h, n, 0, at, n, C.byref(r))
+        return rt.cp_generate_host(h, n, 0, n, at, n, C.byref(r))
+
+    assert rt.cp_set_wmax(h, 1.0) == OK and rt.cp_flow_init(h, 7) == OK
+    assert pass_() == OK and rt.cp_flow_sample(h, 0, 64, 0, 0, at) == OK
+    before = rt.fake_device_bytes()
+    assert rt.cp_flow_train(h, 1, 4096, 1e-3, None) == OK
+    kept = rt.fake_device_bytes() - before
+    assert 2000 * 4096 < kept < 1 << 30
+    for _ in range(2):
+        assert all(pass_() == OK for _ in range(7))
+        assert rt.fake_device_bytes() == before + kept
+        assert rt.cp_flow_train(h, 1, 4096, 1e-3, None) == OK
+    assert all(pass_() == OK for _ in range(8))
+    assert rt.fake_device_bytes() == before
+    moments, loss = (C.c_double * 2)(), C.c_double()
+    assert rt.cp_flow_step_moments(h, 0, 4096, moments) == OK
+    assert all(pass_() == OK for _ in range(9))
+    assert rt.fake_device_bytes() == before + kept
+    assert rt.cp_flow_step_gradient(h, moments, 4096, None, C.byref(loss)) == OK
