@@ -560,7 +560,8 @@ int cp_flow_tc_status(cp_handle* h)
 // Test hook of the failure path: with on != 0 no layer is issued, so the first bounded
 // wait of the epilogue expires (about one second of clock), the kernel raises its status word and
 // releases its TMEM, and the call returns CP_ERR_TIMEOUT with the context still usable.  With on = 2 the layers
-// are issued and the last warp of each warpgroup waits in vain after its last tile.
+// are issued and the last warp of each warpgroup waits in vain after its last tile.  In training on = 1 leaves out the
+// copies of the weights into shared memory, whose bounded waits expire.
 extern "C" int cp_flow_test_stall(cp_handle* h, int on)
 {
   CP_CHECK_HANDLE(h);

@@ -56,7 +56,7 @@ struct FlowTrainBufs {
 #define CP_TRAIN_THREADS 512
 
 // Starts the copies of the first `count` fragments of every coupling into shared memory (one thread,
-// which has initialised the barrier), and the bounded wait for them (whole warps; on expiry the
+// which has initialised the barrier; under the test hook, stall = 1, no kernel does), and the bounded wait for them (whole warps; on expiry the
 // status word is raised and the copies get one more bounded wait before the warp may leave).
 __device__ __forceinline__ void cp_train_weights_load(uint32_t bar, uint2* dst, const uint2* __restrict__ pk_g, int count)
 {
@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_fwd_train(const uint2
                                                                const double* __restrict__ edges, int nb,
                                                                uint64_t seed, uint32_t iter, uint32_t stream, uint64_t point0,
                                                                uint64_t n, float* __restrict__ zs, float4* __restrict__ vj,
-                                                               int* __restrict__ status)
+                                                               int* __restrict__ status, int stall)
 {
   extern __shared__ __align__(16) uint2 sPk[];
   float* sBias = reinterpret_cast<float*>(sPk + CP_FLOW_NC * CP_FLOW_P_FWD);
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_fwd_train(const uint2
   }
   cp_wait_previous();
   cp_next_may_launch();
-  if (threadIdx.x == 0) cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_FWD);
+  if (threadIdx.x == 0 && stall != 1) cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_FWD);
   for (int k = threadIdx.x; k < 3 * nb; k += CP_TRAIN_THREADS) {
     const int d = k / nb, b = k - d * nb;
     sEdge[d][b] = make_float2((float)edges[d * (nb + 1) + b], (float)(edges[d * (nb + 1) + b + 1] - edges[d * (nb + 1) + b]));
@@ -293,7 +293,7 @@ __device__ __forceinline__ void cp_flow_back64(const uint32_t (&a)[2][KT][4], co
 __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_bwd(const uint2* __restrict__ pk_g, const float* __restrict__ bias_g, uint64_t n,
                                                   double n_batch, const float* __restrict__ zs, const float4* __restrict__ vj,
                                                   const float4* __restrict__ wg, const double* __restrict__ sums,
-                                                  FlowTrainBufs out, float loss_p, int* __restrict__ status)
+                                                  FlowTrainBufs out, float loss_p, int* __restrict__ status, int stall)
 {
   extern __shared__ __align__(16) uint2 sPk[];   // all CP_FLOW_P_PER fragments of the 4 couplings, then biases
   float* sBias = reinterpret_cast<float*>(sPk + CP_FLOW_NC * CP_FLOW_P_PER);
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(CP_TRAIN_THREADS) k_flow_bwd(const uint2* __re
   }
   cp_wait_previous();
   cp_next_may_launch();
-  if (threadIdx.x == 0) cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_PER);
+  if (threadIdx.x == 0 && stall != 1) cp_train_weights_load(bar, sPk, pk_g, CP_FLOW_P_PER);
   for (int j = threadIdx.x; j < CP_FLOW_NC * CP_FLOW_NB; j += blockDim.x) sBias[j] = bias_g[j];
   __syncthreads();
   const int lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
@@ -983,7 +983,7 @@ static int flow_phase_moments(cp_handle* h, const FlowTrainBufs& t, uint64_t poi
 {
   CP_CUDA(h, cp_launch_chained_smem(k_flow_fwd_train, h->num_sms, CP_TRAIN_THREADS, fwd_smem(), h->stream, h->d_flow_pk,
                                     h->d_flow_bias, h->d_edges, h->nb, h->cfg.seed, iter, 2u, point0, count, t.zs, t.vj,
-                                    h->mail->status + 1));
+                                    h->mail->status + 1, h->flow_stall));
   const int gblk = h->num_sms * 4;
   int rc = cp_ensure_slots(h, (size_t)2 * gblk);
   if (rc) return rc;
@@ -1007,7 +1007,7 @@ static int flow_phase_gradient(cp_handle* h, const FlowTrainBufs& t, uint64_t co
   }
   CP_CUDA(h, cp_launch_chained_smem(k_flow_bwd, h->num_sms, CP_TRAIN_THREADS, bwd_smem(), h->stream, h->d_flow_pk, h->d_flow_bias,
                                     count, (double)n_batch, t.zs, t.vj, t.wg, t.sums, t, (float)h->flow_loss_p,
-                                    h->mail->status + 1));
+                                    h->mail->status + 1, h->flow_stall));
   float* G = h->d_flow + CP_FLOW_NPARAM;
   // at most CP_WG_MAXBLK blocks per coupling and layer; chunks are whole multiples of the staged
   // rows.  The three launches share the grid, so together they write every entry of the

@@ -354,7 +354,9 @@ int cp_flow_fuse_production(cp_handle* h, int on);
 /* Test hook of the failure path of the tcgen05 forward (no reference counterpart): with on != 0
  * the kernel issues no MMA, every bounded wait expires after about one second, the kernel
  * releases its tensor memory and the call returns CP_ERR_TIMEOUT; the handle stays usable.  on = 2:
- * the MMAs are issued and one warp of each warpgroup alone waits in vain, after its last tile. */
+ * the MMAs are issued and one warp of each warpgroup alone waits in vain, after its last tile.  Training
+ * with on = 1 leaves out the copies of the weights into shared memory: the same error, and parameters
+ * that are not to be used (cp_flow_set_state). */
 int cp_flow_test_stall(cp_handle* h, int on);
 /* Routes cp_vegas_iteration / cp_integrate / cp_point_weights / cp_unweight / cp_generate_host
  * through the flow (on = 1) or the Philox words directly (on = 0). */
