@@ -568,29 +568,45 @@ CP_HD void cp_brackets(const CpHadParams& P, float tp, float up, CpBrackets& b)
   b.qqD = cp_addr(b.qqUTU, -b.qqT);
 }
 
-// SINGLE: the products of the opposite-flavour sum, the sea's among them, and of the q qbar -> g g
-// term are each rounded instead of fused (the nominal sum of the scale-variation ratios has them so).
+// Flavour sums over q = +-1..+-5 (s, c, b enter twice: quark = antiquark; 2 x is exact): the quarks of each beam,
+// the pairs of equal and of opposite flavour, and the gluons' product.
+// SINGLE: the products of the opposite-flavour sum, the sea's among them, are each rounded instead of fused.  The
+// kernels that run over records have them so: they need the products by themselves as well (the pair picks), and
+// the process picks and scale ratios that programs have stored were formed from those.
+struct CpFlavourSums {
+  float QA, QB, Dsame, Dopp, G;
+};
 template <bool SINGLE = false>
-CP_HD float cp_channel_sum(const float mask[5], const CpBrackets& b, const float A[8], const float Bq[8])
+CP_HD CpFlavourSums cp_flavour_sums(const float A[8], const float Bq[8])
 {
-  // flavour sums over q = +-1..+-5 (s, c, b enter twice: quark = antiquark; 2 x is exact)
-  float QA = A[0] + A[1] + A[3] + A[4] + 2.f * (A[5] + A[6] + A[7]);
-  float QB = Bq[0] + Bq[1] + Bq[3] + Bq[4] + 2.f * (Bq[5] + Bq[6] + Bq[7]);
+  CpFlavourSums f;
+  f.QA = A[0] + A[1] + A[3] + A[4] + 2.f * (A[5] + A[6] + A[7]);
+  f.QB = Bq[0] + Bq[1] + Bq[3] + Bq[4] + 2.f * (Bq[5] + Bq[6] + Bq[7]);
   const float sea = 2.f * (SINGLE ? cp_addr(cp_addr(cp_mulr(A[5], Bq[5]), cp_mulr(A[6], Bq[6])), cp_mulr(A[7], Bq[7]))
                                   : cp_fmaf(A[7], Bq[7], cp_fmaf(A[5], Bq[5], cp_mulr(A[6], Bq[6]))));
-  const float Dsame = cp_addr(cp_fmaf(A[4], Bq[4], cp_fmaf(A[3], Bq[3], cp_fmaf(A[0], Bq[0], cp_mulr(A[1], Bq[1])))), sea);
+  f.Dsame = cp_addr(cp_fmaf(A[4], Bq[4], cp_fmaf(A[3], Bq[3], cp_fmaf(A[0], Bq[0], cp_mulr(A[1], Bq[1])))), sea);
   const float d4 = SINGLE ? cp_addr(cp_addr(cp_addr(cp_mulr(A[0], Bq[4]), cp_mulr(A[4], Bq[0])), cp_mulr(A[1], Bq[3])),
                                     cp_mulr(A[3], Bq[1]))
                           : cp_fmaf(A[3], Bq[1], cp_fmaf(A[1], Bq[3], cp_fmaf(A[0], Bq[4], cp_mulr(A[4], Bq[0]))));
-  const float Dopp = cp_addr(d4, sea);
-  const float G = cp_mulr(A[2], Bq[2]);
+  f.Dopp = cp_addr(d4, sea);
+  f.G = cp_mulr(A[2], Bq[2]);
+  return f;
+}
+
+// SINGLE, the nominal sum under the scale-variation ratios: the opposite-flavour sum as above, and the q qbar -> g g
+// term rounded before it is added.  It is thus not bit for bit the one in the weight (nor the varied ones above it);
+// either is within its rounding.
+template <bool SINGLE = false>
+CP_HD float cp_channel_sum(const float mask[5], const CpBrackets& b, const float A[8], const float Bq[8])
+{
+  const CpFlavourSums f = cp_flavour_sums<SINGLE>(A, Bq);
   // the masks are 0 or 1, so their products are exact
-  const float qg = cp_mulr(cp_mulr(mask[2], b.qg2qg), cp_fmaf(QA, Bq[2], cp_mulr(A[2], QB)));
-  float sum = cp_fmaf(G, mask[0] * b.gg2gg + mask[1] * b.gg2qqbar, qg);
+  const float qg = cp_mulr(cp_mulr(mask[2], b.qg2qg), cp_fmaf(f.QA, Bq[2], cp_mulr(A[2], f.QB)));
+  float sum = cp_fmaf(f.G, mask[0] * b.gg2gg + mask[1] * b.gg2qqbar, qg);
   // Sigma2qq2qq::sigmaHat: identical 1/2 (T + U + TU), q qbar T + ST, otherwise T
-  const float qq = cp_fmaf(Dopp, b.qqST, cp_fmaf(cp_mulr(QA, QB), b.qqT, cp_mulr(Dsame, 0.5f * b.qqD)));
+  const float qq = cp_fmaf(f.Dopp, b.qqST, cp_fmaf(cp_mulr(f.QA, f.QB), b.qqT, cp_mulr(f.Dsame, 0.5f * b.qqD)));
   sum = cp_fmaf(mask[3], qq, sum);
-  const float m4 = cp_mulr(mask[4], Dopp);
+  const float m4 = cp_mulr(mask[4], f.Dopp);
   return SINGLE ? cp_addr(sum, cp_mulr(m4, b.qqbar2gg)) : cp_fmaf(m4, b.qqbar2gg, sum);
 }
 
@@ -784,21 +800,18 @@ CP_HD float cp_qq_pair_bracket(const CpBrackets& b, int id1, int id2)
   return b.qqT;
 }
 
-// Process shares at one point: {gg2gg, gg2qqbar, qg2qg, qq2qq, qqbar2gg}
-CP_HD void cp_process_shares(const float mask[5], const CpBrackets& b, const float* A, const float* Bq, float c[5])
+// Process shares at one point: {gg2gg, gg2qqbar, qg2qg, qq2qq, qqbar2gg}, and their sum.  Every rounding is named, as
+// in the integrand, so that no change around the record builder moves a process pick (1.2e11 records: none had
+// another byte than with the compiler's choice; masks are 0 or 1, so products with them are exact).
+CP_HD float cp_process_shares(const float mask[5], const CpBrackets& b, const float* A, const float* Bq, float c[5])
 {
-  float QA = A[0] + A[1] + A[3] + A[4] + 2.f * (A[5] + A[6] + A[7]);
-  float QB = Bq[0] + Bq[1] + Bq[3] + Bq[4] + 2.f * (Bq[5] + Bq[6] + Bq[7]);
-  float Dsame = A[0] * Bq[0] + A[1] * Bq[1] + A[3] * Bq[3] + A[4] * Bq[4] +
-                2.f * (A[5] * Bq[5] + A[6] * Bq[6] + A[7] * Bq[7]);
-  float Dopp = A[0] * Bq[4] + A[4] * Bq[0] + A[1] * Bq[3] + A[3] * Bq[1] +
-               2.f * (A[5] * Bq[5] + A[6] * Bq[6] + A[7] * Bq[7]);
-  float G = A[2] * Bq[2];
-  c[0] = mask[0] * G * b.gg2gg;
-  c[1] = mask[1] * G * b.gg2qqbar;
-  c[2] = mask[2] * b.qg2qg * (QA * Bq[2] + A[2] * QB);
-  c[3] = mask[3] * (QA * QB * b.qqT + Dsame * (0.5f * b.qqD) + Dopp * b.qqST);
-  c[4] = mask[4] * Dopp * b.qqbar2gg;
+  const CpFlavourSums f = cp_flavour_sums<true>(A, Bq);
+  c[0] = cp_mulr(mask[0] * f.G, b.gg2gg);
+  c[1] = cp_mulr(mask[1] * f.G, b.gg2qqbar);
+  c[2] = cp_mulr(mask[2] * b.qg2qg, cp_fmaf(f.QA, Bq[2], cp_mulr(A[2], f.QB)));
+  c[3] = mask[3] * cp_fmaf(f.Dopp, b.qqST, cp_fmaf(cp_mulr(f.QA, f.QB), b.qqT, cp_mulr(f.Dsame, 0.5f * b.qqD)));
+  c[4] = cp_mulr(mask[4] * f.Dopp, b.qqbar2gg);
+  return cp_addr(cp_addr(cp_addr(cp_addr(c[0], c[1]), c[2]), c[3]), c[4]);
 }
 
 // pickInState of process k (0..4 = codes 111..115; SigmaProcess.cc:486-508) with uniform r1 and
@@ -890,11 +903,10 @@ CP_HD void cp_pick_flavours(const CpHadParams& P, const CpPoint& pt, float r0, f
                             int& code, int id[4])
 {
   float c[5];
-  cp_process_shares(P.mask, pt.b, pt.fa, pt.fb, c);
-  float tot = c[0] + c[1] + c[2] + c[3] + c[4];
-  float t = r0 * tot;
+  const float tot = cp_process_shares(P.mask, pt.b, pt.fa, pt.fb, c);
+  float t = cp_mulr(r0, tot);
   int k = 0;
-  while (k < 4 && (t >= c[k] || c[k] <= 0.f)) { t -= c[k]; ++k; }
+  while (k < 4 && (t >= c[k] || c[k] <= 0.f)) { t = cp_addr(t, -c[k]); ++k; }
   if (c[k] <= 0.f) { k = 0; while (k < 4 && !(c[k] > 0.f)) ++k; }
   code = 111 + k;
   cp_pick_pair(P, k, pt, r1, r3, id);
