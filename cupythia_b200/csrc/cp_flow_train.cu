@@ -720,7 +720,7 @@ __device__ __forceinline__ void cp_wgt_layer(const uint8_t* __restrict__ A, cons
   }
 }
 
-__global__ void __launch_bounds__(128) k_flow_wgrad_tc(FlowTrainBufs t, uint64_t n, int chunk, int* __restrict__ status)
+__global__ void __launch_bounds__(128) k_flow_wgrad_tc(FlowTrainBufs t, int chunk, int* __restrict__ status)
 {
   __shared__ __align__(1024) uint8_t smem[4 * CP_WGT_BYTES(64)];   // two A and two B stages
   __shared__ float sBias[128];
@@ -1016,7 +1016,7 @@ static int flow_phase_gradient(cp_handle* h, const FlowTrainBufs& t, uint64_t co
   const int nblk = (int)((count + chunk - 1) / chunk);
   if (h->flow_kernel == 0) {
     // tensor cores (tcgen05): every coupling and layer shape in one launch
-    CP_CUDA(h, cp_launch_chained_smem(k_flow_wgrad_tc, dim3((unsigned)nblk, CP_FLOW_NC, 3), 128, 0, h->stream, t, count, (int)chunk,
+    CP_CUDA(h, cp_launch_chained_smem(k_flow_wgrad_tc, dim3((unsigned)nblk, CP_FLOW_NC, 3), 128, 0, h->stream, t, (int)chunk,
                                       h->mail->status + 1));
   } else {
     // warp-level mma.sync, one launch per layer shape (the cross-check path)

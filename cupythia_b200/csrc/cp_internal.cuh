@@ -136,7 +136,7 @@ struct cp_handle {
   double* d_wmax = nullptr;                // [0] threshold used by cp_unweight, [1] quantile q
   unsigned long long* d_counter = nullptr; // accepted-event counter
   // production staging for pdfbuf_cap points (K1 -> K2): PDFs and record tails per point, accept
-  // masks per 32-point block, totals and output offsets per 1024-point range; per-chunk sums
+  // masks per 32-point block, totals and output offsets per 1024-point range
   void* d_staging = nullptr;               // one allocation for the arrays below
   float4* d_pdfbuf = nullptr;
   uint4* d_tails = nullptr;

@@ -6,11 +6,13 @@
 // 383-385).  Per 32-point block (one warp's points) it stores the warp's accept mask and adds
 // the number accepted to its 1024-point range's total (an integer atomic: exact in any order),
 // and packs the accepted points' event weights, mapped coordinates and 16 PDF values, in point
-// order, at the front of the block's staging slots.  A one-block scan of the range totals gives each range's output offset, so the records
+// order, at the front of the block's staging slots.  A launch of two blocks then adds the accept blocks' sums and
+// scans the range totals into the ranges' output offsets, so the records
 // come out in point order, exactly as the reference's library compaction orders them
 // (cub::DeviceSelect::Flagged, cuPythia/10_cub_compaction/cub_compaction.cu:76-80,
-// cuPythia/pipeline/generate.cu:97-104), without any block waiting on another.  K2 takes one
-// range per warp, spreads its accepted points over the lanes (every lane busy), takes each one's
+// cuPythia/pipeline/generate.cu:97-104), without any block waiting on another.  K2 gives every
+// warp an equal run of 32-point blocks, which may begin and end inside ranges, spreads the run's accepted points
+// over the lanes a whole warp at a time, takes each one's
 // point index from its block's mask, recomputes the points' kinematics and brackets from the
 // staged coordinates (the PDFs come from K1 too), picks process, flavours and colour
 // flow, and writes the 64-byte records as four 16-byte stores; on request K3 adds the 7-point

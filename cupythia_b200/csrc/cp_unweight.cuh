@@ -6,7 +6,7 @@
 
 #define CP_UNW_SLOT 8   // sum w, sum w^2, max w, n_bad, n_acc, sum event weight, n_over, unused
 #define CP_UNW_CHUNK (1ull << 24)   // points per production chunk (staging: 80 B per point)
-#define CP_UNW_RANGE 32             // 32-point blocks per record-builder warp (1024 points)
+#define CP_UNW_RANGE 32             // 32-point blocks per range of the output offsets (1024 points)
 // accept blocks: 128 threads, four resident per SM (128 registers a thread; five at 96 or six at 80
 // registers measure within 2%: the FMA pipe bounds the kernel, not the warps in flight), up to 32
 // points a thread
@@ -24,7 +24,7 @@ struct UnwLaunch {
   float4* pdf;                 // staging per point: fa[8], fb[8] of the accepted points (K1 -> K2)
   uint4* tails;                // staging per point: event weight and x[3] (bits), or null (no records)
   unsigned* bmask;             // accept mask of each 32-point block (bit = lane = point - 32 block)
-  unsigned* rsum;              // accepted points per 1024-point range (zeroed before K1)
+  unsigned* rsum;              // accepted points per 1024-point range (left zero by the scan of the chunk before)
   const unsigned long long* roff;   // output index of the first record of each range
   uint64_t nblk, nrange;
   float* scalew;               // per record: 6 scale-variation ratios, or null

@@ -6,8 +6,8 @@
 //   sum w, sum w^2   Kahan-compensated FP32 per thread, compensated warp and block trees,
 //   max w, n_bad     per thread, then warp / block,
 //   sum w^2 per bin  warp-private shared-memory histograms, deterministic lane-order adds.
-// Each block writes one FP64 slot; a second kernel reduces the slots in a fixed order (FP64)
-// and its last block refines the grid in FP64, so iterations chain on the stream
+// Each block writes one FP64 slot; a second kernel, one cluster of blocks, reduces the slots in a fixed order (FP64)
+// and its first block refines the grid in FP64, so iterations chain on the stream
 // without host round trips (the reference round-trips through the host every iteration:
 // cuPythia/11_vegas_importance/vegas.cu:107-124).
 #include <cooperative_groups.h>
@@ -205,9 +205,11 @@ __device__ __forceinline__ void cp_refine_sync(int id) { asm volatile("bar.sync 
 // Lepage's refinement of one dimension (FP64) by two warps (so 50 bins are one round), from S.h and S.e:
 // smooth (1,1)/(1,1,1)/(1,1), normalise, compress r = ((d - 1) / ln d)^alpha, and rebin to equal shares of
 // sum r.  The new edge k lies in the first bin j with cum[j + 1] >= k rsum / nb, cum the
-// running sum of r: a binary search, since r >= 0.  It is all latency: the two sums over the bins are
-// warp trees (serial on one thread: 2,200 of 6,500 cycles for 50 bins, now 700), and the usual
-// alpha of 3/2 is a product and a square root instead of a power.
+// running sum of r: a binary search.  The sum is formed by a tree, so over bins without a share it may fall by its
+// rounding; what two edges look for lies further apart than that, so they keep their order, and an edge that
+// falls on such a flat stretch may take either end of it, as with any other rounding of the sum.  It is all latency:
+// the two sums over the bins are warp trees (serial on one thread: 2,200 of 6,500 cycles for 50 bins, now 700), and
+// the usual alpha of 3/2 is a product and a square root instead of a power.
 __device__ __forceinline__ void cp_refine_dim(CpRefineDim& S, double* __restrict__ edges, int nb, double alpha, int bar)
 {
   const int t = threadIdx.x % (32 * CP_REFINE_WARPS), n = 32 * CP_REFINE_WARPS, lane = t & 31, w = t >> 5;
@@ -307,8 +309,8 @@ __global__ void __launch_bounds__(256) k_refine(double* edges, const double* red
 // of warp w adds column c of the slots b = w + 4 o (mod 32), so a load of the warp covers whole sectors
 // and 296 slots are two batches of loads.  It is latency from end to end, and a pass of a few thousand points waits
 // for it longer than for its own kernel.  With a grid of 20 blocks, a ticket for the last of them, the sums read
-// back through L2 and serial sums in the refinement, five iterations of 4,099 points took 137 us, now 128, and ten
-// of a million 818, now 803.  The block is as small as that because the pass kernels on either side leave room for
+// back through L2 and serial sums in the refinement, five iterations of 4,099 points took 137 us, then 128, and ten
+// of a million 818, then 803.  The block is as small as that because the pass kernels on either side leave room for
 // it, and it for them, so that chained launches take their places early (640 threads: 125 and 816 us).
 #define CP_FINISH_BLOCKS 8
 #define CP_FINISH_THREADS 320
